@@ -2,7 +2,8 @@
 // timestep (no reference counterpart: the reference steps one domain per
 // OpenCL queue, src/lbm/mod.rs:250-272).
 //
-// Two persistent launches advance every domain of a batch by one step:
+// Two persistent launches advance every domain of a batch by one step (and, where a domain's
+// FAST field is a convolution over its bins, the launches of field_fft.cu):
 // k_batch_stream (cooperative) runs
 //   A  stream_collide of every cell of every domain   (sc_cell)
 //   B  LOD bin sums of every domain                     (lod_bin_warp)
@@ -249,6 +250,38 @@ __global__ void __launch_bounds__(256, 2) k_batch_field(const BatchDev B) {
     }
 }
 
+// Phase C where a domain's convolution (field_fft.cu) left its field to the direct sum: the
+// blocks leave at once unless some domain's gate is set
+static __global__ void __launch_bounds__(256, 2) k_batch_field_gated(const BatchDev B, const uint32_t* const* gates) {
+    __shared__ __align__(16) EbSmem<true> sm;
+    __shared__ DevLbm sL;
+    __shared__ uint32_t s_dom, s_gate;
+    int any = 0;
+    for (uint32_t d = threadIdx.x; d < B.ndom; d += blockDim.x) any |= gates[d] != nullptr && *gates[d] != 0u;
+    if (!__syncthreads_or(any)) return;
+    eb_init(sm);
+    uint32_t uses[2] = {0u, 0u};
+    for (uint32_t t = blockIdx.x; t < B.total_bricks; t += gridDim.x) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_dom = find_domain(B.brick_off, B.ndom, t);
+            s_gate = *gates[s_dom];
+            if (s_gate) sL = B.doms[s_dom];
+        }
+        __syncthreads();
+        if (!s_gate) continue;
+        if (!eb_tile<true>(sL, t - B.brick_off[s_dom], 0u, sm, uses)) {
+            if (threadIdx.x == 0) atomicExch(B.err, 1u);
+            return;
+        }
+    }
+}
+
+cudaError_t launch_batch_gated(const BatchDev& B, const uint32_t* const* gates, uint32_t grid, cudaStream_t s) {
+    k_batch_field_gated<<<grid, 256, 0, s>>>(B, gates);
+    return cudaGetLastError();
+}
+
 static const void* stream_kernel(int ft, bool mhd, bool rows) {
     if (rows) {
         if (ft == ION_FP32)
@@ -310,7 +343,7 @@ cudaError_t launch_batch_step(const BatchDev& B, int ft, bool mhd, bool fast, ui
     cfg.numAttrs = 1;
     void* args[] = {(void*)&B, (void*)&odd};
     e = cudaLaunchKernelExC(&cfg, ks, args);
-    if (e != cudaSuccess || !mhd) return e;
+    if (e != cudaSuccess || !mhd || B.total_bricks == 0u) return e;
     cudaLaunchConfig_t cf = {};
     cf.gridDim = dim3(grid);
     cf.blockDim = dim3(block);

@@ -1,0 +1,121 @@
+// fft_regs.cuh -- complex Fourier transforms of 4, 8, 16 and 32 points held in a
+// thread's registers (Cooley-Tukey, J. W. Cooley and J. W. Tukey, Math. Comp. 19, 1965).
+// Every index is known at compile time, so outputs that are not used cost nothing.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace ion {
+
+template <class T> struct C2 { T x, y; };
+
+__device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
+
+// cos(2 pi j / 32), j = 0..8 (rounded from the exact values)
+__host__ __device__ constexpr double cos32(int j) {
+    constexpr double t[9] = {1.0, 0.98078528040323044913, 0.92387953251128675613, 0.83146961230254523708,
+                             0.70710678118654752440, 0.55557023301960222474, 0.38268343236508977173,
+                             0.19509032201612826785, 0.0};
+    const int k = j & 31;
+    return k <= 8 ? t[k] : k <= 16 ? -t[16 - k] : k <= 24 ? -t[k - 16] : t[32 - k];
+}
+__host__ __device__ constexpr double sin32(int j) { return cos32(j + 24); }  // cos(a - pi/2)
+
+// v * exp(SIGN 2 pi i j / 32)
+template <int SIGN, class T>
+__device__ __forceinline__ C2<T> twist(const C2<T> v, const int j) {
+    const int k = j & 31;
+    if (k == 0) return v;
+    if (k == 8) return SIGN > 0 ? C2<T>{-v.y, v.x} : C2<T>{v.y, -v.x};
+    if (k == 16) return {-v.x, -v.y};
+    if (k == 24) return SIGN > 0 ? C2<T>{v.y, -v.x} : C2<T>{-v.y, v.x};
+    const T c = (T)cos32(k), s = (T)(SIGN * sin32(k));
+    return {fma_(v.x, c, -(v.y * s)), fma_(v.x, s, v.y * c)};
+}
+// a + v exp(SIGN 2 pi i j / 32)
+template <int SIGN, class T>
+__device__ __forceinline__ C2<T> add_twist(const C2<T> a, const C2<T> v, const int j) {
+    const int k = j & 31;
+    if (k % 8 == 0) {
+        const C2<T> w = twist<SIGN>(v, j);
+        return {a.x + w.x, a.y + w.y};
+    }
+    const T c = (T)cos32(k), s = (T)(SIGN * sin32(k));
+    return {fma_(v.x, c, fma_(-v.y, s, a.x)), fma_(v.x, s, fma_(v.y, c, a.y))};
+}
+
+template <int SIGN, class T>
+__device__ __forceinline__ void dft4(C2<T>& a, C2<T>& b, C2<T>& c, C2<T>& d) {
+    const C2<T> s0 = {a.x + c.x, a.y + c.y}, d0 = {a.x - c.x, a.y - c.y};
+    const C2<T> s1 = {b.x + d.x, b.y + d.y}, d1 = {b.x - d.x, b.y - d.y};
+    const C2<T> r = SIGN > 0 ? C2<T>{-d1.y, d1.x} : C2<T>{d1.y, -d1.x};  // +-i d1
+    a = {s0.x + s1.x, s0.y + s1.y};
+    b = {d0.x + r.x, d0.y + r.y};
+    c = {s0.x - s1.x, s0.y - s1.y};
+    d = {d0.x - r.x, d0.y - r.y};
+}
+
+// v[n] <- sum_k v[k] exp(SIGN 2 pi i n k / N)
+template <int N, int SIGN, class T>
+__device__ __forceinline__ void fft_regs(C2<T> (&v)[N]) {
+    static_assert(N == 8 || N == 16 || N == 32, "transform sizes in use");
+    if constexpr (N == 8) {  // k = 2a + b, n = c + 4d
+        C2<T> t[2][4];
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+#pragma unroll
+            for (int a = 0; a < 4; a++) t[b][a] = v[2 * a + b];
+            dft4<SIGN>(t[b][0], t[b][1], t[b][2], t[b][3]);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const C2<T> w = twist<SIGN>(t[1][c], 4 * c);
+            v[c] = {t[0][c].x + w.x, t[0][c].y + w.y};
+            v[c + 4] = {t[0][c].x - w.x, t[0][c].y - w.y};
+        }
+    } else if constexpr (N == 16) {  // k = 4a + b, n = c + 4d
+        C2<T> t[4][4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+#pragma unroll
+            for (int a = 0; a < 4; a++) t[b][a] = v[4 * a + b];
+            dft4<SIGN>(t[b][0], t[b][1], t[b][2], t[b][3]);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            C2<T> q[4];
+#pragma unroll
+            for (int b = 0; b < 4; b++) q[b] = twist<SIGN>(t[b][c], 2 * b * c);
+            dft4<SIGN>(q[0], q[1], q[2], q[3]);
+#pragma unroll
+            for (int d = 0; d < 4; d++) v[c + 4 * d] = q[d];
+        }
+    } else {  // even and odd k
+        C2<T> e[16], o[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) { e[k] = v[2 * k]; o[k] = v[2 * k + 1]; }
+        fft_regs<16, SIGN>(e);
+        fft_regs<16, SIGN>(o);
+#pragma unroll
+        for (int n = 0; n < 16; n++) {
+            v[n] = add_twist<SIGN>(e[n], o[n], n);
+            v[n + 16] = add_twist<SIGN>(e[n], o[n], n + 16);
+        }
+    }
+}
+
+// the first N outputs of the 2N-point transform of (a[0], b[0], a[1], b[1], ...), into e,
+// from e and o, the N-point transforms of a and b
+template <int N, int SIGN, class T>
+__device__ __forceinline__ void fft_join(C2<T> (&e)[N], const C2<T> (&o)[N]) {
+#pragma unroll
+    for (int n = 0; n < N; n++) e[n] = add_twist<SIGN>(e[n], o[n], n * (16 / N));
+}
+template <int N, int SIGN, class T>
+__device__ __forceinline__ void fft_half(C2<T> (&e)[N], C2<T> (&o)[N]) {
+    fft_regs<N, SIGN>(e);
+    fft_regs<N, SIGN>(o);
+    fft_join<N, SIGN>(e, o);
+}
+
+}  // namespace ion

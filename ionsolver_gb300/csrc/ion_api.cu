@@ -20,6 +20,7 @@
 #include <memory>
 
 #include "ion_device.cuh"
+#include "field_fft.h"
 #include "ion_launch.h"
 #include "surrogate.h"
 
@@ -200,6 +201,7 @@ struct ion_lbm {
     uint64_t kcount[3] = {0, 0, 0};
     std::vector<void*> allocs;
     std::unique_ptr<ion::Surrogate> sur;  // learned far field (field_mode SURROGATE)
+    ion::FftField fft;         // FAST field as a convolution over the bins; fft.G null: the direct sum
 };
 
 namespace {
@@ -245,7 +247,37 @@ int launch_stream_collide(ion_lbm* h, uint64_t t) {
     return ION_OK;
 }
 
+// Lays out the FAST field's convolution for a handle (once; launches work on the handle's
+// stream and allocates, so it runs when a handle is created or switched to FAST, never inside
+// a step).  Where the device has no memory left for it the direct sum stays.
+int setup_fft(ion_lbm* h) {
+    if (h->fft.G || h->cfg.field_mode != ION_FIELD_FAST || !h->cfg.ext_magneto_hydro || !fft_field_fits(h->L)) return ION_OK;
+    FftField F;
+    size_t bytes[4] = {0, 0, 0, 4};
+    fft_field_sizes(h->L, F, &bytes[0], &bytes[1], &bytes[2]);
+    void** const ptr[4] = {(void**)&F.G, (void**)&F.S, (void**)&F.out, (void**)&F.direct};
+    for (int i = 0; i < 4; i++) {
+        if (cudaMalloc(ptr[i], bytes[i]) != cudaSuccess) {
+            cudaGetLastError();
+            while (i-- > 0) cudaFree(*ptr[i]);
+            return ION_OK;
+        }
+    }
+    for (auto* q : ptr) h->allocs.push_back(*q);
+    CK(cudaMemsetAsync(F.direct, 0, 4, h->stream));
+    CK(launch_fft_plan(h->L, F, h->stream));
+    g_launches++;
+    h->fft = F;
+    return ION_OK;
+}
+
 int launch_field(ion_lbm* h) {
+    if (h->cfg.field_mode == ION_FIELD_FAST && h->fft.G) {
+        g_launches += launch_fft_field(h->L, h->fft, h->stream) + 1;
+        launch_update_e_b_gated(h->L, h->d_err, h->fft.direct, h->stream);
+        CKL();
+        return ION_OK;
+    }
     // the exact sum; SURROGATE handles use its FAST arithmetic outside the surrogate path
     launch_update_e_b(h->L, h->cfg.field_mode != ION_FIELD_BITWISE, h->d_err, h->stream);
     g_launches++;
@@ -311,6 +343,7 @@ int enqueue_step(ion_lbm* h, uint64_t t) {
 uint32_t kernels_per_step(const ion_lbm* h) {
     uint32_t k = 1u + (h->cfg.ext_magneto_hydro ? (h->L.depth > 0 ? 2u : 1u) : 0u);
     if (h->cfg.ext_magneto_hydro && h->cfg.field_mode == ION_FIELD_SURROGATE && h->sur) k += h->sur->launches_per_step();
+    if (h->cfg.ext_magneto_hydro && h->cfg.field_mode == ION_FIELD_FAST && h->fft.G) k += 1u + 2u * fft_passes(h->L, h->fft);
     return k;
 }
 
@@ -562,6 +595,8 @@ int ion_lbm_create(const ion_config* cfg, ion_lbm** out) {
             return fail(ION_E_CUDA, "upload of LOD centres failed");
         }
     }
+    rc = setup_fft(h);
+    if (rc) { destroy_handle(h); return rc; }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) { destroy_handle(h); return fail(ION_E_CUDA, "create: stream sync failed"); }
     for (auto& e : h->ev) cudaEventCreate(&e);
     *out = h;
@@ -1229,6 +1264,12 @@ struct ion_batch {
     uint32_t total_bricks[3] = {0, 0, 0};
     uint32_t* d_bin_off = nullptr;
     uint32_t total_bins = 0;
+    // domains whose FAST field is a convolution: their launches by bin count (8^3, 16^3) and
+    // pass, and the bricks of the direct sum that stands by for each (FftField::direct)
+    std::vector<ion::FftBatch> fft[2];
+    uint32_t* d_gated_off = nullptr;
+    const uint32_t** d_gates = nullptr;  // [domains]: FftField::direct, null without a convolution
+    uint32_t gated_bricks = 0;
     uint32_t* d_row_off = nullptr;  // row-staged stencil: prefix sums of ny nz (null: tiles of cells)
     uint32_t total_rows = 0;
     uint32_t* d_sync = nullptr;  // [0] barrier count, [1] barrier generation, [2] error
@@ -1238,6 +1279,7 @@ struct ion_batch {
     bool tuned = false;
     uint32_t block = 256, grid = 0;
     std::vector<std::array<float, 3>> tuning;  // block, grid, ms per step
+    uint32_t step_launches = 0;
     cudaGraphExec_t graph = nullptr;
     bool graph_failed = false;
     cudaEvent_t ev[4] = {};
@@ -1269,12 +1311,94 @@ BatchDev batch_view(ion_batch* b, uint32_t block) {
     return B;
 }
 
+// one step's launches (counted into *launches): the stencil and bins, the direct field sums,
+// the convolutions and the direct sums that stand by for them
+cudaError_t batch_enqueue(ion_batch* b, uint32_t block, uint32_t grid, uint64_t t, uint32_t* launches) {
+    const BatchDev B = batch_view(b, block);
+    cudaError_t e = launch_batch_step(B, b->ft, b->mhd, b->fast, grid, block, t, b->stream);
+    *launches = b->mhd && B.total_bricks ? 2u : 1u;
+    for (const auto& f : b->fft)
+        if (e == cudaSuccess && !f.empty()) {
+            *launches += launch_fft_batch(f.data(), (uint32_t)f.size(), b->stream);
+            e = cudaGetLastError();
+        }
+    if (e == cudaSuccess && b->gated_bricks) {
+        BatchDev D = B;
+        D.brick_off = b->d_gated_off;
+        D.total_bricks = b->gated_bricks;
+        e = launch_batch_gated(D, b->d_gates, 2u * (uint32_t)b->sms, b->stream);
+        *launches += 1u;
+    }
+    return e;
+}
+
 int batch_launch(ion_batch* b, uint32_t block, uint32_t grid) {
-    const cudaError_t e = launch_batch_step(batch_view(b, block), b->ft, b->mhd, b->fast, grid, block, b->t, b->stream);
+    uint32_t launches = 0;
+    const cudaError_t e = batch_enqueue(b, block, grid, b->t, &launches);
     if (e != cudaSuccess) return fail(ION_E_CUDA, "batch step launch: %s", cudaGetErrorString(e));
-    g_launches += b->mhd ? 2 : 1;
+    g_launches += launches;
+    b->step_launches = launches;
     b->t += 1;
     return ION_OK;
+}
+
+// The tables of the domains whose field is a convolution: per bin count and pass the blocks
+// of each domain (prefix sums; a domain with fewer passes has none in the last ones).
+template <class P, class A>
+int batch_fft_tables(ion_batch* b, P&& convolved, A&& dalloc) {
+    auto upload = [&](const void* src, size_t bytes, void** dst) -> int {
+        int rc = dalloc(dst, bytes);
+        if (!rc && cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) rc = fail(ION_E_CUDA, "batch table upload");
+        return rc;
+    };
+    const uint32_t count = (uint32_t)b->doms.size();
+    int rc = ION_OK;
+    for (int k = 0; k < 2 && !rc; k++) {
+        FftBatch B{};
+        B.doms = b->d_doms;
+        B.nd = k == 0 ? 8u : 16u;
+        std::vector<uint32_t> index;
+        std::vector<FftField> fields;
+        uint32_t passes = 0;
+        for (uint32_t i = 0; i < count; i++) {
+            const ion_lbm* h = b->doms[i];
+            if (!convolved(i) || h->L.nd != B.nd) continue;
+            index.push_back(i);
+            fields.push_back(h->fft);
+            passes = std::max(passes, fft_passes(h->L, h->fft));
+        }
+        B.n = (uint32_t)index.size();
+        if (B.n == 0) continue;
+        rc = upload(index.data(), sizeof(uint32_t) * B.n, (void**)&B.index);
+        if (!rc) rc = upload(fields.data(), sizeof(FftField) * B.n, (void**)&B.fields);
+        for (uint32_t p = 0; p < passes && !rc; p++) {
+            std::vector<uint32_t> src(B.n + 1, 0), sum(B.n + 1, 0), put(B.n + 1, 0);
+            for (uint32_t e = 0; e < B.n; e++) {
+                const DevLbm& L = b->doms[index[e]]->L;
+                src[e + 1] = src[e] + fft_src_blocks(L);
+                sum[e + 1] = sum[e] + fft_sum_blocks(L, fields[e], p);
+                put[e + 1] = put[e] + fft_put_blocks(L, fields[e], p);
+            }
+            B.src_blocks = src[B.n]; B.sum_blocks = sum[B.n]; B.put_blocks = put[B.n];
+            rc = upload(src.data(), sizeof(uint32_t) * (B.n + 1), (void**)&B.src_off);
+            if (!rc) rc = upload(sum.data(), sizeof(uint32_t) * (B.n + 1), (void**)&B.sum_off);
+            if (!rc) rc = upload(put.data(), sizeof(uint32_t) * (B.n + 1), (void**)&B.put_off);
+            b->fft[k].push_back(B);
+        }
+    }
+    std::vector<uint32_t> bricks(count + 1, 0);
+    std::vector<const uint32_t*> gates(count, nullptr);
+    for (uint32_t i = 0; i < count; i++) {
+        const DevLbm& L = b->doms[i]->L;
+        if (convolved(i)) gates[i] = b->doms[i]->fft.direct;
+        bricks[i + 1] = bricks[i] + (convolved(i) ? eb_bricks(L.nx, L.ny, L.nz) : 0u);
+    }
+    b->gated_bricks = bricks[count];
+    if (!rc && b->gated_bricks) {
+        rc = upload(bricks.data(), sizeof(uint32_t) * (count + 1), (void**)&b->d_gated_off);
+        if (!rc) rc = upload(gates.data(), sizeof(uint32_t*) * count, (void**)&b->d_gates);
+    }
+    return rc;
 }
 
 void destroy_batch(ion_batch* b) {
@@ -1333,6 +1457,8 @@ int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out) {
         b->allocs.push_back(*p);
         return ION_OK;
     };
+    // a domain takes the path of its own steps
+    auto convolved = [&](uint32_t i) { return b->fast && domains[i]->fft.G != nullptr; };
     std::vector<DevLbm> views(count);
     std::vector<uint32_t> bins(count + 1, 0);
     for (uint32_t i = 0; i < count; i++) {
@@ -1354,13 +1480,14 @@ int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out) {
         std::vector<uint32_t> bricks(count + 1, 0);
         for (uint32_t i = 0; i < count; i++) {
             const DevLbm& L = domains[i]->L;
-            bricks[i + 1] = bricks[i] + eb_bricks(L.nx, L.ny, L.nz) * (256u / kBatchBlocks[s]);
+            bricks[i + 1] = bricks[i] + (convolved(i) ? 0u : eb_bricks(L.nx, L.ny, L.nz) * (256u / kBatchBlocks[s]));
         }
         b->total_bricks[s] = bricks[count];
         if (!rc) rc = dalloc((void**)&b->d_brick_off[s], sizeof(uint32_t) * (count + 1));
         if (!rc && cudaMemcpy(b->d_brick_off[s], bricks.data(), sizeof(uint32_t) * (count + 1), cudaMemcpyHostToDevice) != cudaSuccess)
             rc = fail(ION_E_CUDA, "batch table upload");
     }
+    if (!rc) rc = batch_fft_tables(b, convolved, dalloc);
     // the row-staged stencil when every domain's rows are whole 16-byte streams of at most
     // BATCH_ROW_MAX cells and its slot offsets fit in 32 bits (as for k_sc_rows_ws)
     bool rows_ok = true;
@@ -1442,8 +1569,8 @@ int ion_batch_run(ion_batch* b, uint64_t steps) {
         bool ok = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         if (ok) {
             const uint64_t t0 = b->t;
-            const cudaError_t e1 = launch_batch_step(batch_view(b, b->block), b->ft, b->mhd, b->fast, b->grid, b->block, 0, b->stream);
-            const cudaError_t e2 = launch_batch_step(batch_view(b, b->block), b->ft, b->mhd, b->fast, b->grid, b->block, 1, b->stream);
+            const cudaError_t e1 = batch_enqueue(b, b->block, b->grid, 0, &b->step_launches);
+            const cudaError_t e2 = batch_enqueue(b, b->block, b->grid, 1, &b->step_launches);
             const cudaError_t e3 = cudaStreamEndCapture(b->stream, &g);
             b->t = t0;
             ok = e1 == cudaSuccess && e2 == cudaSuccess && e3 == cudaSuccess &&
@@ -1455,7 +1582,7 @@ int ion_batch_run(ion_batch* b, uint64_t steps) {
     if (b->graph) {
         for (; steps >= 2; steps -= 2) {
             CK(cudaGraphLaunch(b->graph, b->stream));
-            g_launches += b->mhd ? 4 : 2;
+            g_launches += 2u * b->step_launches;
             b->t += 2;
         }
     }
@@ -1666,7 +1793,7 @@ int ion_lbm_set_field_mode(ion_lbm* h, int mode) {
     }
     h->cfg.field_mode = (uint8_t)mode;
     h->graph_dirty = true;
-    return ION_OK;
+    return setup_fft(h);
 }
 
 // ---- device selection and the FP32 peak probe ---------------------------------

@@ -66,6 +66,9 @@ int batch_max_blocks_per_sm(int ft, bool mhd, bool fast, bool rows, int block);
 cudaError_t launch_batch_step(const BatchDev& B, int ft, bool mhd, bool fast, uint32_t grid, uint32_t block,
                               uint64_t t, cudaStream_t s);
 
+// the direct field sum of the domains (256-thread bricks) whose gate is set
+cudaError_t launch_batch_gated(const BatchDev& B, const uint32_t* const* gates, uint32_t grid, cudaStream_t s);
+
 // per velocity set (lbm_q19.cu, lbm_q15.cu, lbm_q9.cu)
 #define ION_DECLARE_LBM_DISPATCH(NAME)                                                                    \
     void NAME##_stream_collide(const DevLbm& L, int ft, int mode, bool trt, uint64_t t, uint32_t* err,       \
