@@ -55,10 +55,24 @@ __device__ __forceinline__ void dft4(C2<T>& a, C2<T>& b, C2<T>& c, C2<T>& d) {
     d = {d0.x - r.x, d0.y - r.y};
 }
 
-// v[n] <- sum_k v[k] exp(SIGN 2 pi i n k / N)
-template <int N, int SIGN, class T>
-__device__ __forceinline__ void fft_regs(C2<T> (&v)[N]) {
-    static_assert(N == 8 || N == 16 || N == 32, "transform sizes in use");
+// dft4 with b and d times sg = +-1 (exact; a fused step costs what the addition does):
+// with -1 the outputs come half a turn on, c d a b
+template <int SIGN, class T>
+__device__ __forceinline__ void dft4_turn(C2<T>& a, C2<T>& b, C2<T>& c, C2<T>& d, const T sg) {
+    const C2<T> s0 = {a.x + c.x, a.y + c.y}, d0 = {a.x - c.x, a.y - c.y};
+    const C2<T> s1 = {b.x + d.x, b.y + d.y}, d1 = {b.x - d.x, b.y - d.y};
+    const C2<T> r = SIGN > 0 ? C2<T>{-d1.y, d1.x} : C2<T>{d1.y, -d1.x};  // +-i d1
+    a = {fma_(s1.x, sg, s0.x), fma_(s1.y, sg, s0.y)};
+    b = {fma_(r.x, sg, d0.x), fma_(r.y, sg, d0.y)};
+    c = {fma_(-s1.x, sg, s0.x), fma_(-s1.y, sg, s0.y)};
+    d = {fma_(-r.x, sg, d0.x), fma_(-r.y, sg, d0.y)};
+}
+
+// v[n] <- sum_k v[k] exp(SIGN 2 pi i n k / N).  TURN (N = 8, 16): with sg = -1 the outputs are
+// stored N/2 on, v[n] = output (n + N/2) mod N
+template <int N, int SIGN, bool TURN = false, class T>
+__device__ __forceinline__ void fft_regs(C2<T> (&v)[N], const T sg = (T)1) {
+    static_assert(N == 8 || N == 16 || (N == 32 && !TURN), "transform sizes in use");
     if constexpr (N == 8) {  // k = 2a + b, n = c + 4d
         C2<T> t[2][4];
 #pragma unroll
@@ -70,8 +84,13 @@ __device__ __forceinline__ void fft_regs(C2<T> (&v)[N]) {
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const C2<T> w = twist<SIGN>(t[1][c], 4 * c);
-            v[c] = {t[0][c].x + w.x, t[0][c].y + w.y};
-            v[c + 4] = {t[0][c].x - w.x, t[0][c].y - w.y};
+            if constexpr (TURN) {
+                v[c] = {fma_(w.x, sg, t[0][c].x), fma_(w.y, sg, t[0][c].y)};
+                v[c + 4] = {fma_(-w.x, sg, t[0][c].x), fma_(-w.y, sg, t[0][c].y)};
+            } else {
+                v[c] = {t[0][c].x + w.x, t[0][c].y + w.y};
+                v[c + 4] = {t[0][c].x - w.x, t[0][c].y - w.y};
+            }
         }
     } else if constexpr (N == 16) {  // k = 4a + b, n = c + 4d
         C2<T> t[4][4];
@@ -86,7 +105,8 @@ __device__ __forceinline__ void fft_regs(C2<T> (&v)[N]) {
             C2<T> q[4];
 #pragma unroll
             for (int b = 0; b < 4; b++) q[b] = twist<SIGN>(t[b][c], 2 * b * c);
-            dft4<SIGN>(q[0], q[1], q[2], q[3]);
+            if constexpr (TURN) dft4_turn<SIGN>(q[0], q[1], q[2], q[3], sg);
+            else dft4<SIGN>(q[0], q[1], q[2], q[3]);
 #pragma unroll
             for (int d = 0; d < 4; d++) v[c + 4 * d] = q[d];
         }
@@ -102,20 +122,6 @@ __device__ __forceinline__ void fft_regs(C2<T> (&v)[N]) {
             v[n + 16] = add_twist<SIGN>(e[n], o[n], n + 16);
         }
     }
-}
-
-// the first N outputs of the 2N-point transform of (a[0], b[0], a[1], b[1], ...), into e,
-// from e and o, the N-point transforms of a and b
-template <int N, int SIGN, class T>
-__device__ __forceinline__ void fft_join(C2<T> (&e)[N], const C2<T> (&o)[N]) {
-#pragma unroll
-    for (int n = 0; n < N; n++) e[n] = add_twist<SIGN>(e[n], o[n], n * (16 / N));
-}
-template <int N, int SIGN, class T>
-__device__ __forceinline__ void fft_half(C2<T> (&e)[N], C2<T> (&o)[N]) {
-    fft_regs<N, SIGN>(e);
-    fft_regs<N, SIGN>(o);
-    fft_join<N, SIGN>(e, o);
 }
 
 }  // namespace ion

@@ -15,7 +15,7 @@
 //               (b/2 + 1) of b offsets per axis are kept.
 //   k_fft_src   spectra of the sources, 4 (nd + 1) blocks; block 0 also looks at the range
 //               of the sources (see below).
-//   k_fft_sum   one block per offset and field (E or B): product of spectra, then the
+//   k_fft_sum   one block per offset and component of E or B: product of spectra, then the
 //               inverse transforms along z, y and x in registers, passed on through
 //               shared memory.
 //   k_fft_put   the sums to the cells, x-rows at a time: E_stat + KE e, B_stat + KMU b.
@@ -34,15 +34,15 @@ namespace ion {
 
 namespace {
 
-__host__ __device__ constexpr uint32_t slot_elems(uint32_t nd) { return 3u * nd * nd; }  // one kx plane, 3 components, [z][y]
-// kx planes transformed together: 3 PL M = 192 threads
+__host__ __device__ constexpr uint32_t slot_elems(uint32_t nd) { return nd * nd; }  // one kx plane, [z][y]
+// kx planes transformed together: PL M = 64 lines, two lanes each
 __host__ __device__ constexpr uint32_t planes(uint32_t nd) { return 32u / nd; }
-__host__ __device__ constexpr uint32_t stage_elems(uint32_t nd) { return planes(nd) * 3u * nd * (2u * nd + 1u); }
+__host__ __device__ constexpr uint32_t stage_elems(uint32_t nd) { return planes(nd) * nd * (2u * nd + 1u); }
 // the staged planes overlay the slots that are not written yet
 __host__ __device__ constexpr uint32_t sum_smem(uint32_t nd) { return ((nd - planes(nd)) * slot_elems(nd) + stage_elems(nd)) * 8u; }
 static_assert(planes(16) * slot_elems(16) <= stage_elems(16) && planes(8) * slot_elems(8) <= stage_elems(8),
               "the last planes' slots lie inside the staging area");
-constexpr uint32_t SUM_THREADS = 192, SRC_THREADS = 256, PUT_THREADS = 256, PUT_X = 128;
+constexpr uint32_t SUM_THREADS = 128, SUM_BLOCKS = 5, SRC_THREADS = 512, PUT_THREADS = 256, PUT_X = 128;
 
 #define ION_TW(j) {(float)cos32(j), (float)sin32(j)}
 __constant__ float2 c_tw[32] = {  // exp(2 pi i j / 32)
@@ -124,14 +124,16 @@ template <int ND>
 __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, const uint32_t block) {
     constexpr uint32_t M = 2u * ND, NB = ND * ND * ND;
     __shared__ float s[ND * ND * (ND + 1)];  // [z][y][x], rows of ND + 1
-    __shared__ float2 a[ND][ND], b[ND][M];
+    __shared__ float2 a[ND][ND], b[ND][M], tw[M];
     __shared__ uint32_t s_max[4], s_bad;
     const uint32_t c = block % 4u, kx = block / 4u;
     const uint32_t first = L.first_src, last = min(L.n_lod_own, L.n_bins);
     if (threadIdx.x < 4u) s_max[threadIdx.x] = 0u;
     if (threadIdx.x == 0u) s_bad = 0u;
+    if (threadIdx.x < M) tw[threadIdx.x] = c_tw[threadIdx.x * (32u / M)];  // the lanes index it apart
     __syncthreads();
     uint32_t m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
     for (uint32_t d = threadIdx.x; d < NB; d += SRC_THREADS) {
         const float4 v = d >= first && d < last ? reinterpret_cast<const float4*>(L.qu_lod)[d] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float w[4] = {v.x, v.x * v.y, v.x * v.z, v.x * v.w};
@@ -159,7 +161,7 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
 #pragma unroll
         for (uint32_t x = 0; x < ND; x++) {
             const float v = s[t * (ND + 1) + x];
-            const float2 w = c_tw[((kx * x) % M) * (32u / M)];
+            const float2 w = tw[(kx * x) % M];
             acc.x = fmaf(v, w.x, acc.x);
             acc.y = fmaf(-v, w.y, acc.y);
         }
@@ -173,7 +175,7 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
         float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (uint32_t y = 0; y < ND; y++) {
-            const float2 v = a[z][y], w = c_tw[((ky * y) % M) * (32u / M)];
+            const float2 v = a[z][y], w = tw[(ky * y) % M];
             acc.x = fmaf(v.x, w.x, fmaf(v.y, w.y, acc.x));
             acc.y = fmaf(v.y, w.x, fmaf(-v.x, w.y, acc.y));
         }
@@ -186,7 +188,7 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
         float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (uint32_t z = 0; z < ND; z++) {
-            const float2 v = b[z][ky], w = c_tw[((kz * z) % M) * (32u / M)];
+            const float2 v = b[z][ky], w = tw[(kz * z) % M];
             acc.x = fmaf(v.x, w.x, fmaf(v.y, w.y, acc.x));
             acc.y = fmaf(v.y, w.x, fmaf(-v.x, w.y, acc.y));
         }
@@ -195,7 +197,7 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
 }
 
 // ---------------------------------------------------------------------------
-// the sums of one offset: block = (((oz - oz0) bsy + oy) bsx + ox) 2 + (0: E, 1: B)
+// the sums of one offset: block = (((oz - oz0) bsy + oy) bsx + ox) 6 + (0..2: E, 3..5: B)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ C2<float> cmul(const float2 a, const float2 b) {
     return {fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x)};
@@ -204,147 +206,183 @@ __device__ __forceinline__ C2<float> cmul_sub(const C2<float> s, const float2 a,
     return {fmaf(-a.x, b.x, fmaf(a.y, b.y, s.x)), fmaf(-a.x, b.y, fmaf(-a.y, b.x, s.y))};
 }
 
+// Lines of M points are transformed by two lanes, 16 apart, as the N-point transforms of their
+// even and odd points (N = nd).  Of the first N outputs the lower lane gets the first half, the
+// upper lane the second; the upper lane's transform comes half a turn on, so that both keep
+// the lower half of their registers and pass on the upper half.
+template <int N>
+__device__ __forceinline__ void fft_pair(C2<float> (&v)[N], const bool upper) {
+    fft_regs<N, 1, true>(v, upper ? -1.0f : 1.0f);
+    if (upper) {
+#pragma unroll
+        for (int n = 0; n < N; n++) v[n] = twist<1>(v[n], ((n + N / 2) % N) * (16 / N));
+    }
+#pragma unroll
+    for (int n = 0; n < N / 2; n++) {
+        v[n].x += __shfl_xor_sync(0xFFFFFFFFu, v[n + N / 2].x, 16);
+        v[n].y += __shfl_xor_sync(0xFFFFFFFFu, v[n + N / 2].y, 16);
+    }
+}
+
 template <int ND>
 __device__ __forceinline__ void fft_sum(const DevLbm& L, const FftField& F, const uint32_t block, const uint32_t oz0,
                                         float2* sm) {
     constexpr uint32_t M = 2u * ND, PL = planes(ND), SLOT = slot_elems(ND), ROW = M + 1u;
-    const uint32_t group = block & 1u, o = block >> 1;
+    const uint32_t field = block % 6u, o = block / 6u, f = field % 3u;
     const uint32_t ox = o % L.bsx, oy = (o / L.bsx) % L.bsy, oz = oz0 + o / (L.bsx * L.bsy);
     // the offset's spectra, or its mirror image's: R_a changes sign with the wave number k_a
     const bool fx = ox >= F.ux, fy = oy >= F.uy, fz = oz >= F.uz;
     const uint32_t u = (fx ? L.bsx - ox : ox) + ((fy ? L.bsy - oy : oy) + (fz ? L.bsz - oz : oz) * F.uy) * F.ux;
-    const float2* G = F.G + (size_t)u * (ND + 1u) * 3u * M * M;
+    auto negative = [&](uint32_t c) { return c == 0u ? fx : c == 1u ? fy : fz; };
+    // component of the product: E_f = G_f q; B_f = (q v)_i G_j - (q v)_j G_i, (f, i, j) cyclic
+    const uint32_t i = f == 2u ? 0u : f + 1u, j = f == 0u ? 2u : f - 1u;
     // G(-kx, ky, kz) = conj G(kx, -ky, -kz): kx stays in 0..nd
     const bool ry = fx != fy, rz = fx != fz;
-    const uint32_t t = threadIdx.x;
-    const uint32_t f = (t / M) % 3u, pl = t / (3u * M), ky = t % M;  // this thread's line along z
-    const uint32_t gy = ry ? (M - ky) % M : ky;
-    // components of the product: E_f = G_f q; B_f = (q v)_i G_j - (q v)_j G_i, (f, i, j) cyclic
-    const uint32_t i = f == 2u ? 0u : f + 1u, j = f == 0u ? 2u : f - 1u;
-    auto flipped = [&](uint32_t c) { return c == 0u ? fx : c == 1u ? fy : fz; };
-    const bool nf = flipped(f), ni = flipped(i), nj = flipped(j);
-    auto product = [&](uint32_t kx, uint32_t kz) -> C2<float> {
-        const uint32_t gz = rz ? (M - kz) % M : kz;
-        const float2* g = G + (size_t)kx * 3u * M * M + gz * M + gy;
-        const float2* s = F.S + (size_t)kx * 4u * M * M + kz * M + ky;
-        auto load_g = [&](uint32_t c, bool neg) {
-            float2 v = __ldg(g + c * M * M);
-            if (fx) v.y = -v.y;
-            if (neg) { v.x = -v.x; v.y = -v.y; }
-            return v;
-        };
-        if (group == 0u) return cmul(load_g(f, nf), __ldg(s));
-        const float2 si = __ldg(s + (1u + i) * M * M), sj = __ldg(s + (1u + j) * M * M);
-        return cmul_sub(cmul(si, load_g(j, nj)), sj, load_g(i, ni));
+    const uint32_t t = threadIdx.x, par = (t >> 4) & 1u;  // even or odd points of the line
+    const uint32_t id = (t >> 5) * 16u + (t & 15u);       // line along z: (plane, ky)
+    const uint32_t ky = id % M, pl = id / M, gy = ry ? (M - ky) % M : ky;
+    const uint32_t conj = fx ? 0x80000000u : 0u, differ = negative(i) != negative(j) ? 0x80000000u : 0u;
+    const float2* const G = F.G + (size_t)u * (ND + 1u) * 3u * M * M + gy;
+    const float2* const S = F.S + par * M + ky;
+    auto flip = [](float v, uint32_t m) { return __uint_as_float(__float_as_uint(v) ^ m); };
+    auto gather = [&](uint32_t kx, C2<float>(&v)[ND], auto&& put) {
+        const float2* g = G + (size_t)kx * 3u * M * M;
+        const float2* s = S + (size_t)kx * 4u * M * M;
+        // kz = 2 k + par, or M - kz; the row's address is formed at each load (an opaque step:
+        // kept in registers from plane to plane the addresses spill)
+        const int start = (int)(rz ? M * M - par * M : par * M);
+        int step = rz ? -(int)(2u * M) : (int)(2u * M);
+        asm volatile("" : "+r"(step));
+        if (field < 3u) {
+#pragma unroll
+            for (uint32_t k = 0; k < (uint32_t)ND; k++) {
+                const int gz = k == 0u ? start & (int)(M * M - 1u) : start + (int)k * step;
+                float2 a = __ldg(g + f * M * M + gz);
+                a.y = flip(a.y, conj);
+                put(v[k], cmul(a, __ldg(s + 2u * k * M)));
+            }
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < (uint32_t)ND; k++) {
+                const int gz = k == 0u ? start & (int)(M * M - 1u) : start + (int)k * step;
+                float2 a = __ldg(g + j * M * M + gz), b = __ldg(g + i * M * M + gz);
+                a.y = flip(a.y, conj);
+                b.x = flip(b.x, differ);
+                b.y = flip(b.y, conj ^ differ);
+                put(v[k], cmul_sub(cmul(__ldg(s + (1u + i) * M * M + 2u * k * M), a),
+                                   __ldg(s + (1u + j) * M * M + 2u * k * M), b));
+            }
+        }
     };
 #pragma unroll 1
     for (uint32_t p0 = 0; p0 < (uint32_t)ND; p0 += PL) {
-        float2* stage = sm + p0 * SLOT;  // [plane][component][z][ky], rows of M + 1
-        {
-            const uint32_t kx = p0 + pl;
-            auto half_line = [&](uint32_t par, C2<float>(&v)[ND]) {  // kz = par, par + 2, ...
+        float2* stage = sm + p0 * SLOT;  // [plane][z][ky], rows of M + 1
+        C2<float> v[ND];
+        gather(p0 + pl, v, [](C2<float>& d, const C2<float> p) { d = p; });
+        // the transforms of kx = 0 and kx = nd are real: one complex line holds both
+        if (p0 + pl == 0u) gather(ND, v, [](C2<float>& d, const C2<float> p) { d = {d.x - p.y, d.y + p.x}; });
+        fft_pair<ND>(v, par != 0u);
+        float2* w = stage + (pl * ND + par * (ND / 2u)) * ROW + ky;
 #pragma unroll
-                for (uint32_t k = 0; k < (uint32_t)ND; k++) v[k] = product(kx, 2u * k + par);
-                if (kx == 0u) {  // the transforms of kx = 0 and kx = nd are real: one complex line holds both
-#pragma unroll
-                    for (uint32_t k = 0; k < (uint32_t)ND; k++) {
-                        const C2<float> a = product(ND, 2u * k + par);
-                        v[k] = {v[k].x - a.y, v[k].y + a.x};
-                    }
-                }
-                fft_regs<ND, 1>(v);
-            };
-            C2<float> e[ND], d[ND];
-            half_line(0u, e);
-            half_line(1u, d);
-            fft_join<ND, 1>(e, d);
-            float2* w = stage + (pl * 3u + f) * ND * ROW + ky;
-#pragma unroll
-            for (uint32_t z = 0; z < (uint32_t)ND; z++) w[z * ROW] = make_float2(e[z].x, e[z].y);
-        }
+        for (uint32_t n = 0; n < (uint32_t)ND / 2u; n++) w[n * ROW] = make_float2(v[n].x, v[n].y);
         __syncthreads();
-        C2<float> e[ND], d[ND];
-        const uint32_t line = t;  // (plane, component, z)
-        const uint32_t z = line % ND;
-        if (line < PL * 3u * ND) {
-            const float2* r = stage + line * ROW;
+        const bool on = id < PL * ND;  // line along y: (plane, z)
+        if (on) {
+            const float2* r = stage + id * ROW + par;
 #pragma unroll
-            for (uint32_t k = 0; k < (uint32_t)ND; k++) {
-                const float2 a = r[2u * k], b = r[2u * k + 1u];
-                e[k] = {a.x, a.y};
-                d[k] = {b.x, b.y};
-            }
-            fft_half<ND, 1>(e, d);
+            for (uint32_t k = 0; k < (uint32_t)ND; k++) v[k] = {r[2u * k].x, r[2u * k].y};
+            fft_pair<ND>(v, par != 0u);
         }
         __syncthreads();  // the staged lines are read: the slots below them may be written
-        if (line < PL * 3u * ND) {
-            // slot [component][z][(y + z) mod nd]: rows of nd without bank conflicts
-            float2* w = sm + (p0 + line / (3u * ND)) * SLOT + (line / ND % 3u * ND + z) * ND;
+        if (on) {
+            // slot [z][(y + z) mod nd]: rows of nd without bank conflicts
+            const uint32_t z = id % ND;
+            float2* q = sm + (p0 + id / ND) * SLOT + z * ND;
 #pragma unroll
-            for (uint32_t y = 0; y < (uint32_t)ND; y++) w[(y + z) % ND] = make_float2(e[y].x, e[y].y);
+            for (uint32_t n = 0; n < (uint32_t)ND / 2u; n++)
+                q[(n + par * (ND / 2u) + z) % ND] = make_float2(v[n].x, v[n].y);
         }
     }
     __syncthreads();
     // along x, real outputs: with X_k the line's transform and h = nd, z_k = (X_k + conj X_{h-k})
     // + i w^k (X_k - conj X_{h-k}) transforms to (x_0 + i x_1, x_2 + i x_3, ...)
-    const uint32_t noz = F.chunk;
     for (uint32_t line = t; line < SLOT; line += SUM_THREADS) {
-        const uint32_t y = line % ND, z = line / ND % ND, c = line / (ND * ND);
-        const float2* r = sm + (c * ND + z) * ND + (y + z) % ND;
+        const uint32_t y = line % ND, z = line / ND;
+        const float2* r = sm + z * ND + (y + z) % ND;
         C2<float> v[ND];
-        const float2 r0 = r[0];
-        v[0] = {r0.x + r0.y, r0.x - r0.y};
-        float2 X[ND];
+        v[0] = {r[0].x + r[0].y, r[0].x - r[0].y};
 #pragma unroll
-        for (uint32_t k = 1; k < (uint32_t)ND; k++) X[k] = r[k * SLOT];
-#pragma unroll
-        for (uint32_t k = 1; k < (uint32_t)ND; k++) {
-            const float2 p = X[k], q = X[ND - k];
-            const C2<float> dif = twist<1>(C2<float>{p.x - q.x, p.y + q.y}, k * (16 / ND) + 8);  // times i w^k
-            v[k] = {(p.x + q.x) + dif.x, (p.y - q.y) + dif.y};
+        for (uint32_t k = 1; k <= (uint32_t)ND / 2u; k++) {
+            const float2 p = r[k * SLOT], q = r[(ND - k) * SLOT];
+            const C2<float> sum = {p.x + q.x, p.y - q.y}, dif = {p.x - q.x, p.y + q.y};
+            const C2<float> a = twist<1>(dif, k * (16 / ND) + 8);  // i w^k dif
+            v[k] = {sum.x + a.x, sum.y + a.y};
+            // k -> h - k: sum -> conj sum, dif -> -conj dif, i w^k -> conj (i w^k)
+            if (2u * k < (uint32_t)ND) v[ND - k] = {sum.x - a.x, a.y - sum.y};
         }
         fft_regs<ND, 1>(v);
         constexpr float scale = 1.0f / (float)(M * M * M);  // a power of two: exact
-        float* out = F.out + (((((size_t)(group * 3u + c) * noz * L.bsy * L.bsx) + o) * ND) * ND + z) * ND + y;
+        const float w = negative(field < 3u ? f : j) ? -scale : scale;
+        float* out = F.out + (((size_t)field * F.chunk * L.bsy * L.bsx + o) * ND * ND + z) * ND + y;
 #pragma unroll
         for (uint32_t n = 0; n < (uint32_t)ND / 2u; n++) {
-            out[(2u * n) * ND * ND] = v[n].x * scale;
-            out[(2u * n + 1u) * ND * ND] = v[n].y * scale;
+            out[(2u * n) * ND * ND] = v[n].x * w;
+            out[(2u * n + 1u) * ND * ND] = v[n].y * w;
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// the sums to the cells: block = component + 6 (x tile + tiles (Iz + nd (oy + bsy (oz - oz0))));
-// a block transposes nd rows (y = Iy bsy + oy) of up to PUT_X cells through shared memory
+// the sums to the cells: block = (0: E, 1: B) + 2 (x tile + tiles (Iz + nd (oy + bsy (oz - oz0))));
+// a block transposes nd rows (y = Iy bsy + oy) of up to PUT_X cells, three components,
+// through shared memory.  A thread's loads are all in flight before the first is used, and the
+// components share its indices (one component a block, loads one after another: 55 us at 128^3)
 // ---------------------------------------------------------------------------
 template <int ND>
 __device__ __forceinline__ void fft_put(const DevLbm& L, const FftField& F, uint32_t block, const uint32_t oz0) {
-    __shared__ float s[ND][PUT_X + 1];
+    __shared__ float s[3][ND][PUT_X + 1];
     const uint32_t tiles = (L.nx + PUT_X - 1u) / PUT_X;
-    const uint32_t c = block % 6u;
-    block /= 6u;
+    const bool B = block & 1u;
+    block >>= 1;
     const uint32_t x0 = block % tiles * PUT_X;
     block /= tiles;
     const uint32_t Iz = block % ND, oy = block / ND % L.bsy, ozl = block / (ND * L.bsy);
     const uint32_t cnt = min(PUT_X, L.nx - x0);
-    const float* in = F.out + (((size_t)(c * F.chunk + ozl) * L.bsy + oy) * L.bsx) * (ND * ND * ND) + Iz * ND;
-    for (uint32_t t = threadIdx.x; t < cnt * ND; t += PUT_THREADS) {
-        const uint32_t Iy = t % ND, xl = t / ND, x = x0 + xl, Ix = x / L.bsx, ox = x - Ix * L.bsx;
-        s[Iy][xl] = in[(size_t)(ox * ND + Ix) * (ND * ND) + Iy];
+    const size_t N = L.n, plane = (size_t)F.chunk * L.bsy * L.bsx * (ND * ND * ND);
+    const float* in = F.out + (B ? 3u : 0u) * plane + ((size_t)ozl * L.bsy + oy) * L.bsx * (ND * ND * ND) + Iz * ND;
+    const uint32_t Iy = threadIdx.x % ND;
+    constexpr uint32_t XS = PUT_THREADS / ND, GET = PUT_X / XS;  // cells apart, cells per thread
+    float v[3][GET];
+#pragma unroll
+    for (uint32_t k = 0; k < GET; k++) {
+        const uint32_t xl = threadIdx.x / ND + k * XS, x = x0 + xl, Ix = x / L.bsx, ox = x - Ix * L.bsx;
+        const float* p = in + (size_t)(ox * ND + Ix) * (ND * ND) + Iy;
+#pragma unroll
+        for (uint32_t c = 0; c < 3; c++) v[c][k] = xl < cnt ? __ldcs(p + c * plane) : 0.0f;
     }
-    __syncthreads();
     const uint32_t z = Iz * L.bsz + oz0 + ozl;
-    const size_t N = L.n;
-    const uint32_t k = c < 3u ? c : c - 3u;
-    const float* stat = (c < 3u ? L.e_stat : L.b_stat) + k * N;
-    float* dyn = (c < 3u ? L.e_dyn : L.b_dyn) + k * N;
-    const float scale = c < 3u ? L.ke : L.kmu;
-    for (uint32_t t = threadIdx.x; t < PUT_X * ND; t += PUT_THREADS) {
-        const uint32_t xl = t % PUT_X, Iy = t / PUT_X;
-        if (xl >= cnt) continue;
-        const uint32_t n = x0 + xl + ((Iy * L.bsy + oy) + z * L.ny) * L.nx;
-        if ((L.flags[n] & F_BO) != F_S) dyn[n] = stat[n] + scale * s[Iy][xl];
+    constexpr uint32_t PUT = PUT_X * ND / PUT_THREADS, YS = PUT_THREADS / PUT_X;
+    const uint32_t xl = threadIdx.x % PUT_X, y0 = threadIdx.x / PUT_X;
+    const uint32_t n0 = x0 + xl + (oy + y0 * L.bsy + z * L.ny) * L.nx, row = YS * L.bsy * L.nx;
+    const float* const stat = B ? L.b_stat : L.e_stat;
+    float* const dyn = B ? L.b_dyn : L.e_dyn;
+    const float scale = B ? L.kmu : L.ke;
+    bool on[PUT];
+#pragma unroll
+    for (uint32_t k = 0; k < PUT; k++) on[k] = xl < cnt && (L.flags[n0 + k * row] & F_BO) != F_S;
+#pragma unroll
+    for (uint32_t c = 0; c < 3; c++)
+#pragma unroll
+        for (uint32_t k = 0; k < GET; k++) s[c][Iy][threadIdx.x / ND + k * XS] = v[c][k];
+    __syncthreads();
+#pragma unroll
+    for (uint32_t c = 0; c < 3; c++) {
+        float st[PUT];
+#pragma unroll
+        for (uint32_t k = 0; k < PUT; k++) st[k] = on[k] ? stat[c * N + n0 + k * row] : 0.0f;
+#pragma unroll
+        for (uint32_t k = 0; k < PUT; k++)
+            if (on[k]) dyn[c * N + n0 + k * row] = st[k] + scale * s[c][y0 + k * YS][xl];
     }
 }
 
@@ -353,7 +391,7 @@ __global__ void __launch_bounds__(SRC_THREADS) k_fft_src(const DevLbm L, const F
     fft_src<ND>(L, F, blockIdx.x);
 }
 template <int ND>
-__global__ void __launch_bounds__(SUM_THREADS, 2) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0) {
+__global__ void __launch_bounds__(SUM_THREADS, SUM_BLOCKS) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0) {
     extern __shared__ __align__(16) float2 sum_sm[];
     if (*F.direct) return;
     fft_sum<ND>(L, F, blockIdx.x, oz0, sum_sm);
@@ -395,7 +433,7 @@ __global__ void __launch_bounds__(SRC_THREADS) k_fft_src_batch(const FftBatch B)
     fft_src<ND>(L, F, block);
 }
 template <int ND>
-__global__ void __launch_bounds__(SUM_THREADS, 2) k_fft_sum_batch(const FftBatch B, const uint32_t pass) {
+__global__ void __launch_bounds__(SUM_THREADS, SUM_BLOCKS) k_fft_sum_batch(const FftBatch B, const uint32_t pass) {
     extern __shared__ __align__(16) float2 sum_sm[];
     __shared__ DevLbm L;
     __shared__ FftField F;
@@ -487,10 +525,10 @@ cudaError_t launch_fft_plan(const DevLbm& L, const FftField& F, cudaStream_t s) 
 uint32_t fft_passes(const DevLbm& L, const FftField& F) { return (L.bsz + F.chunk - 1u) / F.chunk; }
 uint32_t fft_src_blocks(const DevLbm& L) { return 4u * (L.nd + 1u); }
 uint32_t fft_sum_blocks(const DevLbm& L, const FftField& F, uint32_t pass) {
-    return 2u * chunk_len(L, F, pass) * L.bsy * L.bsx;
+    return 6u * chunk_len(L, F, pass) * L.bsy * L.bsx;
 }
 uint32_t fft_put_blocks(const DevLbm& L, const FftField& F, uint32_t pass) {
-    return 6u * ((L.nx + PUT_X - 1u) / PUT_X) * L.nd * L.bsy * chunk_len(L, F, pass);
+    return 2u * ((L.nx + PUT_X - 1u) / PUT_X) * L.nd * L.bsy * chunk_len(L, F, pass);
 }
 
 uint32_t launch_fft_batch(const FftBatch* B, uint32_t passes, cudaStream_t s) {
