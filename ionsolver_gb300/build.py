@@ -24,7 +24,7 @@ LIB = OUT / "libionsolver.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false",
               "-Xcompiler", "-fPIC,-ffp-contract=off", "-Xptxas", "-v", f"-I{REPO / 'include'}", f"-I{CSRC}"]
-SOURCES = ["lbm_q19.cu", "lbm_q15.cu", "lbm_q9.cu", "field_kernels.cu", "field_fft.cu", "setup_kernels.cu", "batch_kernels.cu",
+SOURCES = ["lbm_q19.cu", "lbm_q15.cu", "lbm_q9.cu", "field_kernels.cu", "field_fft.cu", "field_table.cu", "setup_kernels.cu", "batch_kernels.cu",
            "noalloc.cu", "surrogate.cu", "config_json.cpp", "ion_api.cu"]
 # (source, object name, extra flags): one translation unit compiled more than once
 VARIANTS = [("lbm_q19_sc.cu", f"lbm_q19_sc_{ft.lower()}", [f"-DION_SC_FT=ION_{ft}"]) for ft in ("FP32", "FP16S", "FP16C")]

@@ -1,0 +1,160 @@
+// field_table.cu -- the BITWISE E/B field with R/|R|^3 from a table.
+//
+// Cell and bin coordinates are integers and halves, so R of a cell and a bin is exact and
+// depends only on the bins' difference and the cell's offset in its bin, and so do the three
+// quotients R/|R|^3 (IEEE sqrt and divides) that are most of eb_tile<false>'s work: 36 of its
+// 57 operations per term.  Here they are computed once per grid shape, with the operations of
+// add_src<false>, for every |2 R| (a sign passes through all of them unchanged), 16 bytes per
+// distance, about as many as cells.  A term's other 21 operations and the order of the sums
+// are those of eb_tile<false>: the field is bit-identical to it.
+//
+// A thread holds the cells of one in-bin offset in R neighbouring bins along x.  Along a row
+// of source bins every step needs one new table entry, the others move on by a cell: R + nd - 1
+// entries per row of nd sources and R cells.  Lanes are neighbouring offsets (coalesced table
+// rows, one broadcast source), the warps of a block the R-groups of the same offsets, whose
+// entries overlap in L1.  Bound by FP32 issue: 21 of 24 instructions per term.
+#include "field_table.h"
+#include "ion_device.cuh"
+#include "ion_launch.h"
+
+namespace ion {
+
+namespace {
+
+// |2 R| along an axis has the parity of the bin edge: entry a >> 1 holds a = |2 R|
+__global__ void __launch_bounds__(256) k_field_table(const DevLbm L, const FieldTable F) {
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+    if (x >= F.tx) return;
+    const float rx = 0.5f * (float)(2u * x + (L.bsx & 1u)), ry = 0.5f * (float)(2u * y + (L.bsy & 1u)),
+                rz = 0.5f * (float)(2u * z + (L.bsz & 1u));
+    float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (rx != 0.0f || ry != 0.0f || rz != 0.0f) {  // R = 0 only in the own bin, which is skipped
+        const float s = sqrtf((rx * rx + ry * ry) + rz * rz);
+        const float c3 = (s * s) * s;
+        const float r = __frcp_rn(c3);
+        p = make_float4(div_rn_shared(rx, c3, r), div_rn_shared(ry, c3, r), div_rn_shared(rz, c3, r), 0.0f);
+    }
+    F.T[((size_t)z * F.ty + y) * F.tx + x] = p;
+}
+
+struct P3 { float x, y, z; };
+
+__device__ __forceinline__ void add_term(const P3& p, const float4& v, float (&e)[3], float (&b)[3]) {
+    e[0] = e[0] + v.x * p.x; e[1] = e[1] + v.x * p.y; e[2] = e[2] + v.x * p.z;
+    const float bx = v.z * p.z - v.w * p.y, by = v.w * p.x - v.y * p.z, bz = v.y * p.y - v.z * p.x;
+    b[0] = b[0] + v.x * bx; b[1] = b[1] + v.x * by; b[2] = b[2] + v.x * bz;
+}
+
+template <int ND, int R, int EB>
+__global__ void __launch_bounds__(EB * (ND / R), 512 / (EB * (ND / R))) k_update_e_b_table(const DevLbm L, const FieldTable F) {
+    constexpr uint32_t THREADS = EB * (ND / R);
+    __shared__ float4 src[ND * ND];  // one z plane of sources: (q, vx, vy, vz)
+    const uint32_t no = L.bsx * L.bsy * L.bsz;
+    const uint32_t item = blockIdx.x * EB + threadIdx.x % EB;  // (Iz, Iy, offset)
+    const bool valid = item < no * (ND * ND);
+    const uint32_t i0 = threadIdx.x / EB * R;
+    const uint32_t it = valid ? item : 0u;
+    const uint32_t o = it % no, iy = it / no % ND, iz = it / (no * ND);
+    const uint32_t ox = o % L.bsx, oy = o / L.bsx % L.bsy, oz = o / (L.bsx * L.bsy);
+    const int ax0 = (int)(2u * (L.bsx * i0 + ox)) - (int)L.bsx;  // 2 R_x of cell 0 and source 0
+    const int first = (int)L.first_src, last = (int)min(L.n_lod_own, L.n_bins);
+    float e[R][3], b[R][3];
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) { e[i][c] = 0.0f; b[i][c] = 0.0f; }
+    for (int jz = first / (ND * ND); jz < ND; jz++) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < ND * ND; k += THREADS)
+            src[k] = reinterpret_cast<const float4*>(L.qu_lod)[jz * (ND * ND) + k];
+        __syncthreads();
+        const int az = (int)(2u * (L.bsz * iz + oz)) - (int)L.bsz - 2 * (int)L.bsz * jz;
+        const uint32_t sz = (uint32_t)az & 0x80000000u;
+#pragma unroll 1
+        for (int jy = 0; jy < ND; jy++) {
+            const int d0 = (jz * ND + jy) * ND;
+            if (d0 + ND <= first || d0 >= last) continue;
+            const int ay = (int)(2u * (L.bsy * iy + oy)) - (int)L.bsy - 2 * (int)L.bsy * jy;
+            const uint32_t sy = (uint32_t)ay & 0x80000000u;
+            const float4* row = F.T + ((size_t)((uint32_t)abs(az) >> 1) * F.ty + ((uint32_t)abs(ay) >> 1)) * F.tx;
+            auto entry = [&](int ax) -> P3 {
+                const float4 t = __ldg(row + ((uint32_t)abs(ax) >> 1));
+                return {__uint_as_float(__float_as_uint(t.x) ^ ((uint32_t)ax & 0x80000000u)),
+                        __uint_as_float(__float_as_uint(t.y) ^ sy), __uint_as_float(__float_as_uint(t.z) ^ sz)};
+            };
+            int step = 2 * (int)L.bsx;
+            asm volatile("" : "+r"(step));  // the entries' indices are formed per row, not kept
+            const bool own_row = (uint32_t)jy == iy && (uint32_t)jz == iz;
+            if (d0 >= first && d0 + ND <= last && !__any_sync(0xFFFFFFFFu, own_row)) {
+                P3 p[R + ND - 1];  // entry k: bins R - 1 - k apart
+#pragma unroll
+                for (int k = 0; k < R - 1; k++) p[k] = entry(ax0 + (R - 1 - k) * step);
+#pragma unroll
+                for (int j = 0; j < ND; j++) {
+                    p[R - 1 + j] = entry(ax0 - j * step);
+                    const float4 v = src[jy * ND + j];
+#pragma unroll
+                    for (int i = 0; i < R; i++) add_term(p[R - 1 - i + j], v, e[i], b[i]);
+                }
+            } else {  // a row with a lane's own bin, or the first row (which starts inside a row)
+#pragma unroll 1
+                for (int j = max(first - d0, 0); j < min(last - d0, ND); j++) {
+                    const float4 v = src[jy * ND + j];
+#pragma unroll
+                    for (int i = 0; i < R; i++)
+                        if (!own_row || (int)i0 + i != j) add_term(entry(ax0 + (i - j) * step), v, e[i], b[i]);
+                }
+            }
+        }
+    }
+    if (!valid) return;
+    const size_t N = L.n;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const uint32_t n = (i0 + i) * L.bsx + ox + ((iy * L.bsy + oy) + (iz * L.bsz + oz) * L.ny) * L.nx;
+        if ((L.flags[n] & F_BO) == F_S) continue;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            L.e_dyn[c * N + n] = L.e_stat[c * N + n] + L.ke * e[i][c];
+            L.b_dyn[c * N + n] = L.b_stat[c * N + n] + L.kmu * b[i][c];
+        }
+    }
+}
+
+template <int ND, int R, int EB>
+cudaError_t launch(const DevLbm& L, const FieldTable& F, cudaStream_t s) {
+    const uint64_t items = (uint64_t)(L.n / ND);  // cells over the bins along x
+    k_update_e_b_table<ND, R, EB><<<(unsigned)((items + EB - 1) / EB), EB * (ND / R), 0, s>>>(L, F);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+// Depths 3 and 4 without cells of the reference's near field; edges below 2^16 cells keep 2 R
+// in 32 bits and every coordinate exact.
+bool field_table_fits(const DevLbm& L) {
+    return (L.nd == 8u || L.nd == 16u) && L.near_x == 1u && L.near_y == 1u && L.near_z == 1u && L.nx < 65536u &&
+           L.ny < 65536u && L.nz < 65536u;
+}
+
+size_t field_table_size(const DevLbm& L, FieldTable& F) {
+    F.tx = (2u * L.nx - L.bsx) / 2u + 1u;  // the largest |2 R| is 2 n - b
+    F.ty = (2u * L.ny - L.bsy) / 2u + 1u;
+    F.tz = (2u * L.nz - L.bsz) / 2u + 1u;
+    return (size_t)F.tx * F.ty * F.tz * sizeof(float4);
+}
+
+cudaError_t launch_field_table(const DevLbm& L, const FieldTable& F, cudaStream_t s) {
+    k_field_table<<<dim3((F.tx + 255u) / 256u, F.ty, F.tz), 256, 0, s>>>(L, F);
+    return cudaGetLastError();
+}
+
+// Four cells a thread amortise the table entries and the source best (24 against 26 instructions
+// a term); below 2^18 cells two cells a thread keep more of the SMs' schedulers supplied.
+cudaError_t launch_update_e_b_table(const DevLbm& L, const FieldTable& F, cudaStream_t s) {
+    const bool wide = L.n >= (1u << 18);
+    if (L.nd == 16u) return wide ? launch<16, 4, 64>(L, F, s) : launch<16, 2, 16>(L, F, s);
+    return wide ? launch<8, 4, 64>(L, F, s) : launch<8, 2, 32>(L, F, s);
+}
+
+}  // namespace ion

@@ -21,6 +21,7 @@
 
 #include "ion_device.cuh"
 #include "field_fft.h"
+#include "field_table.h"
 #include "ion_launch.h"
 #include "surrogate.h"
 
@@ -202,6 +203,7 @@ struct ion_lbm {
     std::vector<void*> allocs;
     std::unique_ptr<ion::Surrogate> sur;  // learned far field (field_mode SURROGATE)
     ion::FftField fft;         // FAST field as a convolution over the bins; fft.G null: the direct sum
+    ion::FieldTable table;     // BITWISE field: R/|R|^3 of the grid; table.T null: the direct sum
 };
 
 namespace {
@@ -247,11 +249,24 @@ int launch_stream_collide(ion_lbm* h, uint64_t t) {
     return ION_OK;
 }
 
-// Lays out the FAST field's convolution for a handle (once; launches work on the handle's
-// stream and allocates, so it runs when a handle is created or switched to FAST, never inside
-// a step).  Where the device has no memory left for it the direct sum stays.
-int setup_fft(ion_lbm* h) {
-    if (h->fft.G || h->cfg.field_mode != ION_FIELD_FAST || !h->cfg.ext_magneto_hydro || !fft_field_fits(h->L)) return ION_OK;
+// Lays out what a handle's field mode keeps per grid shape, the FAST field's convolution or the
+// BITWISE field's table (once; launches work on the handle's stream and allocates, so it runs
+// when a handle is created or switched to a mode, never inside a step).  Where the device has
+// no memory left for it the direct sum stays.
+int setup_field(ion_lbm* h) {
+    if (!h->cfg.ext_magneto_hydro) return ION_OK;
+    if (h->cfg.field_mode == ION_FIELD_BITWISE && !h->table.T && field_table_fits(h->L)) {
+        FieldTable T;
+        if (cudaMalloc((void**)&T.T, field_table_size(h->L, T)) != cudaSuccess) {
+            cudaGetLastError();
+            return ION_OK;
+        }
+        h->allocs.push_back(T.T);
+        CK(launch_field_table(h->L, T, h->stream));
+        g_launches++;
+        h->table = T;
+    }
+    if (h->fft.G || h->cfg.field_mode != ION_FIELD_FAST || !fft_field_fits(h->L)) return ION_OK;
     FftField F;
     size_t bytes[4] = {0, 0, 0, 4};
     fft_field_sizes(h->L, F, &bytes[0], &bytes[1], &bytes[2]);
@@ -276,6 +291,11 @@ int launch_field(ion_lbm* h) {
         g_launches += launch_fft_field(h->L, h->fft, h->stream) + 1;
         launch_update_e_b_gated(h->L, h->d_err, h->fft.direct, h->stream);
         CKL();
+        return ION_OK;
+    }
+    if (h->cfg.field_mode == ION_FIELD_BITWISE && h->table.T) {
+        CK(launch_update_e_b_table(h->L, h->table, h->stream));
+        g_launches++;
         return ION_OK;
     }
     // the exact sum; SURROGATE handles use its FAST arithmetic outside the surrogate path
@@ -595,7 +615,7 @@ int ion_lbm_create(const ion_config* cfg, ion_lbm** out) {
             return fail(ION_E_CUDA, "upload of LOD centres failed");
         }
     }
-    rc = setup_fft(h);
+    rc = setup_field(h);
     if (rc) { destroy_handle(h); return rc; }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) { destroy_handle(h); return fail(ION_E_CUDA, "create: stream sync failed"); }
     for (auto& e : h->ev) cudaEventCreate(&e);
@@ -1793,7 +1813,7 @@ int ion_lbm_set_field_mode(ion_lbm* h, int mode) {
     }
     h->cfg.field_mode = (uint8_t)mode;
     h->graph_dirty = true;
-    return setup_fft(h);
+    return setup_field(h);
 }
 
 // ---- device selection and the FP32 peak probe ---------------------------------
