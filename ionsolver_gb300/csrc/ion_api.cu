@@ -165,6 +165,8 @@ struct HostMesh {
     }
 };
 
+constexpr size_t PSI_KEEP = 64ull << 20;
+
 struct KEv {
     int kernel;
     cudaEvent_t a, b;
@@ -188,6 +190,8 @@ struct ion_lbm {
     uint32_t* d_tiles = nullptr;
     uint32_t* d_list = nullptr;
     uint32_t* d_count = nullptr;
+    void* psi_ws = nullptr;  // terms and runs of the magnets' potential (kept up to PSI_KEEP bytes)
+    size_t psi_ws_bytes = 0;
     float *d_p0 = nullptr, *d_p1 = nullptr, *d_p2 = nullptr;
     size_t tri_cap = 0;
     std::vector<HostMesh> meshes;
@@ -227,6 +231,7 @@ void destroy_handle(ion_lbm* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     for (void* p : h->allocs) cudaFree(p);
+    cudaFree(h->psi_ws);
     for (auto& e : h->ev) if (e) cudaEventDestroy(e);
     for (auto& e : h->kev) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
     for (auto e : h->ev_pool) cudaEventDestroy(e);
@@ -950,6 +955,41 @@ static int ensure_compaction(ion_lbm* h) {
     return ION_OK;
 }
 
+// The tabulated form of the magnets' potential (P.T null: the direct sum runs): the runs of the
+// compacted list, read back for the table's size, and the table's memory.  The part of E_dyn
+// that the potential will overwrite holds the runs (8 bytes each) until their number is known.  Below 64 cells the direct sum costs less than the table.
+static int psi_table(ion_lbm* h, PsiTable& P, uint32_t& kinds) {
+    if (h->L.n >= 1u << 30) return ION_OK;  // a run keeps its magnetisation in the index's top bits
+    uint2* const runs = (uint2*)h->L.e_dyn;
+    PsiInfo* const d_info = (PsiInfo*)h->d_partials;
+    PsiInfo info;
+    const size_t npsi = (size_t)(h->L.nx + 2) * (h->L.ny + 2) * (h->L.nz + 2);
+    launch_psi_runs(h->L, h->d_list, h->d_count, runs, (uint32_t)(npsi / 2 - 1), d_info, h->stream);
+    g_launches++;
+    CKL();
+    CK(cudaMemcpyAsync(&info, d_info, sizeof info, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    if (info.count < 64u || info.kinds > PSI_KINDS) return ION_OK;
+    const size_t bytes = psi_table_size(h->L, info, P), run_bytes = sizeof(uint2) * ((size_t)info.runs + 1);
+    const size_t at = (bytes + 255) / 256 * 256;
+    if (P.tx > 65535u || (uint64_t)P.tz * info.kinds > 65535u) return ION_OK;
+    if (h->psi_ws_bytes < at + run_bytes) {
+        cudaFree(h->psi_ws);
+        h->psi_ws_bytes = 0;
+        if (cudaMalloc(&h->psi_ws, at + run_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            h->psi_ws = nullptr;
+            return ION_OK;
+        }
+        h->psi_ws_bytes = at + run_bytes;
+    }
+    P.runs = (const uint2*)((char*)h->psi_ws + at);
+    CK(cudaMemcpyAsync((void*)P.runs, runs, run_bytes, cudaMemcpyDeviceToDevice, h->stream));
+    P.T = (float*)h->psi_ws;
+    kinds = info.kinds;
+    return ION_OK;
+}
+
 int ion_lbm_precompute_b(ion_lbm* h) {
     if (!h) return fail(ION_E_INVALID, "null handle");
     if (!h->cfg.ext_magneto_hydro) return fail(ION_E_STATE, "precompute_b needs ext_magneto_hydro");
@@ -957,10 +997,24 @@ int ion_lbm_precompute_b(ion_lbm* h) {
     if (rc) return rc;
     launch_compact(h->L, F_M, h->d_tiles, h->d_list, h->d_count, h->stream);
     g_launches += 3;
-    launch_psi_static_b(h->L, h->d_list, h->d_count, h->stream);
-    g_launches += 2;
+    PsiTable P{};
+    uint32_t kinds = 0;
+    rc = psi_table(h, P, kinds);
+    if (rc) return rc;
+    if (P.T) {
+        launch_psi_table_static_b(h->L, P, kinds, h->stream);
+        g_launches += 3;
+    } else {
+        launch_psi_static_b(h->L, h->d_list, h->d_count, h->stream);
+        g_launches += 2;
+    }
     CKL();
     CK(cudaStreamSynchronize(h->stream));
+    if (h->psi_ws_bytes > PSI_KEEP) {
+        cudaFree(h->psi_ws);
+        h->psi_ws = nullptr;
+        h->psi_ws_bytes = 0;
+    }
     return ION_OK;
 }
 

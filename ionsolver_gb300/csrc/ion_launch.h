@@ -23,6 +23,21 @@ struct VoxArgs {
     float mx, my, mz;
 };
 
+// a list of magnet cells as runs along x (setup_kernels.cu, k_psi_runs)
+constexpr uint32_t PSI_KINDS = 4;  // distinct magnetisations with a table of their own
+struct PsiInfo {
+    uint32_t count, runs, kinds;   // kinds > PSI_KINDS: not tabulated
+    uint32_t lo[3], hi[3];         // bounds of the cells
+    float m[PSI_KINDS][3];
+};
+struct PsiTable {
+    float* T;
+    const uint2* runs;
+    uint32_t nruns, tx, ty, tz;    // T is [kind][z][x][y]
+    int x0, y0, z0;                // the first differences
+    float m[PSI_KINDS][3];
+};
+
 constexpr unsigned RED_BLOCK = 256;
 
 // Cells per thread of the E/B update: each staged source is applied to
@@ -86,6 +101,11 @@ void launch_update_e_b_gated(const DevLbm& L, uint32_t* err, const uint32_t* gat
 void launch_voxelize(const DevLbm& L, const VoxArgs& A, cudaStream_t s);
 void launch_compact(const DevLbm& L, uint8_t mask, uint32_t* tiles, uint32_t* list, uint32_t* total, cudaStream_t s);
 void launch_psi_static_b(const DevLbm& L, const uint32_t* mags, const uint32_t* count, cudaStream_t s);
+// runs of the list; the table's size for them; the table, the potential and the static field
+void launch_psi_runs(const DevLbm& L, const uint32_t* list, const uint32_t* count, uint2* runs, uint32_t max_runs,
+                     PsiInfo* info, cudaStream_t s);
+size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P);
+void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, cudaStream_t s);
 void launch_static_e(const DevLbm& L, const uint32_t* list, const uint32_t* count, float* E, cudaStream_t s);
 void launch_sum_f64(const void* x, int ft, uint64_t count, double* partials, uint32_t nparts, double* out,
                     cudaStream_t s);

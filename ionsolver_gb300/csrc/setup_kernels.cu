@@ -1,6 +1,6 @@
 // setup_kernels.cu -- geometry and static-field kernels, FP64 reductions.
 //
-//   voxelize  : IonSolver src/kernels/sim_kernels.cl:1150-1231 (one thread
+//   voxelize  : IonSolver src/kernels/sim_kernels.cl:1150-1231 (one warp
 //               per bounding-box column, Moeller-Trumbore in both ray
 //               directions, 16-bit hit distances, parity with correction).
 //   psi / B   : sim_kernels.cl:1234-1276.  The reference loops over all N
@@ -25,8 +25,15 @@ __device__ __forceinline__ V3 vcross(V3 a, V3 b) { return {a.y * b.z - a.z * b.y
 __device__ __forceinline__ float vdot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ int iclamp(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
-__global__ void __launch_bounds__(128) k_voxelize(const DevLbm L, VoxArgs A) {
-    const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per column: the lanes take the triangles side by side and file their hits in triangle
+// order (a thread per column left most SMs with a few warps, each waiting on one triangle's
+// divide after another: 150 us for 128 triangles at 128^3).
+constexpr uint32_t VOX_WARPS = 4, VOX_HITS = 64;
+
+__global__ void __launch_bounds__(VOX_WARPS * 32) k_voxelize(const DevLbm L, VoxArgs A) {
+    __shared__ uint16_t s_dist[VOX_WARPS][VOX_HITS], s_sorted[VOX_WARPS][VOX_HITS];
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t a = blockIdx.x * VOX_WARPS + wid;
     if (a >= A.columns) return;
     const int nx = (int)L.nx, ny = (int)L.ny, nz = (int)L.nz;
     const int dir = A.direction;
@@ -43,59 +50,71 @@ __global__ void __launch_bounds__(128) k_voxelize(const DevLbm L, VoxArgs A) {
     else outside = org.x < A.x0 || org.y < A.y0 || org.x >= A.x1 || org.y >= A.y1;
     if (outside) return;
     const V3 rdir = {(float)(dir == 0), (float)(dir == 1), (float)(dir == 2)};
-    uint16_t dist[64];
-    for (int i = 0; i < 64; i++) dist[i] = 0;
+    uint16_t* const dist = s_dist[wid];
+    uint16_t* const sorted = s_sorted[wid];
+    for (uint32_t i = lane; i < VOX_HITS; i += 32u) dist[i] = sorted[i] = 0;
+    __syncwarp();
     uint32_t hits = 0, back = 0;
-    for (uint32_t i = 0; i < A.ntri; i++) {
-        const V3 P0 = {A.p0[3 * i], A.p0[3 * i + 1], A.p0[3 * i + 2]};
-        const V3 P1 = {A.p1[3 * i], A.p1[3 * i + 1], A.p1[3 * i + 2]};
-        const V3 P2 = {A.p2[3 * i], A.p2[3 * i + 1], A.p2[3 * i + 2]};
-        const V3 e1 = vsub(P1, P0), e2 = vsub(P2, P0), s0 = vsub(org, P0);
-        const V3 pv = vcross(rdir, e2), qv = vcross(s0, e1);
-        const float inv = 1.0f / vdot(e1, pv);
-        const float su = inv * vdot(s0, pv), sv = inv * vdot(rdir, qv), sd = inv * vdot(e2, qv);
-        if (su >= 0.0f && su < 1.0f && sv >= 0.0f && su + sv < 1.0f) {
-            if (sd > 0.0f) {
-                if (hits < 64u && sd < 65536.0f) dist[hits] = (uint16_t)sd;
-                hits++;
-            } else {
-                back++;
-            }
+    for (uint32_t base = 0; base < A.ntri; base += 32u) {
+        const uint32_t i = base + lane;
+        bool hit = false;
+        float sd = 0.0f;
+        if (i < A.ntri) {
+            const V3 P0 = {A.p0[3 * i], A.p0[3 * i + 1], A.p0[3 * i + 2]};
+            const V3 P1 = {A.p1[3 * i], A.p1[3 * i + 1], A.p1[3 * i + 2]};
+            const V3 P2 = {A.p2[3 * i], A.p2[3 * i + 1], A.p2[3 * i + 2]};
+            const V3 e1 = vsub(P1, P0), e2 = vsub(P2, P0), s0 = vsub(org, P0);
+            const V3 pv = vcross(rdir, e2), qv = vcross(s0, e1);
+            const float inv = 1.0f / vdot(e1, pv);
+            const float su = inv * vdot(s0, pv), sv = inv * vdot(rdir, qv);
+            sd = inv * vdot(e2, qv);
+            hit = su >= 0.0f && su < 1.0f && sv >= 0.0f && su + sv < 1.0f;
         }
+        const uint32_t ahead = __ballot_sync(0xFFFFFFFFu, hit && sd > 0.0f);
+        back += __popc(__ballot_sync(0xFFFFFFFFu, hit && !(sd > 0.0f)));
+        const uint32_t at = hits + __popc(ahead & ((1u << lane) - 1u));
+        if (hit && sd > 0.0f && at < VOX_HITS && sd < 65536.0f) dist[at] = (uint16_t)sd;
+        hits += __popc(ahead);
     }
-    const uint32_t ns = hits < 64u ? hits : 64u;
-    for (uint32_t i = 1; i < ns; i++) {
+    __syncwarp();
+    const uint32_t ns = hits < VOX_HITS ? hits : VOX_HITS;
+    for (uint32_t i = lane; i < ns; i += 32u) {  // ascending, by rank
         const uint16_t key = dist[i];
-        int k = (int)i - 1;
-        while (k >= 0 && dist[k] > key) { dist[k + 1] = dist[k]; k--; }
-        dist[k + 1] = key;
+        uint32_t rank = 0;
+        for (uint32_t k = 0; k < ns; k++) rank += dist[k] < key || (dist[k] == key && k < i);
+        sorted[rank] = key;
     }
+    __syncwarp();
     bool inside = (hits % 2u) && (back % 2u);
     uint32_t next = (hits % 2u) != (back % 2u);
     const uint32_t h0 = c[dir];
     const uint32_t hmax = dir == 0 ? (uint32_t)iclamp((int)A.x1, 0, nx) : dir == 1 ? (uint32_t)iclamp((int)A.y1, 0, ny)
                                                                                   : (uint32_t)iclamp((int)A.z1, 0, nz);
-    const uint32_t last = hits - 1u < 63u ? hits - 1u : 63u;
-    const uint32_t hmesh = h0 + (uint32_t)dist[last];
+    const uint32_t last = hits - 1u < VOX_HITS - 1u ? hits - 1u : VOX_HITS - 1u;
+    const uint32_t hmesh = h0 + (uint32_t)sorted[last];
     const size_t N = L.n;
-    for (uint32_t hh = h0; hh < hmax; hh++) {
-        while (next < hits && hh > h0 + (uint32_t)dist[next < 63u ? next : 63u]) { inside = !inside; next++; }
-        inside = inside && (next < hits && hh < hmesh);
+    for (uint32_t base = h0; base < hmax; base += 32u) {
+        uint32_t in = 0u;  // the next 32 cells of the column: every lane follows the crossings, then writes its cell
+        for (uint32_t k = 0; k < 32u && base + k < hmax; k++) {
+            const uint32_t hh = base + k;
+            while (next < hits && hh > h0 + (uint32_t)sorted[next < VOX_HITS - 1u ? next : VOX_HITS - 1u]) { inside = !inside; next++; }
+            inside = inside && (next < hits && hh < hmesh);
+            in |= (uint32_t)inside << k;
+        }
+        if (!((in >> lane) & 1u)) continue;
         uint32_t cc[3] = {c[0], c[1], c[2]};
-        cc[dir] = hh;
+        cc[dir] = base + lane;
         const uint32_t n = cc[0] + (cc[1] + cc[2] * L.ny) * L.nx;
-        if (inside) {
-            L.flags[n] = (uint8_t)((L.flags[n] & ~F_BO) | A.flag);
-            if (L.ext_mhd) {
-                if (A.flag & F_M) { L.b_dyn[n] = A.mx; L.b_dyn[N + n] = A.my; L.b_dyn[2 * N + n] = A.mz; }
-                else if ((A.flag & F_F) || (A.flag & F_C)) L.b_dyn[n] = A.mx;
-            }
+        L.flags[n] = (uint8_t)((L.flags[n] & ~F_BO) | A.flag);
+        if (L.ext_mhd) {
+            if (A.flag & F_M) { L.b_dyn[n] = A.mx; L.b_dyn[N + n] = A.my; L.b_dyn[2 * N + n] = A.mz; }
+            else if ((A.flag & F_F) || (A.flag & F_C)) L.b_dyn[n] = A.mx;
         }
     }
 }
 
 void launch_voxelize(const DevLbm& L, const VoxArgs& A, cudaStream_t s) {
-    k_voxelize<<<grid_for(A.columns, 128), 128, 0, s>>>(L, A);
+    k_voxelize<<<grid_for(A.columns, VOX_WARPS), VOX_WARPS * 32, 0, s>>>(L, A);
 }
 
 // ---------------------------------------------------------------------------
@@ -205,6 +224,192 @@ __global__ void __launch_bounds__(256) k_static_b(const DevLbm L, const float* p
     L.b_stat[n] = L.b_stat[n] + m * gx;
     L.b_stat[N + n] = L.b_stat[N + n] + m * gy;
     L.b_stat[2 * N + n] = L.b_stat[2 * N + n] + m * gz;
+}
+
+// ---------------------------------------------------------------------------
+// the potential from tabulated terms.  A term ((d . M) / |d|^3, d = point - magnet cell) depends
+// on d and M only, so for a list with few distinct magnetisations the terms of every d are
+// computed once (k_psi's operations, k_psi_terms) and a point's sum is one addition per magnet
+// cell, in list order as before: bit-identical.  (+0 stands in where k_psi skips d = 0: a sum
+// that starts at +0 is never -0, so adding it changes nothing.)
+//
+// The list is cut into runs of cells that follow each other along x with one M (k_psi_runs).  A
+// thread sums PSI_R points in x: a step along a run takes one new term for PSI_R additions.
+// Lanes are neighbouring (y, z), and the table is laid out [z][x][y] so that they load
+// consecutive terms; rows that follow each other in y find most of their terms in L1.  Bound by
+// the FP32 additions.
+// ---------------------------------------------------------------------------
+constexpr uint32_t PSI_R = 16, PSI_THREADS = 256, RUN_THREADS = 1024;
+
+// one block, the list in tiles: distinct magnetisations, bounds and runs, in list order.
+// runs[r] = (first list entry, its cell | magnetisation << 30), runs[number of runs] = (list length, 0)
+__global__ void __launch_bounds__(RUN_THREADS) k_psi_runs(const DevLbm L, const uint32_t* list, const uint32_t* count,
+                                                          uint2* runs, const uint32_t max_runs, PsiInfo* info) {
+    __shared__ uint32_t s_m[PSI_KINDS][3], s_kinds, s_first, s_warp[RUN_THREADS / 32], s_lo[3], s_hi[3];
+    const uint32_t nm = *count, t = threadIdx.x, lane = t & 31u;
+    const size_t N = L.n;
+    if (t == 0) s_kinds = 0u;
+    if (t < 3) { s_lo[t] = 0xFFFFFFFFu; s_hi[t] = 0u; }
+    uint32_t nruns = 0;
+    auto mag = [&](uint32_t n, int c) { return __float_as_uint(L.b_dyn[c * N + n]); };
+    for (uint32_t base = 0; base < nm; base += RUN_THREADS) {
+        const uint32_t i = base + t;
+        const bool in = i < nm;
+        uint32_t n = 0, x = 0, y = 0, z = 0, m[3] = {0u, 0u, 0u}, kind = 0;
+        bool start = false;
+        if (in) {
+            n = list[i];
+            cell_xyz(L, n, x, y, z);
+            for (int c = 0; c < 3; c++) m[c] = mag(n, c);
+            const uint32_t before = i ? list[i - 1] : 0u;
+            start = i == 0 || n != before + 1u || x == 0u || mag(before, 0) != m[0] || mag(before, 1) != m[1] ||
+                    mag(before, 2) != m[2];
+        }
+        for (;;) {  // the first entry of a magnetisation that is not known yet adds it
+            __syncthreads();
+            if (t == 0) s_first = 0xFFFFFFFFu;
+            __syncthreads();
+            bool known = !in;
+            for (uint32_t k = 0; k < s_kinds; k++)
+                if (in && s_m[k][0] == m[0] && s_m[k][1] == m[1] && s_m[k][2] == m[2]) { known = true; kind = k; }
+            if (!known) atomicMin(&s_first, t);
+            __syncthreads();
+            const uint32_t f = s_first;
+            if (f == 0xFFFFFFFFu) break;
+            if (s_kinds == PSI_KINDS) {  // too many: the host takes k_psi
+                if (t == 0) { info->count = nm; info->kinds = PSI_KINDS + 1u; }
+                return;
+            }
+            __syncthreads();
+            if (t == f) {
+                for (int c = 0; c < 3; c++) s_m[s_kinds][c] = m[c];
+                s_kinds++;
+            }
+        }
+        if (in) {
+            const uint32_t p[3] = {x, y, z};
+            for (int c = 0; c < 3; c++) { atomicMin(&s_lo[c], p[c]); atomicMax(&s_hi[c], p[c]); }
+        }
+        const uint32_t ball = __ballot_sync(0xFFFFFFFFu, start);
+        if (lane == 0) s_warp[t >> 5] = __popc(ball);
+        __syncthreads();
+        uint32_t at = nruns;
+        for (uint32_t w = 0; w < RUN_THREADS / 32; w++) {
+            if (w < (t >> 5)) at += s_warp[w];
+            nruns += s_warp[w];
+        }
+        if (nruns >= max_runs) {  // no room (nor much use): the host takes k_psi
+            if (t == 0) { info->count = nm; info->kinds = PSI_KINDS + 1u; }
+            return;
+        }
+        if (start) runs[at + __popc(ball & ((1u << lane) - 1u))] = make_uint2(i, n | kind << 30);
+        __syncthreads();
+    }
+    if (t == 0) {
+        runs[nruns] = make_uint2(nm, 0u);
+        info->count = nm;
+        info->runs = nruns;
+        info->kinds = s_kinds;
+    }
+    if (t < 3) { info->lo[t] = s_lo[t]; info->hi[t] = s_hi[t]; }
+    if (t < 3u * PSI_KINDS) (&info->m[0][0])[t] = __uint_as_float((&s_m[0][0])[t]);
+}
+
+// terms T[kind][z][x][y] of the differences point - cell, from (x0, y0, z0) on
+__global__ void __launch_bounds__(256) k_psi_terms(const PsiTable P) {
+    const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x, x = blockIdx.y, k = blockIdx.z / P.tz, z = blockIdx.z % P.tz;
+    if (y >= P.ty) return;
+    const float dx = (float)(P.x0 + (int)x), dy = (float)(P.y0 + (int)y), dz = (float)(P.z0 + (int)z);
+    const float* m = P.m[k];
+    const float l = sqrtf((dx * dx + dy * dy) + dz * dz);
+    float v = 0.0f;
+    if (!(l == 0.0f)) v = ((dx * m[0] + dy * m[1]) + dz * m[2]) / ((l * l) * l);
+    P.T[(((size_t)k * P.tz + z) * P.tx + x) * P.ty + y] = v;
+}
+
+__global__ void __launch_bounds__(PSI_THREADS) k_psi_runs_sum(const DevLbm L, const PsiTable P, float* psi) {
+    const uint32_t l0 = L.nx + 2, l1 = L.ny + 2, l2 = L.nz + 2;
+    const uint32_t nxb = (l0 + PSI_R - 1u) / PSI_R, rows = l1 * l2;
+    // warps of a block: the x blocks of the same 32 rows first
+    const uint32_t w = blockIdx.x * (PSI_THREADS / 32u) + (threadIdx.x >> 5);
+    const uint32_t xb = w % nxb, row = w / nxb * 32u + (threadIdx.x & 31u);
+    if (w / nxb * 32u >= rows) return;  // whole warps
+    const bool valid = row < rows;
+    const uint32_t cy = (valid ? row : 0u) % l1, cz = (valid ? row : 0u) / l1;
+    // the term of point (PSI_R xb, cy, cz) and a cell whose run offset is 0
+    const float* const origin = P.T + ((int64_t)((int)cz - P.z0) * P.tx + ((int)(xb * PSI_R) - P.x0)) * P.ty + ((int)cy - P.y0);
+    float acc[PSI_R];
+#pragma unroll
+    for (uint32_t i = 0; i < PSI_R; i++) acc[i] = 0.0f;
+    uint2 run = P.runs[0];
+    for (uint32_t r = 0; r < P.nruns; r++) {
+        const uint2 next = P.runs[r + 1u];
+        uint32_t x, y, z;
+        cell_xyz(L, run.y & 0x3FFFFFFFu, x, y, z);
+        const int64_t kind = (int64_t)(run.y >> 30) * P.tz;
+        // points are the padded grid's: the cell lies at (x + 1, y + 1, z + 1)
+        const float* p = origin + ((kind - (int64_t)(z + 1u)) * P.tx - (int64_t)(x + 1u)) * P.ty - (int64_t)(y + 1u);
+        uint32_t left = next.x - run.x;
+        run = next;
+        float v[2 * PSI_R];  // v[k]: the term k - PSI_R cells from the run's position
+#pragma unroll
+        for (uint32_t i = 0; i < PSI_R; i++) v[PSI_R + i] = __ldg(p + (int64_t)i * P.ty);
+        while (left) {
+            const uint32_t steps = min(left, PSI_R);
+#pragma unroll
+            for (uint32_t i = 1; i <= PSI_R; i++) v[PSI_R - i] = __ldg(p - (int64_t)i * P.ty);
+            if (steps == PSI_R) {
+#pragma unroll
+                for (uint32_t s = 0; s < PSI_R; s++)
+#pragma unroll
+                    for (uint32_t i = 0; i < PSI_R; i++) acc[i] = acc[i] + v[PSI_R + i - s];
+            } else {
+#pragma unroll
+                for (uint32_t s = 0; s < PSI_R - 1u; s++) {
+                    if (s >= steps) break;
+#pragma unroll
+                    for (uint32_t i = 0; i < PSI_R; i++) acc[i] = acc[i] + v[PSI_R + i - s];
+                }
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < PSI_R; i++) v[PSI_R + i] = v[i];
+            p -= (int64_t)PSI_R * P.ty;
+            left -= steps;
+        }
+    }
+    if (!valid) return;
+#pragma unroll
+    for (uint32_t i = 0; i < PSI_R; i++) {
+        const uint32_t cx = xb * PSI_R + i;
+        if (cx < l0) psi[cx + (size_t)row * l0] = (float)((double)acc[i] / (4.0 * 3.14159265358979323846));
+    }
+}
+
+void launch_psi_runs(const DevLbm& L, const uint32_t* list, const uint32_t* count, uint2* runs, uint32_t max_runs,
+                     PsiInfo* info, cudaStream_t s) {
+    k_psi_runs<<<1, RUN_THREADS, 0, s>>>(L, list, count, runs, max_runs, info);
+}
+
+size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P) {
+    const uint32_t nxb = (L.nx + 2u + PSI_R - 1u) / PSI_R;
+    // x: a thread's points reach PSI_R nxb - 1, its loads run up to PSI_R past the end of a run
+    P.x0 = -(int)(I.hi[0] + 1u) - (int)(2u * PSI_R);
+    P.y0 = -(int)(I.hi[1] + 1u);
+    P.z0 = -(int)(I.hi[2] + 1u);
+    P.tx = nxb * PSI_R + (I.hi[0] - I.lo[0]) + 2u * PSI_R;
+    P.ty = L.ny + 2u + (I.hi[1] - I.lo[1]);
+    P.tz = L.nz + 2u + (I.hi[2] - I.lo[2]);
+    P.nruns = I.runs;
+    for (uint32_t k = 0; k < PSI_KINDS; k++)
+        for (int c = 0; c < 3; c++) P.m[k][c] = I.m[k][c];
+    return (size_t)I.kinds * P.tz * P.tx * P.ty * sizeof(float);
+}
+
+void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, cudaStream_t s) {
+    k_psi_terms<<<dim3((P.ty + 255u) / 256u, P.tx, P.tz * kinds), 256, 0, s>>>(P);
+    const uint64_t rows = (uint64_t)(L.ny + 2) * (L.nz + 2), nxb = (L.nx + 2u + PSI_R - 1u) / PSI_R;
+    k_psi_runs_sum<<<grid_for((rows + 31u) / 32u * nxb * 32u, PSI_THREADS), PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
+    k_static_b<<<grid_for(L.n, 256), 256, 0, s>>>(L, L.e_dyn);
 }
 
 void launch_psi_static_b(const DevLbm& L, const uint32_t* mags, const uint32_t* count, cudaStream_t s) {
