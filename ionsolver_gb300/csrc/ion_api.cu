@@ -972,7 +972,7 @@ static int psi_table(ion_lbm* h, PsiTable& P, uint32_t& kinds) {
     if (info.count < 64u || info.kinds > PSI_KINDS) return ION_OK;
     const size_t bytes = psi_table_size(h->L, info, P), run_bytes = sizeof(uint2) * ((size_t)info.runs + 1);
     const size_t at = (bytes + 255) / 256 * 256;
-    if (P.tx > 65535u || (uint64_t)P.tz * info.kinds > 65535u) return ION_OK;
+    if ((uint64_t)P.tx * P.ny >= 1ull << 32 || (uint64_t)P.tz * info.kinds > 65535u) return ION_OK;
     if (h->psi_ws_bytes < at + run_bytes) {
         cudaFree(h->psi_ws);
         h->psi_ws_bytes = 0;

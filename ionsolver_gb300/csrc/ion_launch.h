@@ -33,7 +33,8 @@ struct PsiInfo {
 struct PsiTable {
     float* T;
     const uint2* runs;
-    uint32_t nruns, tx, ty, tz;    // T is [kind][z][x][y]
+    uint32_t nruns, tx, ty, tz;    // T is [kind][z][x][y], of ty the first ny are used
+    uint32_t ny;
     int x0, y0, z0;                // the first differences
     float m[PSI_KINDS][3];
 };

@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(256) k_static_b(const DevLbm L, const float* p
 // thread sums PSI_R points in x: a step along a run takes one new term for PSI_R additions.
 // Lanes are neighbouring (y, z), and the table is laid out [z][x][y] so that they load
 // consecutive terms; rows that follow each other in y find most of their terms in L1.  Bound by
-// the FP32 additions.
+// the additions: at 128^3 and 6,800 cells 0.63 ms (immediate load offsets; 0.76 ms with computed
+// addresses, 0.69 ms with two rows in packed additions at half the warps), k_psi 15.9 ms.
 // ---------------------------------------------------------------------------
 constexpr uint32_t PSI_R = 16, PSI_THREADS = 256, RUN_THREADS = 1024;
 
@@ -317,8 +318,9 @@ __global__ void __launch_bounds__(RUN_THREADS) k_psi_runs(const DevLbm L, const 
 
 // terms T[kind][z][x][y] of the differences point - cell, from (x0, y0, z0) on
 __global__ void __launch_bounds__(256) k_psi_terms(const PsiTable P) {
-    const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x, x = blockIdx.y, k = blockIdx.z / P.tz, z = blockIdx.z % P.tz;
-    if (y >= P.ty) return;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, x = i / P.ny, y = i % P.ny;
+    const uint32_t k = blockIdx.y / P.tz, z = blockIdx.y % P.tz;
+    if (x >= P.tx) return;
     const float dx = (float)(P.x0 + (int)x), dy = (float)(P.y0 + (int)y), dz = (float)(P.z0 + (int)z);
     const float* m = P.m[k];
     const float l = sqrtf((dx * dx + dy * dy) + dz * dz);
@@ -327,9 +329,14 @@ __global__ void __launch_bounds__(256) k_psi_terms(const PsiTable P) {
     P.T[(((size_t)k * P.tz + z) * P.tx + x) * P.ty + y] = v;
 }
 
-__global__ void __launch_bounds__(PSI_THREADS) k_psi_runs_sum(const DevLbm L, const PsiTable P, float* psi) {
+// PITCH: the table's row length in elements (0: P.ty), a constant so that a step's load is an
+// immediate offset
+template <uint32_t PITCH>
+__global__ void __launch_bounds__(PSI_THREADS, 4) k_psi_runs_sum(const DevLbm L, const PsiTable P, float* psi) {
+    constexpr int R = (int)PSI_R;
     const uint32_t l0 = L.nx + 2, l1 = L.ny + 2, l2 = L.nz + 2;
     const uint32_t nxb = (l0 + PSI_R - 1u) / PSI_R, rows = l1 * l2;
+    const int64_t ty = PITCH ? PITCH : P.ty;
     // warps of a block: the x blocks of the same 32 rows first
     const uint32_t w = blockIdx.x * (PSI_THREADS / 32u) + (threadIdx.x >> 5);
     const uint32_t xb = w % nxb, row = w / nxb * 32u + (threadIdx.x & 31u);
@@ -337,10 +344,10 @@ __global__ void __launch_bounds__(PSI_THREADS) k_psi_runs_sum(const DevLbm L, co
     const bool valid = row < rows;
     const uint32_t cy = (valid ? row : 0u) % l1, cz = (valid ? row : 0u) / l1;
     // the term of point (PSI_R xb, cy, cz) and a cell whose run offset is 0
-    const float* const origin = P.T + ((int64_t)((int)cz - P.z0) * P.tx + ((int)(xb * PSI_R) - P.x0)) * P.ty + ((int)cy - P.y0);
-    float acc[PSI_R];
+    const float* const origin = P.T + ((int64_t)((int)cz - P.z0) * P.tx + ((int)(xb * PSI_R) - P.x0)) * ty + ((int)cy - P.y0);
+    float acc[R];
 #pragma unroll
-    for (uint32_t i = 0; i < PSI_R; i++) acc[i] = 0.0f;
+    for (int i = 0; i < R; i++) acc[i] = 0.0f;
     uint2 run = P.runs[0];
     for (uint32_t r = 0; r < P.nruns; r++) {
         const uint2 next = P.runs[r + 1u];
@@ -348,33 +355,40 @@ __global__ void __launch_bounds__(PSI_THREADS) k_psi_runs_sum(const DevLbm L, co
         cell_xyz(L, run.y & 0x3FFFFFFFu, x, y, z);
         const int64_t kind = (int64_t)(run.y >> 30) * P.tz;
         // points are the padded grid's: the cell lies at (x + 1, y + 1, z + 1)
-        const float* p = origin + ((kind - (int64_t)(z + 1u)) * P.tx - (int64_t)(x + 1u)) * P.ty - (int64_t)(y + 1u);
+        const float* p = origin + ((kind - (int64_t)(z + 1u)) * P.tx - (int64_t)(x + 1u)) * ty - (int64_t)(y + 1u);
         uint32_t left = next.x - run.x;
         run = next;
-        float v[2 * PSI_R];  // v[k]: the term k - PSI_R cells from the run's position
+        // up to R steps along the run: `above` holds the terms of the points at its position,
+        // `below` gets the R terms before them
+        auto steps = [&](const float (&above)[R], float (&below)[R]) {
+            if (left >= PSI_R) {
 #pragma unroll
-        for (uint32_t i = 0; i < PSI_R; i++) v[PSI_R + i] = __ldg(p + (int64_t)i * P.ty);
-        while (left) {
-            const uint32_t steps = min(left, PSI_R);
+                for (int k = 1; k <= R; k++) below[R - k] = __ldg(p - k * ty);
 #pragma unroll
-            for (uint32_t i = 1; i <= PSI_R; i++) v[PSI_R - i] = __ldg(p - (int64_t)i * P.ty);
-            if (steps == PSI_R) {
+                for (int k = 0; k < R; k++)
 #pragma unroll
-                for (uint32_t s = 0; s < PSI_R; s++)
-#pragma unroll
-                    for (uint32_t i = 0; i < PSI_R; i++) acc[i] = acc[i] + v[PSI_R + i - s];
+                    for (int i = 0; i < R; i++) acc[i] = acc[i] + (i >= k ? above[i - k] : below[R + i - k]);
+                p -= R * ty;
+                left -= PSI_R;
             } else {
 #pragma unroll
-                for (uint32_t s = 0; s < PSI_R - 1u; s++) {
-                    if (s >= steps) break;
+                for (int k = 0; k < R - 1; k++) {
+                    if (k >= (int)left) break;
+                    if (k > 0) below[R - k] = __ldg(p - k * ty);
 #pragma unroll
-                    for (uint32_t i = 0; i < PSI_R; i++) acc[i] = acc[i] + v[PSI_R + i - s];
+                    for (int i = 0; i < R; i++) acc[i] = acc[i] + (i >= k ? above[i - k] : below[R + i - k]);
                 }
+                left = 0u;
             }
+        };
+        float a[R], b[R];
 #pragma unroll
-            for (uint32_t i = 0; i < PSI_R; i++) v[PSI_R + i] = v[i];
-            p -= (int64_t)PSI_R * P.ty;
-            left -= steps;
+        for (int i = 0; i < R; i++) a[i] = __ldg(p + i * ty);
+        for (;;) {
+            steps(a, b);
+            if (!left) break;
+            steps(b, a);
+            if (!left) break;
         }
     }
     if (!valid) return;
@@ -398,6 +412,8 @@ size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P) {
     P.z0 = -(int)(I.hi[2] + 1u);
     P.tx = nxb * PSI_R + (I.hi[0] - I.lo[0]) + 2u * PSI_R;
     P.ty = L.ny + 2u + (I.hi[1] - I.lo[1]);
+    P.ny = P.ty;
+    if (P.ty <= 256u) P.ty = (P.ty + 63u) / 64u * 64u;  // the constant pitches
     P.tz = L.nz + 2u + (I.hi[2] - I.lo[2]);
     P.nruns = I.runs;
     for (uint32_t k = 0; k < PSI_KINDS; k++)
@@ -406,9 +422,14 @@ size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P) {
 }
 
 void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, cudaStream_t s) {
-    k_psi_terms<<<dim3((P.ty + 255u) / 256u, P.tx, P.tz * kinds), 256, 0, s>>>(P);
+    k_psi_terms<<<dim3((P.tx * P.ny + 255u) / 256u, P.tz * kinds), 256, 0, s>>>(P);
     const uint64_t rows = (uint64_t)(L.ny + 2) * (L.nz + 2), nxb = (L.nx + 2u + PSI_R - 1u) / PSI_R;
-    k_psi_runs_sum<<<grid_for((rows + 31u) / 32u * nxb * 32u, PSI_THREADS), PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
+    const unsigned grid = grid_for((rows + 31u) / 32u * nxb * 32u, PSI_THREADS);
+    if (P.ty == 64u) k_psi_runs_sum<64><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
+    else if (P.ty == 128u) k_psi_runs_sum<128><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
+    else if (P.ty == 192u) k_psi_runs_sum<192><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
+    else if (P.ty == 256u) k_psi_runs_sum<256><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
+    else k_psi_runs_sum<0><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
     k_static_b<<<grid_for(L.n, 256), 256, 0, s>>>(L, L.e_dyn);
 }
 
