@@ -348,10 +348,10 @@ int ion_batch_destroy(ion_batch* b);
 int ion_batch_run(ion_batch* b, uint64_t steps);
 /* bounded wait for the batch's stream; reports device-side timeouts */
 int ion_batch_finish(ion_batch* b, int timeout_ms);
-/* the batch step's poll limits: grid barrier between its phases (default
- * ION_BARRIER_LIMIT_DEFAULT, polls 64 ns apart) and staged-tile waits of every
- * domain (as ion_lbm_set_wait_limit); a wait that gives up ends the launch
- * and ion_batch_finish returns ION_E_TIMEOUT */
+/* the batch step's poll limit: staged-tile waits of every domain (as
+ * ion_lbm_set_wait_limit); a wait that gives up ends the launch and
+ * ion_batch_finish returns ION_E_TIMEOUT.  barrier_polls is accepted and not
+ * used: the phases of a step are launches of their own, no grid barrier waits */
 #define ION_BARRIER_LIMIT_DEFAULT 67108864u
 int ion_batch_set_wait_limits(ion_batch* b, uint32_t barrier_polls, uint32_t tile_polls);
 /* autotuner record i (block, grid, ms per step); i = 0xFFFFFFFF: the chosen shape */

@@ -2,21 +2,19 @@
 // timestep (no reference counterpart: the reference steps one domain per
 // OpenCL queue, src/lbm/mod.rs:250-272).
 //
-// Two persistent launches advance every domain of a batch by one step (and, where a domain's
-// FAST field is a convolution over its bins, the launches of field_fft.cu):
-// k_batch_stream (cooperative) runs
-//   A  stream_collide of every cell of every domain   (sc_cell)
-//   B  LOD bin sums of every domain                     (lod_bin_warp)
-// separated by a grid-wide barrier, and k_batch_field runs
-//   C  E/B update of every cell of every domain         (eb_tile)
-// (the kernel boundary orders C after B; each kernel has its own register budget).
-// Work is handed out in tiles of EB_CPT*blockDim consecutive cells (A), bricks
-// or half bricks (C, as in the single-domain E/B kernel) or one warp per bin
-// (B); a tile's domain is found by binary search over prefix sums of the
-// per-domain tile counts.  Every cell runs exactly the per-cell code of the
-// single-domain kernels, so a batched step is bit-identical to stepping the
-// domains one by one.  The grid barrier spins with an iteration limit and
-// reports a timeout through an error flag instead of hanging.
+// A few launches advance every domain of a batch by one step:
+//   A  stream_collide of every cell of every domain   (sc_cell; k_batch_stream[_rows])
+//   B  LOD bin sums of every domain                   (lod_bins_block; k_batch_lod)
+//   C  E/B update of every cell of every domain       (eb_tile; k_batch_field), or, where a
+//      domain's FAST field is a convolution over its bins, the launches of field_fft.cu
+// each with its own register budget.  (A and B in one cooperative launch with a grid barrier
+// between them and one warp per bin: 1.13 ms for 24 domains of 32 to 96 cells; apart 0.65 +
+// 0.09 ms.)
+// Work is handed out in tiles of EB_CPT*blockDim consecutive cells or x-rows (A), groups of
+// bins (B), bricks or half bricks (C, as in the single-domain E/B kernel); a tile's domain is
+// found by binary search over prefix sums of the per-domain counts.  Every cell runs exactly
+// the per-cell code of the single-domain kernels, so a batched step is bit-identical to
+// stepping the domains one by one.
 #include "field_kernels.cuh"
 #include "ion_launch.h"
 #include "lbm_kernels.cuh"
@@ -34,49 +32,22 @@ __device__ __forceinline__ uint32_t find_domain(const uint32_t* off, uint32_t nd
     return lo;
 }
 
-// Generation barrier over all blocks of a co-resident grid.  Returns false
-// (block-uniform) when it gave up after `limit` polls.
-__device__ __forceinline__ bool grid_barrier(uint32_t* count, uint32_t* gen, uint32_t nblocks, uint32_t limit) {
-    __syncthreads();
-    int ok = 1;
+// Phase B (MHD): the LOD bins of every domain, the single-domain kernel's blocks
+static __global__ void __launch_bounds__(LB_THREADS) k_batch_lod(const BatchDev B) {
+    __shared__ LodSmem sm;
+    __shared__ DevLbm sL;
+    __shared__ uint32_t s_dom;
     if (threadIdx.x == 0) {
-        const uint32_t g = *(volatile uint32_t*)gen;
-        __threadfence();
-        if (atomicAdd(count, 1u) == nblocks - 1u) {
-            atomicExch(count, 0u);
-            __threadfence();
-            atomicAdd(gen, 1u);
-        } else {
-            uint32_t i = 0;
-            while (*(volatile uint32_t*)gen == g) {
-                if (++i > limit) { ok = 0; break; }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
+        s_dom = find_domain(B.bin_off, B.ndom, blockIdx.x);
+        sL = B.doms[s_dom];
     }
-    return __syncthreads_and(ok) != 0;
+    __syncthreads();
+    if (sL.depth > 0u) lod_bins_block(sL, blockIdx.x - B.bin_off[s_dom], sm);
+    else if (threadIdx.x < 4u) sL.qu_lod[threadIdx.x] = 0.0f;
 }
 
-// Phase B (MHD): a grid barrier, then the LOD bins of every domain, one warp per bin
-__device__ __forceinline__ void batch_lod_phase(const BatchDev& B) {
-    const uint32_t nblocks = gridDim.x;
-    if (!grid_barrier(B.bar_count, B.bar_gen, nblocks, B.barrier_limit)) {
-        if (threadIdx.x == 0) atomicExch(B.err, 2u);
-        return;
-    }
-    const uint32_t warps = nblocks * (blockDim.x >> 5);
-    for (uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < B.total_bins; w += warps) {
-        const uint32_t d = find_domain(B.bin_off, B.ndom, w);
-        const DevLbm& L = B.doms[d];
-        if (L.depth > 0u) lod_bin_warp(L, w - B.bin_off[d], threadIdx.x & 31u);
-        else if ((threadIdx.x & 31u) < 4u) L.qu_lod[threadIdx.x & 31u] = 0.0f;
-    }
-}
-
-// Phase A (+ B with MHD): stream_collide of every cell of every domain, a grid barrier,
-// then the LOD bin sums; a cooperative launch of BATCH_SC_THREADS-thread blocks.  It has
-// its own register budget (the global-load MHD stencil wants ~140 registers; in one
+// Phase A: stream_collide of every cell of every domain, in resident blocks of
+// BATCH_SC_THREADS threads.  It has its own register budget (the global-load MHD stencil wants ~140 registers; in one
 // kernel with the E/B phase both were held to 128 and spilled).
 template <int FT, bool MHD>
 __global__ void __launch_bounds__(BATCH_SC_THREADS, MHD ? 3 : 4) k_batch_stream(const BatchDev B, const uint32_t odd_t) {
@@ -100,10 +71,9 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, MHD ? 3 : 4) k_batch_stream(
             }
         }
     }
-    if constexpr (MHD) batch_lod_phase(B);
 }
 
-// Phase A (+ B with MHD) over x-rows, when every domain's rows are whole 16-byte streams of
+// Phase A over x-rows, when every domain's rows are whole 16-byte streams of
 // at most BATCH_ROW_MAX cells: the producer-warp form of k_sc_rows_ws (lbm_kernels.cuh)
 // walking the rows of all domains (global row g = blockIdx.x + k gridDim.x, its domain by
 // binary search over the prefix sums of ny nz).  The last warp stages each row and writes
@@ -222,7 +192,6 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, 5) k_batch_stream_rows(const
             mbar_wait(&full[k & 1u], (k >> 1) & 1u, WAIT_LIMIT);
         atomicExch(B.err, 1u);
     }
-    if constexpr (MHD) batch_lod_phase(B);
 }
 
 // Phase C: the E/B update of every brick (or half brick) of every domain, after phase B
@@ -316,8 +285,8 @@ int batch_max_blocks_per_sm(int ft, bool mhd, bool fast, bool rows, int block) {
     return n;
 }
 
-// One timestep of a batch: the cooperative stencil (+ bins) kernel at full occupancy,
-// then, with MHD, the E/B kernel with the tuned shape (grid x block).
+// One timestep of a batch: the stencil kernel at full occupancy, then, with MHD, the bins and
+// the E/B kernel with the tuned shape (grid x block).
 cudaError_t launch_batch_step(const BatchDev& B, int ft, bool mhd, bool fast, uint32_t grid, uint32_t block,
                               uint64_t t, cudaStream_t s) {
     const bool rows = B.total_rows > 0u;
@@ -336,14 +305,12 @@ cudaError_t launch_batch_step(const BatchDev& B, int ft, bool mhd, bool fast, ui
     cfg.blockDim = dim3(BATCH_SC_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     void* args[] = {(void*)&B, (void*)&odd};
     e = cudaLaunchKernelExC(&cfg, ks, args);
-    if (e != cudaSuccess || !mhd || B.total_bricks == 0u) return e;
+    if (e != cudaSuccess || !mhd) return e;
+    k_batch_lod<<<B.total_bins, LB_THREADS, 0, s>>>(B);
+    e = cudaGetLastError();
+    if (e != cudaSuccess || B.total_bricks == 0u) return e;
     cudaLaunchConfig_t cf = {};
     cf.gridDim = dim3(grid);
     cf.blockDim = dim3(block);

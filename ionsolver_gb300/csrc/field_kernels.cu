@@ -4,7 +4,7 @@
 namespace ion {
 
 void launch_lod_bins(const DevLbm& L, cudaStream_t s) {
-    k_lod_bins<<<L.n_lod_own, LB_THREADS, 0, s>>>(L);
+    k_lod_bins<<<lod_blocks(L.nd), LB_THREADS, 0, s>>>(L);
 }
 
 void launch_update_e_b_gated(const DevLbm& L, uint32_t* err, const uint32_t* gate, cudaStream_t s) {

@@ -2,9 +2,9 @@
 // (IonSolver src/kernels/sim_kernels.cl:666-677, 897-1003) on sm_103a.
 //
 // LOD bins.  The reference accumulates every fluid cell's charge and
-// velocity/volume into its depth-D bin with float atomics.  Here one warp
-// owns one bin: lanes fetch 32 cells at a time in ascending cell order and
-// lanes 0..3 (charge, ux, uy, uz) add them one after another.  The result
+// velocity/volume into its depth-D bin with float atomics.  Here a lane owns
+// one of a bin's four sums (charge, ux, uy, uz) and adds the bin's cells one
+// after another in ascending cell order.  The result
 // is the sum the reference produces when its work-items run in index order,
 // and it is the same on every run.
 //
@@ -23,43 +23,6 @@
 
 namespace ion {
 
-// ---------------------------------------------------------------------------
-// LOD bins: one warp per bin (bins >= 8^D are cleared, as clear_qu_lod does)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void lod_bin_warp(const DevLbm& L, const uint32_t bin, const uint32_t lane) {
-    float acc = 0.0f;
-    if (bin < L.n_bins) {
-        const uint32_t nd = L.nd;
-        const uint32_t bx = bin % nd, by = (bin / nd) % nd, bz = bin / (nd * nd);
-        const uint32_t cells = L.bsx * L.bsy * L.bsz;
-        const size_t N = L.n;
-        for (uint32_t base = 0; base < cells; base += 32u) {
-            const uint32_t li = base + lane;
-            float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f, v3 = 0.0f;
-            bool has = false;
-            if (li < cells) {
-                const uint32_t lx = li % L.bsx, ly = (li / L.bsx) % L.bsy, lz = li / (L.bsx * L.bsy);
-                const uint32_t n = (bx * L.bsx + lx) + ((by * L.bsy + ly) + (bz * L.bsz + lz) * L.ny) * L.nx;
-                has = (L.flags[n] & F_BO) != F_S;
-                if (has) { v0 = L.q[n]; v1 = L.lod_cell[n]; v2 = L.lod_cell[N + n]; v3 = L.lod_cell[2 * N + n]; }
-            }
-            const uint32_t cnt = cells - base < 32u ? cells - base : 32u;
-            for (uint32_t k = 0; k < cnt; k++) {
-                const float a0 = __shfl_sync(0xFFFFFFFFu, v0, k);
-                const float a1 = __shfl_sync(0xFFFFFFFFu, v1, k);
-                const float a2 = __shfl_sync(0xFFFFFFFFu, v2, k);
-                const float a3 = __shfl_sync(0xFFFFFFFFu, v3, k);
-                const int hk = __shfl_sync(0xFFFFFFFFu, (int)has, k);
-                if (hk) {
-                    const float a = lane == 0u ? a0 : lane == 1u ? a1 : lane == 2u ? a2 : a3;
-                    acc = acc + a;
-                }
-            }
-        }
-    }
-    if (lane < 4u) L.qu_lod[(size_t)bin * 4u + lane] = acc;
-}
-
 // n / d by a multiply-high: floor(n m / 2^32) with m = floor((2^32 - 1) / d) + 1 (d > 1).
 // With n = q d + r, n m / 2^32 = n / d + n e / 2^32 with 0 <= e < 1, and n e / 2^32 < 1 / d
 // whenever n d < 2^32, so the floor is q (division by invariant integers, Granlund &
@@ -70,60 +33,93 @@ struct Magic {
     __device__ __forceinline__ uint32_t div(uint32_t n) const { return d > 1u ? __umulhi(n, m) : n; }
 };
 
-// LOD bins of one domain, one thread block per bin: warps 1..7 stream the
-// bin's cells (ascending cell index) through shared memory in slabs of
-// LB_SLAB cells, double-buffered, while lanes 0..3 of warp 0 add charge and
-// the three velocity components one cell after another -- the same sequence
-// of float additions as lod_bin_warp.  A cell outside the fluid is stored as
-// -0.0f, which leaves every float (+0 included) unchanged under
-// round-to-nearest addition, so the sums need no branch and the summing
-// lanes read four cells per shared-memory load.
-
-constexpr uint32_t LB_THREADS = 256, LB_SLAB = 512;
+// LOD bins, LB_BINS neighbours along x per thread block: warps 1.. stream the bins' cells
+// (ascending cell index, LB_SLAB of each bin at a time, double-buffered) through shared memory,
+// laid out so that the 32 lanes of warp 0 -- lane = bin + LB_BINS component -- each add the
+// next cell of their sum in one load and one addition.  A cell outside the fluid is stored as -0.0f, which leaves every float (+0
+// included) unchanged under round-to-nearest addition, so the sums need no branch.
+// Bound by memory (17 bytes a cell) for large bins and by the additions, 4 cycles each, for
+// small ones: 12.3 us at 128^3, 67 us at 256^3 (4.2 TB/s).  A block per bin with four summing
+// lanes took 21.7 and 97 us (a quarter of the bins resident at a time); lanes across the bins
+// instead of along the row 16.5 and 103 us (8 sectors of 16 bytes a load).
+constexpr uint32_t LB_THREADS = 288, LB_SLAB = 128;
+// cells 34 floats apart: the 32 lanes of a store (4 cells apart, 8 bins) write 32 different banks
+constexpr uint32_t LB_CELL = 34;
 struct LodSmem {
-    float v[2][4][LB_SLAB];  // [buffer][component][cell]
+    float v[2][LB_SLAB * LB_CELL];  // [buffer][cell][component][bin]
 };
+template <uint32_t V> struct LodVec;
+template <> struct LodVec<1> { using F = float; using B = uint8_t; };
+template <> struct LodVec<2> { using F = float2; using B = uchar2; };
+template <> struct LodVec<4> { using F = float4; using B = uchar4; };
 
-static __global__ void __launch_bounds__(LB_THREADS) k_lod_bins(const DevLbm L) {
-    __shared__ __align__(16) LodSmem sm;
-    const uint32_t bin = blockIdx.x;
-    if (bin >= L.n_bins) {  // bins of the lower LOD levels stay zero (single domain)
-        if (threadIdx.x < 4u) L.qu_lod[(size_t)bin * 4u + threadIdx.x] = 0.0f;
-        return;
-    }
-    const uint32_t nd = L.nd;
-    const uint32_t bx = bin % nd, by = (bin / nd) % nd, bz = bin / (nd * nd);
-    const uint32_t cells = L.bsx * L.bsy * L.bsz;
-    const uint32_t nslabs = (cells + LB_SLAB - 1u) / LB_SLAB;
+// cells of slab `base` of the block's bins to shared memory (warps 1..), V neighbours a thread.
+// Lanes run along the bins' common x-row (bins of up to LB_SLAB cells an edge), so a warp's
+// loads are contiguous.
+template <uint32_t V>
+__device__ __forceinline__ void lod_load(const DevLbm& L, float* const buf, uint32_t x0, uint32_t y0, uint32_t z0,
+                                         uint32_t nb, uint32_t base, uint32_t cnt, bool rows, bool magic, const Magic& mx,
+                                         const Magic& mxy, const Magic& mq) {
+    using F = typename LodVec<V>::F;
+    using B = typename LodVec<V>::B;
     const size_t N = L.n;
-    const Magic mx(L.bsx), mxy(L.bsx * L.bsy);
-    const bool magic = (uint64_t)cells * (L.bsx * L.bsy) < (1ull << 32);  // Magic's bound (bins of <= ~2^16 cells)
-    auto load = [&](uint32_t k) {  // warps 1..7; the slab is padded with -0.0f to a multiple of 4 cells
-        const uint32_t base = k * LB_SLAB;
-        const uint32_t cnt = min(LB_SLAB, cells - base);
-        const uint32_t padded = (cnt + 3u) & ~3u;
-        float(*v)[LB_SLAB] = sm.v[k & 1u];
-#pragma unroll 3
-        for (uint32_t i = threadIdx.x - 32u; i < padded; i += LB_THREADS - 32u) {
-            float4 c = make_float4(-0.0f, -0.0f, -0.0f, -0.0f);
-            if (i < cnt) {  // all five loads in flight at once; the flag selects afterwards
-                const uint32_t li = base + i;
-                uint32_t lx, ly, lz;
-                if (magic) {
-                    lz = mxy.div(li);
-                    const uint32_t r = li - lz * mxy.d;
-                    ly = mx.div(r);
-                    lx = r - ly * mx.d;
-                } else {
-                    lx = li % L.bsx; ly = (li / L.bsx) % L.bsy; lz = li / (L.bsx * L.bsy);
-                }
-                const uint32_t n = (bx * L.bsx + lx) + ((by * L.bsy + ly) + (bz * L.bsz + lz) * L.ny) * L.nx;
-                const uint8_t f = L.flags[n];
-                const float4 a = make_float4(L.q[n], L.lod_cell[n], L.lod_cell[N + n], L.lod_cell[2 * N + n]);
-                if ((f & F_BO) != F_S) c = a;
-            }
-            v[0][i] = c.x; v[1][i] = c.y; v[2][i] = c.z; v[3][i] = c.w;
+#pragma unroll 2
+    for (uint32_t e = threadIdx.x - 32u; e < cnt / V * nb; e += LB_THREADS - 32u) {
+        uint32_t b, j;
+        if (rows) {
+            const uint32_t rb = mq.div(e), q = e - rb * mq.d;  // (row, bin), group of V cells
+            b = rb & (nb - 1u);
+            j = rb / nb * L.bsx + q * V;
+        } else {
+            b = e & (nb - 1u);
+            j = e / nb;
         }
+        const uint32_t li = base + j;
+        uint32_t lx, ly, lz;
+        if (magic) {
+            lz = mxy.div(li);
+            const uint32_t r = li - lz * mxy.d;
+            ly = mx.div(r);
+            lx = r - ly * mx.d;
+        } else {
+            lx = li % L.bsx; ly = (li / L.bsx) % L.bsy; lz = li / (L.bsx * L.bsy);
+        }
+        const uint32_t n = (x0 + b * L.bsx + lx) + ((y0 + ly) + (z0 + lz) * L.ny) * L.nx;
+        // all five loads in flight at once; the flag selects afterwards
+        const B f = *reinterpret_cast<const B*>(L.flags + n);
+        F a[4];
+        a[0] = *reinterpret_cast<const F*>(L.q + n);
+#pragma unroll
+        for (uint32_t c = 0; c < 3; c++) a[c + 1u] = *reinterpret_cast<const F*>(L.lod_cell + c * N + n);
+#pragma unroll
+        for (uint32_t u = 0; u < V; u++) {
+            const bool fluid = (reinterpret_cast<const uint8_t*>(&f)[u] & F_BO) != F_S;
+            float* const o = buf + (j + u) * LB_CELL + b;
+#pragma unroll
+            for (uint32_t c = 0; c < 4; c++) o[c * LB_BINS] = fluid ? reinterpret_cast<const float*>(&a[c])[u] : -0.0f;
+        }
+    }
+}
+
+__device__ __forceinline__ void lod_bins_block(const DevLbm& L, const uint32_t block, LodSmem& sm) {
+    const uint32_t nd = L.nd, groups = (nd + LB_BINS - 1u) / LB_BINS, nb = min(nd, LB_BINS);
+    const uint32_t bx0 = block % groups * LB_BINS, by = block / groups % nd, bz = block / (groups * nd);
+    if (block == 0u)  // bins of the lower LOD levels stay zero (single domain)
+        for (uint32_t i = L.n_bins * 4u + threadIdx.x; i < L.n_lod_own * 4u; i += LB_THREADS) L.qu_lod[i] = 0.0f;
+    const uint32_t cells = L.bsx * L.bsy * L.bsz;
+    const bool rows = L.bsx <= LB_SLAB;  // whole rows a slab
+    // neighbours a thread; rows of n bins, so a multiple of V cells keeps every access aligned
+    const uint32_t vec = !rows ? 1u : L.bsx % 4u == 0u ? 4u : L.bsx % 2u == 0u ? 2u : 1u;
+    const uint32_t slab = rows ? LB_SLAB / L.bsx * L.bsx : LB_SLAB, nslabs = (cells + slab - 1u) / slab;
+    const Magic mx(L.bsx), mxy(L.bsx * L.bsy), mq(L.bsx / vec);
+    const bool magic = (uint64_t)cells * (L.bsx * L.bsy) < (1ull << 32);  // Magic's bound (bins of <= ~2^16 cells)
+    auto load = [&](uint32_t k) {
+        float* const buf = sm.v[k & 1u];
+        const uint32_t base = k * slab, cnt = min(slab, cells - base);
+        const uint32_t x0 = bx0 * L.bsx, y0 = by * L.bsy, z0 = bz * L.bsz;
+        if (vec == 4u) lod_load<4>(L, buf, x0, y0, z0, nb, base, cnt, rows, magic, mx, mxy, mq);
+        else if (vec == 2u) lod_load<2>(L, buf, x0, y0, z0, nb, base, cnt, rows, magic, mx, mxy, mq);
+        else lod_load<1>(L, buf, x0, y0, z0, nb, base, cnt, rows, magic, mx, mxy, mq);
     };
     if (threadIdx.x >= 32u) load(0);
     __syncthreads();
@@ -131,25 +127,28 @@ static __global__ void __launch_bounds__(LB_THREADS) k_lod_bins(const DevLbm L) 
     for (uint32_t k = 0; k < nslabs; k++) {
         if (threadIdx.x >= 32u) {
             if (k + 1u < nslabs) load(k + 1u);
-        } else if (threadIdx.x < 4u) {
-            const uint32_t quads = (min(LB_SLAB, cells - k * LB_SLAB) + 3u) / 4u;
-            const float4* v = (const float4*)sm.v[k & 1u][threadIdx.x];
+        } else {
+            const uint32_t cnt = min(slab, cells - k * slab);
+            const float* v = sm.v[k & 1u] + threadIdx.x;
             uint32_t i = 0;
-            for (; i + 4u <= quads; i += 4u) {  // 16 cells: loads first, then the dependent additions
-                const float4 a = v[i], b = v[i + 1u], c = v[i + 2u], d = v[i + 3u];
-                acc = acc + a.x; acc = acc + a.y; acc = acc + a.z; acc = acc + a.w;
-                acc = acc + b.x; acc = acc + b.y; acc = acc + b.z; acc = acc + b.w;
-                acc = acc + c.x; acc = acc + c.y; acc = acc + c.z; acc = acc + c.w;
-                acc = acc + d.x; acc = acc + d.y; acc = acc + d.z; acc = acc + d.w;
+            for (; i + 16u <= cnt; i += 16u) {  // loads first, then the dependent additions
+                float a[16];
+#pragma unroll
+                for (uint32_t u = 0; u < 16u; u++) a[u] = v[(i + u) * LB_CELL];
+#pragma unroll
+                for (uint32_t u = 0; u < 16u; u++) acc = acc + a[u];
             }
-            for (; i < quads; i++) {
-                const float4 a = v[i];
-                acc = acc + a.x; acc = acc + a.y; acc = acc + a.z; acc = acc + a.w;
-            }
+            for (; i < cnt; i++) acc = acc + v[i * LB_CELL];
         }
         __syncthreads();
     }
-    if (threadIdx.x < 4u) L.qu_lod[(size_t)bin * 4u + threadIdx.x] = acc;
+    const uint32_t bin = threadIdx.x % LB_BINS, c = threadIdx.x / LB_BINS;
+    if (threadIdx.x < 32u && bin < nb) L.qu_lod[(size_t)(bx0 + bin + (by + bz * nd) * nd) * 4u + c] = acc;
+}
+
+static __global__ void __launch_bounds__(LB_THREADS) k_lod_bins(const DevLbm L) {
+    __shared__ LodSmem sm;
+    lod_bins_block(L, blockIdx.x, sm);
 }
 
 // ---------------------------------------------------------------------------

@@ -1321,9 +1321,7 @@ int ion_lbm_reset_kernel_time(ion_lbm* h) {
 }  // extern "C"
 
 namespace {
-constexpr uint32_t BARRIER_LIMIT = 1u << 26;  // polls (64 ns apart) before a grid barrier gives up
-static_assert(BARRIER_LIMIT == ION_BARRIER_LIMIT_DEFAULT && WAIT_LIMIT == ION_WAIT_LIMIT_DEFAULT,
-              "the header's documented defaults");
+static_assert(WAIT_LIMIT == ION_WAIT_LIMIT_DEFAULT, "the header's documented default");
 }
 
 struct ion_batch {
@@ -1346,8 +1344,7 @@ struct ion_batch {
     uint32_t gated_bricks = 0;
     uint32_t* d_row_off = nullptr;  // row-staged stencil: prefix sums of ny nz (null: tiles of cells)
     uint32_t total_rows = 0;
-    uint32_t* d_sync = nullptr;  // [0] barrier count, [1] barrier generation, [2] error
-    uint32_t barrier_limit = BARRIER_LIMIT;
+    uint32_t* d_err = nullptr;
     uint64_t t = 0;
     int sms = 0;
     bool tuned = false;
@@ -1376,10 +1373,7 @@ BatchDev batch_view(ion_batch* b, uint32_t block) {
     B.total_bricks = b->total_bricks[block_slot(block)];
     B.bin_off = b->d_bin_off;
     B.total_bins = b->total_bins;
-    B.bar_count = b->d_sync;
-    B.bar_gen = b->d_sync + 1;
-    B.err = b->d_sync + 2;
-    B.barrier_limit = b->barrier_limit;
+    B.err = b->d_err;
     B.row_off = b->d_row_off;
     B.total_rows = b->total_rows;
     return B;
@@ -1390,7 +1384,7 @@ BatchDev batch_view(ion_batch* b, uint32_t block) {
 cudaError_t batch_enqueue(ion_batch* b, uint32_t block, uint32_t grid, uint64_t t, uint32_t* launches) {
     const BatchDev B = batch_view(b, block);
     cudaError_t e = launch_batch_step(B, b->ft, b->mhd, b->fast, grid, block, t, b->stream);
-    *launches = b->mhd && B.total_bricks ? 2u : 1u;
+    *launches = !b->mhd ? 1u : B.total_bricks ? 3u : 2u;
     for (const auto& f : b->fft)
         if (e == cudaSuccess && !f.empty()) {
             *launches += launch_fft_batch(f.data(), (uint32_t)f.size(), b->stream);
@@ -1537,12 +1531,12 @@ int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out) {
     std::vector<uint32_t> bins(count + 1, 0);
     for (uint32_t i = 0; i < count; i++) {
         views[i] = domains[i]->L;
-        bins[i + 1] = bins[i] + (b->mhd ? domains[i]->L.n_lod_own : 0u);
+        bins[i + 1] = bins[i] + (b->mhd ? lod_blocks(domains[i]->L.nd) : 0u);
     }
     b->total_bins = bins[count];
     int rc = dalloc((void**)&b->d_doms, sizeof(DevLbm) * count);
     if (!rc) rc = dalloc((void**)&b->d_bin_off, sizeof(uint32_t) * (count + 1));
-    if (!rc) rc = dalloc((void**)&b->d_sync, sizeof(uint32_t) * 4);
+    if (!rc) rc = dalloc((void**)&b->d_err, sizeof(uint32_t));
     for (int s = 0; s < 2 && !rc; s++) {
         std::vector<uint32_t> tiles(count + 1, 0);
         const uint32_t per = kBatchBlocks[s] * EB_CPT;  // cells per tile
@@ -1579,7 +1573,7 @@ int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out) {
     }
     if (!rc && (cudaMemcpy(b->d_doms, views.data(), sizeof(DevLbm) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
                 cudaMemcpy(b->d_bin_off, bins.data(), sizeof(uint32_t) * (count + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
-                cudaMemset(b->d_sync, 0, sizeof(uint32_t) * 4) != cudaSuccess))
+                cudaMemset(b->d_err, 0, sizeof(uint32_t)) != cudaSuccess))
         rc = fail(ION_E_CUDA, "batch table upload");
     if (rc) { destroy_batch(b); return rc; }
     for (auto& e : b->ev) cudaEventCreate(&e);
@@ -1671,7 +1665,7 @@ int ion_batch_run(ion_batch* b, uint64_t steps) {
 int ion_batch_set_wait_limits(ion_batch* b, uint32_t barrier_polls, uint32_t tile_polls) {
     if (!b) return fail(ION_E_INVALID, "null batch");
     CK(cudaStreamSynchronize(b->stream));
-    b->barrier_limit = barrier_polls;
+    (void)barrier_polls;  // the step's phases are launches of their own: no grid barrier waits
     std::vector<DevLbm> views(b->doms.size());
     for (size_t i = 0; i < b->doms.size(); i++) {
         b->doms[i]->L.wait_limit = tile_polls;
@@ -1679,7 +1673,7 @@ int ion_batch_set_wait_limits(ion_batch* b, uint32_t barrier_polls, uint32_t til
         views[i] = b->doms[i]->L;
     }
     CK(cudaMemcpy(b->d_doms, views.data(), sizeof(DevLbm) * views.size(), cudaMemcpyHostToDevice));
-    if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }  // holds the old barrier limit
+    if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }  // (launched again with the new limits)
     b->graph_failed = false;
     return ION_OK;
 }
@@ -1696,10 +1690,10 @@ int ion_batch_finish(ion_batch* b, int timeout_ms) {
         std::this_thread::sleep_for(std::chrono::microseconds(50));
     }
     uint32_t err = 0;
-    CK(cudaMemcpy(&err, b->d_sync + 2, 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&err, b->d_err, 4, cudaMemcpyDeviceToHost));
     if (err) {
-        cudaMemset(b->d_sync, 0, 4 * sizeof(uint32_t));
-        return fail(ION_E_TIMEOUT, err == 2 ? "batch grid barrier timed out" : "batch field tile did not arrive in time");
+        cudaMemset(b->d_err, 0, sizeof(uint32_t));
+        return fail(ION_E_TIMEOUT, "batch field tile did not arrive in time");
     }
     return ION_OK;
 }

@@ -50,6 +50,9 @@ constexpr uint32_t EB_CPT = 4;
 // block one half of a brick (sub = 0, 1 in y).  FAST coordinates are taken
 // relative to the brick's centre, which depends only on the cell.
 constexpr uint32_t EB_BX = 16, EB_BY = 16;
+// LOD bins summed together by one block, neighbours along x
+constexpr uint32_t LB_BINS = 8;
+inline uint32_t lod_blocks(uint32_t nd) { return (nd + LB_BINS - 1u) / LB_BINS * nd * nd; }
 inline uint32_t eb_bricks(uint32_t nx, uint32_t ny, uint32_t nz) {
     return ((nx + EB_BX - 1) / EB_BX) * ((ny + EB_BY - 1) / EB_BY) * ((nz + EB_CPT - 1) / EB_CPT);
 }
@@ -62,12 +65,9 @@ struct BatchDev {
     uint32_t total_tiles;
     const uint32_t* brick_off;  // [ndom+1] prefix sums of bricks x (256 / blockDim) (E/B tiles)
     uint32_t total_bricks;
-    const uint32_t* bin_off;   // [ndom+1] prefix sums of n_lod_own
+    const uint32_t* bin_off;   // [ndom+1] prefix sums of lod_blocks (LOD bin groups; 1 at depth 0)
     uint32_t total_bins;
-    uint32_t* bar_count;
-    uint32_t* bar_gen;
     uint32_t* err;
-    uint32_t barrier_limit;  // polls before a grid barrier gives up
     const uint32_t* row_off;   // [ndom+1] prefix sums of ny nz (the row-staged stencil), or null
     uint32_t total_rows;       // 0: the stencil runs in tiles of cells with global loads
 };

@@ -486,7 +486,7 @@ class Batch:
         N.check(N.lib().ion_batch_run(self._h, int(steps)))
 
     def set_wait_limits(self, barrier_polls: int | None = None, tile_polls: int | None = None) -> None:
-        """Poll limits of the batch step's grid barriers and staged-tile waits (None: the defaults)."""
+        """Poll limit of the batch step's staged-tile waits (None: the default); ``barrier_polls`` is accepted, no wait uses it."""
         N.check(N.lib().ion_batch_set_wait_limits(
             self._h, N.ION_BARRIER_LIMIT_DEFAULT if barrier_polls is None else int(barrier_polls),
             N.ION_WAIT_LIMIT_DEFAULT if tile_polls is None else int(tile_polls)))
