@@ -107,46 +107,40 @@ __host__ __device__ __forceinline__ float bitsf(uint32_t u) {
 #endif
 }
 
-// v >> s with shifts of 32 or more giving 0 (PTX shr clamps the shift amount)
-__host__ __device__ __forceinline__ uint32_t shr_clamped(uint32_t v, uint32_t s) {
-#ifdef __CUDA_ARCH__
-    uint32_t r;
-    asm("shr.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(s));
-    return r;
-#else
-    return s >= 32u ? 0u : v >> s;
-#endif
-}
-
 // A NaN is encoded as the canonical quiet NaN 0x7FFFFFFF would be (the bit
 // pattern NVIDIA hardware gives every NaN result), so the stored value does
 // not depend on where a NaN came from.  The reference's MHD step produces
 // NaNs by itself: its electron density starts at 0 (sim_kernels.cl:823) and
 // reaches exactly 0 again, so u_e = 0/0 (sim_kernels.cl:230-232).
-__host__ __device__ __forceinline__ uint16_t fp16c_encode(float x) {
-    const uint32_t xb = fbits(x);
-    const uint32_t b = (((xb & 0x7FFFFFFFu) > 0x7F800000u) ? 0x7FFFFFFFu : xb) + 0x800u;
-    const uint32_t e = (b >> 23) & 0xFFu;
-    // both candidates, then a select (no divergent branch when a warp mixes normal and
-    // subnormal results).  Normal (e > 112): the exponent rebiased by -112 into 4 bits
-    // next to the top 11 mantissa bits, i.e. (b >> 12) - (112 << 11) in 15 bits.
-    // Subnormal: the 24-bit significand shifted by 124 - e, then halved with rounding;
-    // for e <= 100 the shift is 24 or more and the result 0, as the reference's
-    // (e > 100) factor gives.  Equal to the reference's expression for all 2^32 inputs.
-    const uint32_t nrm = ((b >> 12) - (112u << 11)) & 0x7FFFu;
-    const uint32_t sub = (shr_clamped((b & 0x007FFFFFu) + 0x007FF800u, 124u - e) + 1u) >> 1;
-    return (uint16_t)(((b >> 16) & 0x8000u) | (e > 112u ? nrm : sub));
+//
+// fp16c_encode_result: for the result of an arithmetic operation, whose NaN is canonical
+// already.  Normal (the exponent of b = bits + 2^11 above 112, i.e. |x| >= 0x387FF800): the
+// top 15 bits next to the sign are the code's, as rebiasing by -112 changes the exponent's bits
+// above the fourth only.  Subnormal: floor(|x| 2^25 + 1/2), the reference's shifted significand
+// halved with rounding; the two sums are rounded down, so no sum crosses an integer, and 2^23
+// brings the integer to the low bits.  The canonical NaN compares as normal and has the code
+// 0x8000.  Equal to the reference's expression for all 2^32 inputs.  8 instructions instead of
+// 18 (with the decoder below 314 M -> 254 M in the MHD stencil of
+// 192x160x128 cells, 406 -> 298 us).
+__host__ __device__ __forceinline__ uint16_t fp16c_encode_result(float x) {
+    const uint32_t b = fbits(x) + 0x800u;
+#ifdef __CUDA_ARCH__
+    const uint32_t sub = fbits(__fadd_rd(__fmaf_rd(fabsf(x), 33554432.0f, 0.5f), 8388608.0f));
+    const bool small = fabsf(x) < bitsf(0x387FF800u);
+#else
+    const bool small = (fbits(x) & 0x7FFFFFFFu) < 0x387FF800u;
+    const uint32_t sub = small ? (uint32_t)((double)bitsf(fbits(x) & 0x7FFFFFFFu) * 33554432.0 + 0.5) : 0u;
+#endif
+    return (uint16_t)(((small ? sub : b >> 12) & 0x7FFFu) | ((b >> 16) & 0x8000u));
 }
+__host__ __device__ __forceinline__ uint16_t fp16c_encode(float x) {
+    return fp16c_encode_result((fbits(x) & 0x7FFFFFFFu) > 0x7F800000u ? bitsf(0x7FFFFFFFu) : x);
+}
+// The code's exponent and mantissa as the bits of a float are 2^-112 times its value, with
+// exponent field 0 as the float's subnormals: one product by 2^112 (exact).  Equal to the
+// reference's decoder for all 2^16 inputs.
 __host__ __device__ __forceinline__ float fp16c_decode(uint16_t x) {
-    const uint32_t mag = x & 0x7FFFu, sign = (uint32_t)(x & 0x8000u) << 16;
-    // exponent field > 0: sign | (e + 112) << 23 | m << 12, one shift and one add.
-    // Exponent field 0: the same bits read as a float are 2^-15 + m 2^-26, so
-    // 2 (that) - 2^-14 = m 2^-25 exactly (one FMA, no integer conversion), which is the
-    // normalised float the reference's leading-zero count builds.  Equal to the
-    // reference's decoder for all 2^16 inputs.
-    const uint32_t nrm = (mag << 12) + (112u << 23);
-    const uint32_t sub = fbits(fmaf(bitsf(nrm), 2.0f, -6.103515625e-05f));
-    return bitsf(sign | (mag >= 0x0800u ? nrm : sub));
+    return bitsf(((uint32_t)(int32_t)(int16_t)x << 12) & 0x87FFFFFFu) * 5.192296858534828e33f;
 }
 
 // Packed FP32 pairs (PTX add/sub/mul/fma .f32x2, sm_100 and later): one
@@ -253,7 +247,7 @@ template <> struct Ddf<ION_FP16S> {
 template <> struct Ddf<ION_FP16C> {
     using T = uint16_t;
     __device__ __forceinline__ static float dec(uint16_t v) { return fp16c_decode(v); }
-    __device__ __forceinline__ static uint16_t enc(float x) { return fp16c_encode(x); }
+    __device__ __forceinline__ static uint16_t enc(float x) { return fp16c_encode_result(x); }
     __device__ __forceinline__ static float ld(const uint16_t* p, size_t i) { return dec(p[i]); }
     __device__ __forceinline__ static void st(uint16_t* p, size_t i, float x) { p[i] = enc(x); }
 };

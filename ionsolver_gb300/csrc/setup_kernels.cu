@@ -500,7 +500,7 @@ __global__ void k_codec(int ft, const float* in, uint16_t* enc, float* dec, cons
         dec[i] = Ddf<ION_FP16S>::ld(enc, i);
         raw_dec[i] = Ddf<ION_FP16S>::ld(raw, i);
     } else {
-        Ddf<ION_FP16C>::st(enc, i, in[i]);
+        enc[i] = fp16c_encode(in[i]);  // any NaN, where Ddf's takes results of arithmetic
         dec[i] = Ddf<ION_FP16C>::ld(enc, i);
         raw_dec[i] = Ddf<ION_FP16C>::ld(raw, i);
     }
