@@ -671,8 +671,8 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
 
 // Rows of up to 384 cells (WS_ROW): blockDim.x = compute threads + 32.  The last warp
 // stages rows and writes them back; the others compute (one cell per thread and row).
-// The row buffer has a fixed stride of RS elements per stream (the smallest of 128, 256
-// and 384 that holds the row: a small buffer keeps more CTAs per SM), so every
+// The row buffer has a fixed stride of RS elements per stream (the smallest of 96,
+// 128, 192, 256 and 384 that holds the row: a small buffer keeps more CTAs per SM), so every
 // shared-memory access of a cell is a register plus a constant offset.  The cells' new
 // DDFs go into the staged rows they were read from (RowDst), and the producer copies
 // each finished row's lattice streams back to their global rows with cp.async.bulk
@@ -680,20 +680,23 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
 // so no other CTA touches them within the step.  The other outputs (q, the LOD
 // velocity, rho, u) are stored directly.
 constexpr uint32_t WS_ROW = 384;
-__host__ __device__ constexpr uint32_t ws_stride(uint32_t nx) { return nx <= 128u ? 128u : nx <= 256u ? 256u : 384u; }
+__host__ __device__ constexpr int ws_variant(uint32_t nx) { return nx <= 96u ? 0 : nx <= 128u ? 1 : nx <= 192u ? 2 : nx <= 256u ? 3 : 4; }
 template <int FT, bool MHD, uint32_t RS>
 __host__ __device__ constexpr uint32_t ws_row_bytes() {
     return row_streams<FT, MHD>() * RS * (uint32_t)sizeof(typename Ddf<FT>::T) + (MHD ? 6u * RS * 4u : 0u) + RS;
 }
 
-// Rows of up to 256 cells: three CTAs of up to 288 threads per SM (72 registers; FP16
-// MHD rows of 256 cells then run 24 compute warps per SM instead of 16: 0.920 -> 0.845
-// ms at 256^3 FP16S), except MHD with TRT, which spills at 72 registers.  Rows of up to
-// 384 cells: two CTAs of up to 416 threads (78 registers), one for MHD with TRT.
+// About 72 registers a thread: three CTAs of up to 288 threads per SM at a stride of 256 (FP16
+// MHD rows of 256 cells then run 24 compute warps per SM instead of 16: 0.920 -> 0.845 ms at
+// 256^3 FP16S), four of 224 at 192, five of 160 at 128 and seven of 128 at 96, except MHD with
+// TRT, which spills there.  Rows of up to 384 cells: two CTAs of up to 416 threads (78
+// registers), one for MHD with TRT.
 template <uint32_t RS>
-__host__ __device__ constexpr int ws_threads() { return RS == 384u ? 416 : 288; }
+__host__ __device__ constexpr int ws_threads() { return (int)RS + 32; }
 template <uint32_t RS, bool MHD, bool TRT>
-__host__ __device__ constexpr int ws_min_ctas() { return RS == 384u ? ((MHD && TRT) ? 1 : 2) : ((MHD && TRT) ? 2 : 3); }
+__host__ __device__ constexpr int ws_min_ctas() {
+    return RS == 384u ? ((MHD && TRT) ? 1 : 2) : ((MHD && TRT) ? 576 : 896) / ws_threads<RS>();
+}
 template <int FT, bool MHD, bool TRT, uint32_t RS>
 __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_t, uint32_t* err) {
     using T = typename Ddf<FT>::T;
@@ -798,26 +801,29 @@ template <int FT, bool MHD, bool TRT>
 bool launch_sc_rows(const DevLbm& L, uint32_t o, uint32_t* err, cudaStream_t s) {
     // whole 16-byte rows, two buffers in shared memory, and 32-bit slot offsets (19 N < 2^32)
     const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
-    const uint32_t rs = ws ? ws_stride(L.nx) : 0u;
+    const int v = ws ? ws_variant(L.nx) : 5;
     static_assert(2u * ws_row_bytes<ION_FP32, true, WS_ROW>() <= 200u * 1024u, "two row buffers of the widest form");
-    const uint32_t smem = 2u * (rs == 128u   ? ws_row_bytes<FT, MHD, 128u>()
-                                : rs == 256u ? ws_row_bytes<FT, MHD, 256u>()
-                                : rs == 384u ? ws_row_bytes<FT, MHD, 384u>()
-                                             : row_bytes<FT, MHD>(L.nx));
+    const uint32_t smem = 2u * (v == 0   ? ws_row_bytes<FT, MHD, 96u>()
+                                : v == 1 ? ws_row_bytes<FT, MHD, 128u>()
+                                : v == 2 ? ws_row_bytes<FT, MHD, 192u>()
+                                : v == 3 ? ws_row_bytes<FT, MHD, 256u>()
+                                : v == 4 ? ws_row_bytes<FT, MHD, 384u>()
+                                         : row_bytes<FT, MHD>(L.nx));
     if (L.nx % 16u || smem > 200u * 1024u || 19ull * L.n >= (1ull << 32)) return false;
     const uint32_t threads =
         ws ? (L.nx + 31u) / 32u * 32u + 32u : ((L.nx + ((L.nx + 255u) / 256u) - 1u) / ((L.nx + 255u) / 256u) + 31u) / 32u * 32u;
-    auto kern = rs == 128u   ? k_sc_rows_ws<FT, MHD, TRT, 128u>
-                : rs == 256u ? k_sc_rows_ws<FT, MHD, TRT, 256u>
-                : rs == 384u ? k_sc_rows_ws<FT, MHD, TRT, 384u>
-                             : k_sc_rows<FT, MHD, TRT>;
+    auto kern = v == 0   ? k_sc_rows_ws<FT, MHD, TRT, 96u>
+                : v == 1 ? k_sc_rows_ws<FT, MHD, TRT, 128u>
+                : v == 2 ? k_sc_rows_ws<FT, MHD, TRT, 192u>
+                : v == 3 ? k_sc_rows_ws<FT, MHD, TRT, 256u>
+                : v == 4 ? k_sc_rows_ws<FT, MHD, TRT, 384u>
+                         : k_sc_rows<FT, MHD, TRT>;
     // the shared-memory opt-in and the occupancy of the last shape, per instantiation
     // (handles may step on several host threads)
     static std::mutex mu;
-    static bool attr[4] = {false, false, false, false};
-    static int per_sm_of[4] = {0, 0, 0, 0};
-    static uint32_t for_smem[4] = {0, 0, 0, 0}, for_threads[4] = {0, 0, 0, 0};
-    const int v = (int)(rs / 128u);
+    static bool attr[6] = {};
+    static int per_sm_of[6] = {};
+    static uint32_t for_smem[6] = {}, for_threads[6] = {};
     int per_sm = 0;
     {
         std::lock_guard<std::mutex> lock(mu);
