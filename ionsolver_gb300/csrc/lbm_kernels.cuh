@@ -305,15 +305,28 @@ __device__ __forceinline__ float force_dir(const ForceState& s, int i) {
     return (9.0f * V::w(V::wc(i))) * fmaf(cf, cu, s.uF);
 }
 
+// the equilibrium itself (sim_kernels.cl:719-723 / 651-655)
+template <class V, class DST>
+__device__ __forceinline__ void eq_store(const DST& o, const EqState& es) {
+    o.st0(eq_zero<V>(es));
+#pragma unroll
+    for (int i = 1; i < V::q; i += 2) {
+        float fa, fb;
+        eq_pair<V>(es, i, fa, fb);
+        o.st_nbr(i, fa);
+        o.st_own(i, fb);
+    }
+}
+
 // SRT collision + Esoteric-Pull store (sim_kernels.cl:714-723 / 649-656).
 // force: 0 = none (Fin = 0), 1 = Guo terms scaled by c_tau.
 template <class V, class DST>
 __device__ __forceinline__ void srt_store(const DST& o, const float* fh, const EqState& es, const ForceState& fs,
-                                          bool force, float c_tau, float w, bool eqc) {
+                                          bool force, float c_tau, float w) {
     {
         const float feq = eq_zero<V>(es);
         const float F = force ? force_dir<V>(fs, 0) * c_tau : 0.0f;
-        o.st0(eqc ? feq : fmaf(1.0f - w, fh[0], fmaf(w, feq, F)));
+        o.st0(fmaf(1.0f - w, fh[0], fmaf(w, feq, F)));
     }
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
@@ -321,17 +334,15 @@ __device__ __forceinline__ void srt_store(const DST& o, const float* fh, const E
         eq_pair<V>(es, i, fa, fb);
         const float Fa = force ? force_dir<V>(fs, i) * c_tau : 0.0f;
         const float Fb = force ? force_dir<V>(fs, i + 1) * c_tau : 0.0f;
-        const float va = eqc ? fa : fmaf(1.0f - w, fh[i], fmaf(w, fa, Fa));
-        const float vb = eqc ? fb : fmaf(1.0f - w, fh[i + 1], fmaf(w, fb, Fb));
-        o.st_nbr(i, va);
-        o.st_own(i, vb);
+        o.st_nbr(i, fmaf(1.0f - w, fh[i], fmaf(w, fa, Fa)));
+        o.st_own(i, fmaf(1.0f - w, fh[i + 1], fmaf(w, fb, Fb)));
     }
 }
 
 // TRT collision + store (sim_kernels.cl:725-754)
 template <class V, class DST>
 __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const EqState& es, const ForceState& fs,
-                                          bool force, float w, bool eqc) {
+                                          bool force, float w) {
     const float wp = w, wm = 1.0f / (0.1875f / (1.0f / w - 0.5f) + 0.5f);
     const float ctp = fmaf(wp, -0.25f, 0.5f), ctm = fmaf(wm, -0.25f, 0.5f);
     {
@@ -343,7 +354,7 @@ __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const E
         }
         const float sym = ((feq - fh[0]) + feq) - fh[0];
         const float asym = ((feq - feq) - fh[0]) + fh[0];
-        o.st0(eqc ? feq : fmaf(0.5f * wp, sym, fmaf(0.5f * wm, asym, fh[0] + F)));
+        o.st0(fmaf(0.5f * wp, sym, fmaf(0.5f * wm, asym, fh[0] + F)));
     }
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
@@ -356,10 +367,8 @@ __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const E
             Fb = fmaf(ctp, B + A, ctm * (B - A));
         }
         const float ha = fh[i], hb = fh[i + 1];
-        const float va = eqc ? ea : fmaf(0.5f * wp, ((ea - ha) + eb) - hb, fmaf(0.5f * wm, ((ea - eb) - ha) + hb, ha + Fa));
-        const float vb = eqc ? eb : fmaf(0.5f * wp, ((eb - hb) + ea) - ha, fmaf(0.5f * wm, ((eb - ea) - hb) + ha, hb + Fb));
-        o.st_nbr(i, va);
-        o.st_own(i, vb);
+        o.st_nbr(i, fmaf(0.5f * wp, ((ea - ha) + eb) - hb, fmaf(0.5f * wm, ((ea - eb) - ha) + hb, ha + Fa)));
+        o.st_own(i, fmaf(0.5f * wp, ((eb - hb) + ea) - ha, fmaf(0.5f * wm, ((eb - ea) - hb) + ha, hb + Fb)));
     }
 }
 
@@ -498,7 +507,7 @@ __device__ __forceinline__ void sc_cell(const DevLbm& L, const uint32_t n, const
                     L.lod_cell[2 * (size_t)N + n] = uz * L.ils;
                 }
             }
-            if (L.ext_vf) {
+            if (MHD || L.ext_vf) {
                 const float r2 = 0.5f / rho;
                 ux = clampf(fmaf(fx, r2, ux), -CS, CS);
                 uy = clampf(fmaf(fy, r2, uy), -CS, CS);
@@ -512,13 +521,16 @@ __device__ __forceinline__ void sc_cell(const DevLbm& L, const uint32_t n, const
                 L.rho[n] = rho;
                 L.u[n] = ux; L.u[(size_t)N + n] = uy; L.u[2 * (size_t)N + n] = uz;
             }
-            force = L.ext_vf;
+            force = MHD || L.ext_vf;  // (a configuration with MHD has the volume force)
         }
         const EqState es = eq_state(rho, ux, uy, uz);
         const ForceState fs = force_state<V>(ux, uy, uz, fx, fy, fz);
         const auto dst = S.template dst<D, Q, IX>(f, N, n, odd, j, lat);
-        if (TRT && !electrons) trt_store<V>(dst, fh, es, fs, force, w, eqc);
-        else srt_store<V>(dst, fh, es, fs, force, c_tau, w, eqc);
+        // boundary cells store the equilibrium: a branch of its own, as a select per value costs
+        // every cell of a domain without them
+        if (eqc) eq_store<V>(dst, es);
+        else if (TRT && !electrons) trt_store<V>(dst, fh, es, fs, force, w);
+        else srt_store<V>(dst, fh, es, fs, force, c_tau, w);
     }
 }
 
