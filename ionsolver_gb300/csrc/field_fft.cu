@@ -333,43 +333,45 @@ __device__ __forceinline__ void fft_sum(const DevLbm& L, const FftField& F, cons
 }
 
 // ---------------------------------------------------------------------------
-// the sums to the cells: block = (0: E, 1: B) + 2 (x tile + tiles (Iz + nd (oy + bsy (oz - oz0))));
-// a block transposes nd rows (y = Iy bsy + oy) of up to PUT_X cells, three components,
+// the sums to the cells: block = (0: E, 1: B) + 2 (tile + tiles (Iz + nd (oz - oz0))); a block
+// transposes PUT_X neighbouring (oy, x) of nd rows each (y = Iy bsy + oy), three components,
 // through shared memory.  A thread's loads are all in flight before the first is used, and the
-// components share its indices (one component a block, loads one after another: 55 us at 128^3)
+// components share its indices (one component a block, loads one after another: 55 us at
+// 128^3; tiles of one oy leave lanes idle on rows below PUT_X cells)
 // ---------------------------------------------------------------------------
 template <int ND>
 __device__ __forceinline__ void fft_put(const DevLbm& L, const FftField& F, uint32_t block, const uint32_t oz0) {
     __shared__ float s[3][ND][PUT_X + 1];
-    const uint32_t tiles = (L.nx + PUT_X - 1u) / PUT_X;
+    const uint32_t plane_xy = L.bsy * L.nx, tiles = (plane_xy + PUT_X - 1u) / PUT_X;
     const bool B = block & 1u;
     block >>= 1;
-    const uint32_t x0 = block % tiles * PUT_X;
+    const uint32_t e0 = block % tiles * PUT_X;
     block /= tiles;
-    const uint32_t Iz = block % ND, oy = block / ND % L.bsy, ozl = block / (ND * L.bsy);
-    const uint32_t cnt = min(PUT_X, L.nx - x0);
+    const uint32_t Iz = block % ND, ozl = block / ND;
     const size_t N = L.n, plane = (size_t)F.chunk * L.bsy * L.bsx * (ND * ND * ND);
-    const float* in = F.out + (B ? 3u : 0u) * plane + ((size_t)ozl * L.bsy + oy) * L.bsx * (ND * ND * ND) + Iz * ND;
+    const float* in = F.out + (B ? 3u : 0u) * plane + (size_t)ozl * L.bsy * L.bsx * (ND * ND * ND) + Iz * ND;
     const uint32_t Iy = threadIdx.x % ND;
     constexpr uint32_t XS = PUT_THREADS / ND, GET = PUT_X / XS;  // cells apart, cells per thread
     float v[3][GET];
 #pragma unroll
     for (uint32_t k = 0; k < GET; k++) {
-        const uint32_t xl = threadIdx.x / ND + k * XS, x = x0 + xl, Ix = x / L.bsx, ox = x - Ix * L.bsx;
-        const float* p = in + (size_t)(ox * ND + Ix) * (ND * ND) + Iy;
+        const uint32_t e = e0 + threadIdx.x / ND + k * XS;
+        const uint32_t oy = L.dx.div(e), x = e - oy * L.nx, Ix = x / L.bsx, ox = x - Ix * L.bsx;
+        const float* p = in + (size_t)((oy * L.bsx + ox) * ND + Ix) * (ND * ND) + Iy;
 #pragma unroll
-        for (uint32_t c = 0; c < 3; c++) v[c][k] = xl < cnt ? __ldcs(p + c * plane) : 0.0f;
+        for (uint32_t c = 0; c < 3; c++) v[c][k] = e < plane_xy ? __ldcs(p + c * plane) : 0.0f;
     }
     const uint32_t z = Iz * L.bsz + oz0 + ozl;
     constexpr uint32_t PUT = PUT_X * ND / PUT_THREADS, YS = PUT_THREADS / PUT_X;
-    const uint32_t xl = threadIdx.x % PUT_X, y0 = threadIdx.x / PUT_X;
-    const uint32_t n0 = x0 + xl + (oy + y0 * L.bsy + z * L.ny) * L.nx, row = YS * L.bsy * L.nx;
+    const uint32_t xl = threadIdx.x % PUT_X, y0 = threadIdx.x / PUT_X, e = e0 + xl;
+    const uint32_t oy = L.dx.div(e), x = e - oy * L.nx;
+    const uint32_t n0 = x + (oy + y0 * L.bsy + z * L.ny) * L.nx, row = YS * L.bsy * L.nx;
     const float* const stat = B ? L.b_stat : L.e_stat;
     float* const dyn = B ? L.b_dyn : L.e_dyn;
     const float scale = B ? L.kmu : L.ke;
     bool on[PUT];
 #pragma unroll
-    for (uint32_t k = 0; k < PUT; k++) on[k] = xl < cnt && (L.flags[n0 + k * row] & F_BO) != F_S;
+    for (uint32_t k = 0; k < PUT; k++) on[k] = e < plane_xy && (L.flags[n0 + k * row] & F_BO) != F_S;
 #pragma unroll
     for (uint32_t c = 0; c < 3; c++)
 #pragma unroll
@@ -528,7 +530,7 @@ uint32_t fft_sum_blocks(const DevLbm& L, const FftField& F, uint32_t pass) {
     return 6u * chunk_len(L, F, pass) * L.bsy * L.bsx;
 }
 uint32_t fft_put_blocks(const DevLbm& L, const FftField& F, uint32_t pass) {
-    return 2u * ((L.nx + PUT_X - 1u) / PUT_X) * L.nd * L.bsy * chunk_len(L, F, pass);
+    return 2u * ((L.bsy * L.nx + PUT_X - 1u) / PUT_X) * L.nd * chunk_len(L, F, pass);
 }
 
 uint32_t launch_fft_batch(const FftBatch* B, uint32_t passes, cudaStream_t s) {
