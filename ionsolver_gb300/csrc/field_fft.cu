@@ -388,20 +388,31 @@ __device__ __forceinline__ void fft_put(const DevLbm& L, const FftField& F, uint
     }
 }
 
+// gate: null, or the kernels run only when *gate != 0.  Then resident blocks walk the work, so
+// that a closed gate costs little; without a gate the grid has a block for each.
 template <int ND>
-__global__ void __launch_bounds__(SRC_THREADS) k_fft_src(const DevLbm L, const FftField F) {
+__global__ void __launch_bounds__(SRC_THREADS) k_fft_src(const DevLbm L, const FftField F, const uint32_t* gate) {
+    if (gate && *gate == 0u) return;
     fft_src<ND>(L, F, blockIdx.x);
 }
 template <int ND>
-__global__ void __launch_bounds__(SUM_THREADS, SUM_BLOCKS) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0) {
+__global__ void __launch_bounds__(SUM_THREADS, SUM_BLOCKS) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0,
+                                                                     const uint32_t* gate, const uint32_t blocks) {
     extern __shared__ __align__(16) float2 sum_sm[];
-    if (*F.direct) return;
-    fft_sum<ND>(L, F, blockIdx.x, oz0, sum_sm);
+    if ((gate && *gate == 0u) || *F.direct) return;
+    for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+        fft_sum<ND>(L, F, b, oz0, sum_sm);
+        if (gate) __syncthreads();
+    }
 }
 template <int ND>
-__global__ void __launch_bounds__(PUT_THREADS) k_fft_put(const DevLbm L, const FftField F, const uint32_t oz0) {
-    if (*F.direct) return;
-    fft_put<ND>(L, F, blockIdx.x, oz0);
+__global__ void __launch_bounds__(PUT_THREADS) k_fft_put(const DevLbm L, const FftField F, const uint32_t oz0,
+                                                         const uint32_t* gate, const uint32_t blocks) {
+    if ((gate && *gate == 0u) || *F.direct) return;
+    for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+        fft_put<ND>(L, F, b, oz0);
+        if (gate) __syncthreads();
+    }
 }
 
 // the same blocks over many domains (FftBatch): a block's domain by its prefix sums
@@ -470,11 +481,19 @@ uint32_t chunk_len(const DevLbm& L, const FftField& F, uint32_t pass) {
 }
 
 template <int ND>
-uint32_t launch_field_nd(const DevLbm& L, const FftField& F, cudaStream_t s) {
-    k_fft_src<ND><<<fft_src_blocks(L), SRC_THREADS, 0, s>>>(L, F);
+uint32_t launch_field_nd(const DevLbm& L, const FftField& F, const uint32_t* gate, cudaStream_t s) {
+    uint32_t resident = 0xFFFFFFFFu;
+    if (gate) {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        resident = SUM_BLOCKS * (uint32_t)(sms > 0 ? sms : 1);
+    }
+    k_fft_src<ND><<<fft_src_blocks(L), SRC_THREADS, 0, s>>>(L, F, gate);
     for (uint32_t p = 0; p < fft_passes(L, F); p++) {
-        k_fft_sum<ND><<<fft_sum_blocks(L, F, p), SUM_THREADS, sum_smem(ND), s>>>(L, F, p * F.chunk);
-        k_fft_put<ND><<<fft_put_blocks(L, F, p), PUT_THREADS, 0, s>>>(L, F, p * F.chunk);
+        const uint32_t sum = fft_sum_blocks(L, F, p), put = fft_put_blocks(L, F, p), oz = p * F.chunk;
+        k_fft_sum<ND><<<sum < resident ? sum : resident, SUM_THREADS, sum_smem(ND), s>>>(L, F, oz, gate, sum);
+        k_fft_put<ND><<<put < resident ? put : resident, PUT_THREADS, 0, s>>>(L, F, oz, gate, put);
     }
     return 1u + 2u * fft_passes(L, F);
 }
@@ -537,8 +556,8 @@ uint32_t launch_fft_batch(const FftBatch* B, uint32_t passes, cudaStream_t s) {
     return B->nd == 16u ? launch_batch_nd<16>(B, passes, s) : launch_batch_nd<8>(B, passes, s);
 }
 
-uint32_t launch_fft_field(const DevLbm& L, const FftField& F, cudaStream_t s) {
-    return L.nd == 16u ? launch_field_nd<16>(L, F, s) : launch_field_nd<8>(L, F, s);
+uint32_t launch_fft_field(const DevLbm& L, const FftField& F, const uint32_t* gate, cudaStream_t s) {
+    return L.nd == 16u ? launch_field_nd<16>(L, F, gate, s) : launch_field_nd<8>(L, F, gate, s);
 }
 
 }  // namespace ion

@@ -27,8 +27,9 @@ bool fft_field_fits(const DevLbm& L);
 void fft_field_sizes(const DevLbm& L, FftField& F, size_t* g_bytes, size_t* s_bytes, size_t* out_bytes);
 cudaError_t launch_fft_plan(const DevLbm& L, const FftField& F, cudaStream_t s);
 // sources -> spectra, sums of every cell, E/B; returns the number of launches.  F.direct is
-// left non-zero (and E/B untouched) when the direct sum has to run instead.
-uint32_t launch_fft_field(const DevLbm& L, const FftField& F, cudaStream_t s);
+// left non-zero (and E/B untouched) when the direct sum has to run instead.  gate: null, or
+// nothing runs while *gate is 0.
+uint32_t launch_fft_field(const DevLbm& L, const FftField& F, const uint32_t* gate, cudaStream_t s);
 
 // blocks of the three kernels; the sums of a large grid go in passes of F.chunk z offsets
 uint32_t fft_passes(const DevLbm& L, const FftField& F);

@@ -271,7 +271,8 @@ int setup_field(ion_lbm* h) {
         g_launches++;
         h->table = T;
     }
-    if (h->fft.G || h->cfg.field_mode != ION_FIELD_FAST || !fft_field_fits(h->L)) return ION_OK;
+    // (SURROGATE handles fall back to the FAST field)
+    if (h->fft.G || h->cfg.field_mode == ION_FIELD_BITWISE || !fft_field_fits(h->L)) return ION_OK;
     FftField F;
     size_t bytes[4] = {0, 0, 0, 4};
     fft_field_sizes(h->L, F, &bytes[0], &bytes[1], &bytes[2]);
@@ -292,9 +293,9 @@ int setup_field(ion_lbm* h) {
 }
 
 int launch_field(ion_lbm* h) {
-    if (h->cfg.field_mode == ION_FIELD_FAST && h->fft.G) {
-        g_launches += launch_fft_field(h->L, h->fft, h->stream) + 1;
-        launch_update_e_b_gated(h->L, h->d_err, h->fft.direct, h->stream);
+    if (h->cfg.field_mode != ION_FIELD_BITWISE && h->fft.G) {
+        g_launches += launch_fft_field(h->L, h->fft, nullptr, h->stream) + 1;
+        launch_update_e_b_gated(h->L, h->d_err, h->fft.direct, nullptr, h->stream);
         CKL();
         return ION_OK;
     }
@@ -315,8 +316,11 @@ int launch_surrogate_field(ion_lbm* h) {
     if (!h->sur || !h->sur->ready())
         return fail(ION_E_STATE, "field_mode SURROGATE: train (ion_lbm_surrogate_train) or load the network first");
     h->sur->step(h->L, h->stream, 0x2545F491u);
-    launch_update_e_b_gated(h->L, h->d_err, h->sur->fallback_flag(), h->stream);
-    g_launches += h->sur->launches_per_step() + 1;
+    // the fallback is the FAST field, bit for bit: its convolution, or the direct sum
+    uint32_t launches = h->sur->launches_per_step() + 1;
+    if (h->fft.G) launches += launch_fft_field(h->L, h->fft, h->sur->fallback_flag(), h->stream);
+    launch_update_e_b_gated(h->L, h->d_err, h->sur->fallback_flag(), h->fft.G ? h->fft.direct : nullptr, h->stream);
+    g_launches += launches;
     CKL();
     return ION_OK;
 }
@@ -368,7 +372,7 @@ int enqueue_step(ion_lbm* h, uint64_t t) {
 uint32_t kernels_per_step(const ion_lbm* h) {
     uint32_t k = 1u + (h->cfg.ext_magneto_hydro ? (h->L.depth > 0 ? 2u : 1u) : 0u);
     if (h->cfg.ext_magneto_hydro && h->cfg.field_mode == ION_FIELD_SURROGATE && h->sur) k += h->sur->launches_per_step();
-    if (h->cfg.ext_magneto_hydro && h->cfg.field_mode == ION_FIELD_FAST && h->fft.G) k += 1u + 2u * fft_passes(h->L, h->fft);
+    if (h->cfg.ext_magneto_hydro && h->cfg.field_mode != ION_FIELD_BITWISE && h->fft.G) k += 1u + 2u * fft_passes(h->L, h->fft);
     return k;
 }
 

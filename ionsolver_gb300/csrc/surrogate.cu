@@ -508,6 +508,7 @@ __global__ void k_source_scale(const float* qu_lod, int V, int first, float* sca
     __shared__ float mean[4];
     const float4* qu = (const float4*)qu_lod;
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll 8
     for (int v = first + threadIdx.x; v < V; v += blockDim.x) {
         const float4 L = qu[v];
         s0 += L.x; s1 += L.x * L.y; s2 += L.x * L.z; s3 += L.x * L.w;
@@ -522,6 +523,7 @@ __global__ void k_source_scale(const float* qu_lod, int V, int first, float* sca
     if (threadIdx.x < 4) mean[threadIdx.x] = V > first ? (float)(r[threadIdx.x][0] / (double)(V - first)) : 0.0f;
     __syncthreads();
     float mq = 0.0f, mv = 0.0f;
+#pragma unroll 8
     for (int v = first + threadIdx.x; v < V; v += blockDim.x) {
         const float4 L = qu[v];
         mq = fmaxf(mq, fabsf(L.x - mean[0]));
@@ -582,7 +584,7 @@ __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, con
                                                int by, int bz, uint32_t tile, uint32_t cells, const Magic& mx,
                                                const Magic& mxy);
 
-__global__ void __launch_bounds__(SC_THREADS, 2) k_surrogate_cells(const DevLbm L, const float* Y, const float* G,
+__global__ void __launch_bounds__(SC_THREADS, 3) k_surrogate_cells(const DevLbm L, const float* Y, const float* G,
                                                                 const float* scales, float yE, float yB) {
     extern __shared__ __align__(16) uint8_t sur_smem[];  // SurSmem, then the t2 table
     SurSmem& sm = *reinterpret_cast<SurSmem*>(sur_smem);
@@ -639,8 +641,9 @@ __global__ void __launch_bounds__(SC_THREADS, 2) k_surrogate_cells(const DevLbm 
         sm.wyz[a][l] = make_float4(w[0], w[1], w[2], 0.0f);
     }
     __syncthreads();
-    // contracted along y as well: t2[(ly bsx + lx) 3 + iz][c] = sum_iy wy_iy(ly) t1[lx][iy + 3 iz][c],
-    // behind SurSmem in dynamic shared memory (bsx bsy 3 x 8 floats)
+    // contracted along y as well: t2[ly bsx + lx][iz][c] = sum_iy wy_iy(ly) t1[lx][iy + 3 iz][c],
+    // behind SurSmem in dynamic shared memory (bsx bsy rows of 3 x 8 floats, 28 apart: the eight
+    // lanes of a 16-byte access then read different banks)
     float4* t2 = reinterpret_cast<float4*>(sur_smem + sizeof(SurSmem));
     for (uint32_t i = threadIdx.x; i < L.bsx * L.bsy * 24u; i += blockDim.x) {
         const uint32_t c = i % 8u, iz = (i / 8u) % 3u, lx = (i / 24u) % L.bsx, ly = i / (24u * L.bsx);
@@ -652,7 +655,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) k_surrogate_cells(const DevLbm 
             v = fmaf(wy.y, t[(1u + 3u * iz) * 8u + c], v);
             v = fmaf(wy.z, t[(2u + 3u * iz) * 8u + c], v);
         }
-        ((float*)t2)[i] = v;
+        ((float*)t2)[(ly * L.bsx + lx) * 28u + iz * 8u + c] = v;
     }
     __syncthreads();
 
@@ -704,14 +707,11 @@ __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, con
         far_zero(fs[j]);
     }
     const uint32_t cnt = sm.count;
-    // the next source's values are read from shared memory while this one is summed
-    FastSrc S = sm.src[0];
 #pragma unroll 1
     for (uint32_t s = 0; s < cnt; s++) {
-        const FastSrc Sn = sm.src[s + 1u < cnt ? s + 1u : s];
+        const FastSrc S = sm.src[s];
 #pragma unroll
         for (uint32_t j = 0; j < SC_CPT / 2; j++) far_fast2(cp[j], cc[j], S, fs[j]);
-        S = Sn;
     }
     asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
@@ -725,7 +725,7 @@ __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, con
         // triquadratic interpolation: the x and y contractions are tabulated per bin (t2)
         const float4 wz = sm.wyz[1][lz];
         const float wz3[3] = {wz.x, wz.y, wz.z};
-        const float4* tc = t2 + (size_t)((ly * L.bsx + lx) * 3u) * 2u;
+        const float4* tc = t2 + (size_t)(ly * L.bsx + lx) * 7u;
         float far[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int iz = 0; iz < 3; iz++) {
@@ -781,11 +781,22 @@ __global__ void __launch_bounds__(128) k_sample_check(const DevLbm L, uint32_t c
     float e[3] = {0, 0, 0}, b[3] = {0, 0, 0};
     const float4* qu = (const float4*)L.qu_lod;
     const uint32_t last = src_last<true>(L);  // bins from 8^D on are always zero
-    for (uint32_t d = L.first_src + lane; d < last; d += 32u) {
-        if (d == own) continue;
-        const float4 p = L.lod_pos[d], v = qu[d];
-        add_src<true>((float)x - p.x, (float)y - p.y, (float)z - p.z, make_float4(v.x, v.x * v.y, v.x * v.z, v.x * v.w),
-                      e, b);
+    constexpr uint32_t AHEAD = 8;  // bins whose loads are in flight together (one at a time: 101 us for 1024 cells)
+    for (uint32_t d0 = L.first_src + lane; d0 < last; d0 += 32u * AHEAD) {
+        float4 p[AHEAD], v[AHEAD];
+#pragma unroll
+        for (uint32_t k = 0; k < AHEAD; k++) {
+            const uint32_t d = min(d0 + 32u * k, last - 1u);
+            p[k] = L.lod_pos[d];
+            v[k] = qu[d];
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < AHEAD; k++) {
+            const uint32_t d = d0 + 32u * k;
+            if (d >= last || d == own) continue;
+            add_src<true>((float)x - p[k].x, (float)y - p[k].y, (float)z - p[k].z,
+                          make_float4(v[k].x, v[k].x * v[k].y, v[k].x * v[k].z, v[k].x * v[k].w), e, b);
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -892,7 +903,7 @@ int Surrogate::init(int nd, float bsx, float bsy, float bsz, int first_src) {
     rc |= alloc((void**)&xb_, (size_t)16 * V_ * 2);
     if (rc) return ION_E_NOMEM;
     if (cudaFuncSetAttribute(k_surrogate_cells, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(SurSmem) + (size_t)MAX_BLOCK * MAX_BLOCK * 96u)) !=
+                             (int)(sizeof(SurSmem) + (size_t)MAX_BLOCK * MAX_BLOCK * 112u)) !=
         cudaSuccess)
         return ION_E_CUDA;
     // far field of a unit charge in every source bin at the 27 nodes: the field of
@@ -1172,7 +1183,7 @@ void Surrogate::step(const DevLbm& L, cudaStream_t s, uint32_t salt) {
     k_source_scale<<<1, 256, 0, s>>>(L.qu_lod, V_, first_, scales_);
     k_pack_input_dev(L, s);
     infer_bf16(xin_, s);
-    k_surrogate_cells<<<L.n_bins, SC_THREADS, sizeof(SurSmem) + (size_t)L.bsx * L.bsy * 96u, s>>>(L, yout_, gunit_,
+    k_surrogate_cells<<<L.n_bins, SC_THREADS, sizeof(SurSmem) + (size_t)L.bsx * L.bsy * 112u, s>>>(L, yout_, gunit_,
                                                                                                  scales_, yE_, yB_);
     k_sample_check<<<blocks_for((size_t)check_cells_ * 32, 128), 128, 0, s>>>(L, check_cells_, salt, stats_, counters_);
     k_sample_decide<<<1, 1, 0, s>>>(stats_, tol_, flag_, last_, counters_);
