@@ -23,8 +23,9 @@
 // Rounding: a 32-bit transform's error is about 1.5e-7 of the field's norm (the direct
 // 32-bit sums: 1.1e-6), spread evenly over the lattice.  An infinite bin would leave NaN
 // where the direct sum keeps the sign, and sums near the ends of the exponent range would
-// over- or underflow at other places; so for sources that are not finite, or whose largest
-// value lies outside [1e-28, 1e25], `direct` is set and k_update_e_b_gated runs instead.
+// over- or underflow at other places; so for sources that are infinite, or whose largest value
+// lies outside [1e-28, 1e25], `direct` is set and k_update_e_b_gated runs instead (a NaN
+// charge leaves NaN in every cell either way).
 #include "field_fft.h"
 #include "fft_regs.cuh"
 #include "ion_device.cuh"
@@ -153,7 +154,8 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
     __syncthreads();
     if (block == 0u && threadIdx.x < 4u) {
         const uint32_t v = s_max[threadIdx.x];
-        if (v != 0u && !(v >= __float_as_uint(1e-28f) && v <= __float_as_uint(1e25f))) atomicExch(&s_bad, 1u);
+        // a NaN charge makes every cell's E and B NaN either way
+        if (s_max[0] <= 0x7F800000u && v != 0u && !(v >= __float_as_uint(1e-28f) && v <= __float_as_uint(1e25f))) atomicExch(&s_bad, 1u);
     }
     // along x at this kx
     for (uint32_t t = threadIdx.x; t < ND * ND; t += SRC_THREADS) {

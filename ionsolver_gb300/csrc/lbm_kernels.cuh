@@ -12,6 +12,7 @@
 #pragma once
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "ion_device.cuh"
 #include "ion_launch.h"
@@ -577,27 +578,40 @@ __host__ __device__ inline uint32_t row_bytes(uint32_t nx) {
 // op(stream, pointer to the row's first element) for each lattice (gas, then electron
 // gas and charge), stream 0 and the odd streams from the own row, stream i + 1 from the
 // row of the neighbour in direction i (periodic in y and z).
+// One thread issues a row's copies, and an MHD row has 97 of them (52 loads, 45 stores): at some
+// twenty instructions each, one after another, they took longer than the other warps took to
+// compute the row.  So the offsets of the seven neighbour rows are formed once, every stream is
+// unrolled, and a slot's address is two multiply-adds (19 N < 2^32: 32-bit offsets).
 template <int FT, bool MHD, class OP>
 __device__ __forceinline__ void for_row_streams(const DevLbm& L, uint32_t r, bool odd, OP&& op) {
     using V = VSet<19>;
     using T = typename Ddf<FT>::T;
     const uint32_t nx = L.nx, ny = L.ny, nz = L.nz, N = L.n;
-    const uint32_t y = r % ny, z = r / ny, own = (y + z * ny) * nx;
-    auto lattice = [&](T* f, uint32_t base, int Q) {
+    const uint32_t z = r / ny, y = r - z * ny;
+    const uint32_t yp = y + 1u == ny ? 0u : y + 1u, ym = y == 0u ? ny - 1u : y - 1u;
+    const uint32_t zp = (z + 1u == nz ? 0u : z + 1u) * ny, zm = (z == 0u ? nz - 1u : z - 1u) * ny, z0 = z * ny;
+    const uint32_t own = (y + z0) * nx;
+    // the neighbour row of (cy, cz)
+    const uint32_t row_p0 = (yp + z0) * nx, row_m0 = (ym + z0) * nx, row_0p = (y + zp) * nx, row_0m = (y + zm) * nx,
+                   row_pp = (yp + zp) * nx, row_pm = (yp + zm) * nx;
+    const uint32_t first = odd ? 0u : N;  // slots of direction i: own odd ? i : i + 1, neighbour odd ? i + 1 : i
+    auto lattice = [&](T* f, uint32_t base, auto q) {
+        constexpr int Q = decltype(q)::value;
         op(base, f + own);
+        const uint32_t o_own = own + first, o_nbr = N - first;
+#pragma unroll
         for (int i = 1; i < Q; i += 2) {
             const int cy = Q == 7 ? (i == 3 ? 1 : 0) : V::c(i, 1), cz = Q == 7 ? (i == 5 ? 1 : 0) : V::c(i, 2);
-            const uint32_t yy = cy > 0 ? (y + 1u == ny ? 0u : y + 1u) : cy < 0 ? (y == 0u ? ny - 1u : y - 1u) : y;
-            const uint32_t zz = cz > 0 ? (z + 1u == nz ? 0u : z + 1u) : cz < 0 ? (z == 0u ? nz - 1u : z - 1u) : z;
-            const uint32_t s_own = odd ? (uint32_t)i : (uint32_t)i + 1u, s_nbr = odd ? (uint32_t)i + 1u : (uint32_t)i;
-            op(base + i, f + (size_t)s_own * N + own);
-            op(base + i + 1, f + (size_t)s_nbr * N + (yy + zz * ny) * nx);
+            const uint32_t row = cy == 0 ? (cz > 0 ? row_0p : cz < 0 ? row_0m : own)
+                                 : cy > 0 ? (cz > 0 ? row_pp : cz < 0 ? row_pm : row_p0) : row_m0;
+            op(base + i, f + ((uint32_t)i * N + o_own));
+            op(base + i + 1, f + ((uint32_t)i * N + (row + o_nbr)));
         }
     };
-    lattice((T*)L.fi, row_stream_base(LAT_FI), 19);
+    lattice((T*)L.fi, row_stream_base(LAT_FI), std::integral_constant<int, 19>{});
     if constexpr (MHD) {
-        lattice((T*)L.ei, row_stream_base(LAT_EI), 19);
-        lattice((T*)L.fqi, row_stream_base(LAT_FQI), 7);
+        lattice((T*)L.ei, row_stream_base(LAT_EI), std::integral_constant<int, 19>{});
+        lattice((T*)L.fqi, row_stream_base(LAT_FQI), std::integral_constant<int, 7>{});
     }
 }
 
