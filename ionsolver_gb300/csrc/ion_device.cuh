@@ -139,9 +139,10 @@ __host__ __device__ __forceinline__ uint16_t fp16c_encode(float x) {
 // The code's exponent and mantissa as the bits of a float are 2^-112 times its value, with
 // exponent field 0 as the float's subnormals: one product by 2^112 (exact).  Equal to the
 // reference's decoder for all 2^16 inputs.
-__host__ __device__ __forceinline__ float fp16c_decode(uint16_t x) {
-    return bitsf(((uint32_t)(int32_t)(int16_t)x << 12) & 0x87FFFFFFu) * 5.192296858534828e33f;
+__host__ __device__ __forceinline__ float fp16c_raw(uint16_t x) {
+    return bitsf(((uint32_t)(int32_t)(int16_t)x << 12) & 0x87FFFFFFu);
 }
+__host__ __device__ __forceinline__ float fp16c_decode(uint16_t x) { return fp16c_raw(x) * 5.192296858534828e33f; }
 
 // Packed FP32 pairs (PTX add/sub/mul/fma .f32x2, sm_100 and later): one
 // instruction does the same IEEE round-to-nearest operation on the two halves
@@ -229,9 +230,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 // flight are then waited for with this full limit before the block exits.
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 
+// dec = raw * RAW and enc(x) = enc_scaled(x * ENC) with powers of two: the stencil sums raw
+// values and folds both factors into the coefficients of its multiply-adds, where a power of
+// two changes no rounding (no sum of codes or of values on their way to a code leaves the
+// exponent range: 16-bit codes hold the density below 40).  Two products less per DDF.
 template <int FT> struct Ddf;
 template <> struct Ddf<ION_FP32> {
     using T = float;
+    static constexpr float RAW = 1.0f, ENC = 1.0f;
+    __device__ __forceinline__ static float raw(float v) { return v; }
+    __device__ __forceinline__ static float enc_scaled(float x) { return x; }
     __device__ __forceinline__ static float dec(float v) { return v; }
     __device__ __forceinline__ static float enc(float x) { return x; }
     __device__ __forceinline__ static float ld(const float* p, size_t i) { return p[i]; }
@@ -239,13 +247,19 @@ template <> struct Ddf<ION_FP32> {
 };
 template <> struct Ddf<ION_FP16S> {
     using T = uint16_t;
-    __device__ __forceinline__ static float dec(uint16_t v) { return __half2float(__ushort_as_half(v)) * 3.0517578E-5f; }
-    __device__ __forceinline__ static uint16_t enc(float x) { return __half_as_ushort(__float2half_rn(x * 32768.0f)); }
+    static constexpr float RAW = 3.0517578125E-5f, ENC = 32768.0f;
+    __device__ __forceinline__ static float raw(uint16_t v) { return __half2float(__ushort_as_half(v)); }
+    __device__ __forceinline__ static uint16_t enc_scaled(float x) { return __half_as_ushort(__float2half_rn(x)); }
+    __device__ __forceinline__ static float dec(uint16_t v) { return raw(v) * RAW; }
+    __device__ __forceinline__ static uint16_t enc(float x) { return enc_scaled(x * ENC); }
     __device__ __forceinline__ static float ld(const uint16_t* p, size_t i) { return dec(p[i]); }
     __device__ __forceinline__ static void st(uint16_t* p, size_t i, float x) { p[i] = enc(x); }
 };
 template <> struct Ddf<ION_FP16C> {
     using T = uint16_t;
+    static constexpr float RAW = 5.192296858534828e33f, ENC = 1.0f;  // 2^112
+    __device__ __forceinline__ static float raw(uint16_t v) { return fp16c_raw(v); }
+    __device__ __forceinline__ static uint16_t enc_scaled(float x) { return fp16c_encode_result(x); }
     __device__ __forceinline__ static float dec(uint16_t v) { return fp16c_decode(v); }
     __device__ __forceinline__ static uint16_t enc(float x) { return fp16c_encode_result(x); }
     __device__ __forceinline__ static float ld(const uint16_t* p, size_t i) { return dec(p[i]); }

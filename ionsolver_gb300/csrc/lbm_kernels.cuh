@@ -35,13 +35,15 @@ struct Nbr {
     }
 };
 
-// density / velocity from DDF-shifted populations (sim_kernels.cl:208-233)
+// density / velocity from DDF-shifted populations (sim_kernels.cl:208-233), given divided by
+// `raw`, a power of two
 template <class V>
-__device__ __forceinline__ void moments(const float* f, float& rho, float& ux, float& uy, float& uz) {
+__device__ __forceinline__ void moments(const float* f, float& rho, float& ux, float& uy, float& uz,
+                                        const float raw = 1.0f) {
     float r = f[0];
 #pragma unroll
     for (int i = 1; i < V::q; i++) r = r + f[i];
-    r = r + 1.0f;
+    r = raw == 1.0f ? r + 1.0f : fmaf(r, raw, 1.0f);
     float u[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -55,7 +57,7 @@ __device__ __forceinline__ void moments(const float* f, float& rho, float& ux, f
             acc = first ? pos - neg : (acc + pos) - neg;
             first = false;
         }
-        u[a] = acc;
+        u[a] = raw == 1.0f ? acc : acc * raw;
     }
     rho = r;
     ux = u[0] / r;
@@ -117,7 +119,16 @@ __device__ __forceinline__ void adv_equilibrium(float Q, float ux, float uy, flo
     a[5] = fmaf(hq, uz, eq); a[6] = fmaf(hq, -uz, eq);
 }
 
-// Esoteric-Pull load/store (sim_kernels.cl:234-247, 397-410)
+// Esoteric-Pull load/store (sim_kernels.cl:234-247, 397-410); ep_load_raw: divided by D::RAW
+template <class D, int Q, class NB>
+__device__ __forceinline__ void ep_load_raw(const typename D::T* f, uint32_t N, uint32_t n, bool odd, const NB& j, float* v) {
+    v[0] = D::raw(f[n]);
+#pragma unroll
+    for (int i = 1; i < Q; i += 2) {
+        v[i] = D::raw(f[(size_t)(odd ? i : i + 1) * N + n]);
+        v[i + 1] = D::raw(f[(size_t)(odd ? i + 1 : i) * N + j(i)]);
+    }
+}
 template <class D, int Q, class NB>
 __device__ __forceinline__ void ep_load(const typename D::T* f, uint32_t N, uint32_t n, bool odd, const NB& j, float* v) {
     v[0] = D::ld(f, n);
@@ -139,22 +150,20 @@ struct GlobalDst {
     uint32_t N, n;
     bool odd;
     const NB& j;
-    __device__ __forceinline__ void st0(float v) const { D::st(f, n, v); }
-    __device__ __forceinline__ void st_nbr(int i, float v) const { D::st(f, (IX)(odd ? i + 1 : i) * N + j(i), v); }
-    __device__ __forceinline__ void st_own(int i, float v) const { D::st(f, (IX)(odd ? i : i + 1) * N + n, v); }
+    using DD = D;
+    __device__ __forceinline__ void st0(typename D::T v) const { f[n] = v; }
+    __device__ __forceinline__ void st_nbr(int i, typename D::T v) const { f[(IX)(odd ? i + 1 : i) * N + j(i)] = v; }
+    __device__ __forceinline__ void st_own(int i, typename D::T v) const { f[(IX)(odd ? i : i + 1) * N + n] = v; }
 };
-template <int Q, class DST>
-__device__ __forceinline__ void ep_store_to(const DST& o, const float* v) {
-    o.st0(v[0]);
-#pragma unroll
-    for (int i = 1; i < Q; i += 2) {
-        o.st_nbr(i, v[i]);
-        o.st_own(i, v[i + 1]);
-    }
-}
 template <class D, int Q, class NB, class IX = size_t>
 __device__ __forceinline__ void ep_store(typename D::T* f, uint32_t N, uint32_t n, bool odd, const NB& j, const float* v) {
-    ep_store_to<Q>(GlobalDst<D, NB, IX>{f, N, n, odd, j}, v);
+    const GlobalDst<D, NB, IX> o{f, N, n, odd, j};
+    o.st0(D::enc(v[0]));
+#pragma unroll
+    for (int i = 1; i < Q; i += 2) {
+        o.st_nbr(i, D::enc(v[i]));
+        o.st_own(i, D::enc(v[i + 1]));
+    }
 }
 
 // L2 prefetch of the slots ep_load will read (no registers held; the later
@@ -195,7 +204,7 @@ struct GlobalSrc {
     template <class D, int Q, class NB>
     __device__ __forceinline__ void load(const typename D::T* f, uint32_t N, uint32_t n, bool odd, const NB& j,
                                          float* v, int) const {
-        ep_load<D, Q>(f, N, n, odd, j, v);
+        ep_load_raw<D, Q>(f, N, n, odd, j, v);
     }
     template <class D, int Q, class IX, class NB>
     __device__ __forceinline__ GlobalDst<D, NB, IX> dst(typename D::T* f, uint32_t N, uint32_t n, bool odd, const NB& j,
@@ -217,11 +226,12 @@ struct RowDst {
     typename D::T* r;  // the lattice's stream 0
     uint32_t nx, x, xp, xm;
     __device__ __forceinline__ uint32_t stride() const { return RS ? RS : nx; }
-    __device__ __forceinline__ void st0(float v) const { r[x] = D::enc(v); }
-    __device__ __forceinline__ void st_own(int i, float v) const { r[(uint32_t)i * stride() + x] = D::enc(v); }
-    __device__ __forceinline__ void st_nbr(int i, float v) const {
+    using DD = D;
+    __device__ __forceinline__ void st0(typename D::T v) const { r[x] = v; }
+    __device__ __forceinline__ void st_own(int i, typename D::T v) const { r[(uint32_t)i * stride() + x] = v; }
+    __device__ __forceinline__ void st_nbr(int i, typename D::T v) const {
         const int cx = row_cx<Q>(i);
-        r[(uint32_t)(i + 1) * stride() + (cx > 0 ? xp : cx < 0 ? xm : x)] = D::enc(v);
+        r[(uint32_t)(i + 1) * stride() + (cx > 0 ? xp : cx < 0 ? xm : x)] = v;
     }
 };
 
@@ -244,12 +254,12 @@ struct RowSrc {
     template <class D, int Q, class NB>
     __device__ __forceinline__ void load(const T*, uint32_t, uint32_t, bool, const NB&, float* v, int lat) const {
         const T* r = reinterpret_cast<const T*>(buf) + row_stream_base(lat) * stride();
-        v[0] = D::dec(r[x]);
+        v[0] = D::raw(r[x]);
 #pragma unroll
         for (int i = 1; i < Q; i += 2) {
             const int cx = row_cx<Q>(i);
-            v[i] = D::dec(r[(uint32_t)i * stride() + x]);
-            v[i + 1] = D::dec(r[(uint32_t)(i + 1) * stride() + (cx > 0 ? xp : cx < 0 ? xm : x)]);
+            v[i] = D::raw(r[(uint32_t)i * stride() + x]);
+            v[i + 1] = D::raw(r[(uint32_t)(i + 1) * stride() + (cx > 0 ? xp : cx < 0 ? xm : x)]);
         }
     }
     template <class D, int Q, class IX, class NB>
@@ -309,34 +319,37 @@ __device__ __forceinline__ float force_dir(const ForceState& s, int i) {
 // the equilibrium itself (sim_kernels.cl:719-723 / 651-655)
 template <class V, class DST>
 __device__ __forceinline__ void eq_store(const DST& o, const EqState& es) {
-    o.st0(eq_zero<V>(es));
+    using D = typename DST::DD;
+    o.st0(D::enc(eq_zero<V>(es)));
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
         float fa, fb;
         eq_pair<V>(es, i, fa, fb);
-        o.st_nbr(i, fa);
-        o.st_own(i, fb);
+        o.st_nbr(i, D::enc(fa));
+        o.st_own(i, D::enc(fb));
     }
 }
 
-// SRT collision + Esoteric-Pull store (sim_kernels.cl:714-723 / 649-656).
-// force: 0 = none (Fin = 0), 1 = Guo terms scaled by c_tau.
+// SRT collision + Esoteric-Pull store (sim_kernels.cl:714-723 / 649-656) of DDFs fh, divided by
+// D::RAW.  force: 0 = none (Fin = 0), 1 = Guo terms scaled by c_tau.
 template <class V, class DST>
 __device__ __forceinline__ void srt_store(const DST& o, const float* fh, const EqState& es, const ForceState& fs,
                                           bool force, float c_tau, float w) {
+    using D = typename DST::DD;
+    const float wf = (1.0f - w) * (D::RAW * D::ENC), we = w * D::ENC, cf = c_tau * D::ENC;
     {
         const float feq = eq_zero<V>(es);
-        const float F = force ? force_dir<V>(fs, 0) * c_tau : 0.0f;
-        o.st0(fmaf(1.0f - w, fh[0], fmaf(w, feq, F)));
+        const float F = force ? force_dir<V>(fs, 0) * cf : 0.0f;
+        o.st0(D::enc_scaled(fmaf(wf, fh[0], fmaf(we, feq, F))));
     }
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
         float fa, fb;
         eq_pair<V>(es, i, fa, fb);
-        const float Fa = force ? force_dir<V>(fs, i) * c_tau : 0.0f;
-        const float Fb = force ? force_dir<V>(fs, i + 1) * c_tau : 0.0f;
-        o.st_nbr(i, fmaf(1.0f - w, fh[i], fmaf(w, fa, Fa)));
-        o.st_own(i, fmaf(1.0f - w, fh[i + 1], fmaf(w, fb, Fb)));
+        const float Fa = force ? force_dir<V>(fs, i) * cf : 0.0f;
+        const float Fb = force ? force_dir<V>(fs, i + 1) * cf : 0.0f;
+        o.st_nbr(i, D::enc_scaled(fmaf(wf, fh[i], fmaf(we, fa, Fa))));
+        o.st_own(i, D::enc_scaled(fmaf(wf, fh[i + 1], fmaf(we, fb, Fb))));
     }
 }
 
@@ -344,8 +357,11 @@ __device__ __forceinline__ void srt_store(const DST& o, const float* fh, const E
 template <class V, class DST>
 __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const EqState& es, const ForceState& fs,
                                           bool force, float w) {
+    using D = typename DST::DD;
+    constexpr float R = D::RAW;
     const float wp = w, wm = 1.0f / (0.1875f / (1.0f / w - 0.5f) + 0.5f);
-    const float ctp = fmaf(wp, -0.25f, 0.5f), ctm = fmaf(wm, -0.25f, 0.5f);
+    const float ctp = fmaf(wp, -0.25f, 0.5f) * D::ENC, ctm = fmaf(wm, -0.25f, 0.5f) * D::ENC;
+    const float hp = 0.5f * wp * D::ENC, hm = 0.5f * wm * D::ENC;
     {
         const float feq = eq_zero<V>(es);
         float F = 0.0f;
@@ -353,9 +369,9 @@ __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const E
             const float F0 = force_dir<V>(fs, 0);
             F = fmaf(ctp, F0 + F0, ctm * (F0 - F0));
         }
-        const float sym = ((feq - fh[0]) + feq) - fh[0];
-        const float asym = ((feq - feq) - fh[0]) + fh[0];
-        o.st0(fmaf(0.5f * wp, sym, fmaf(0.5f * wm, asym, fh[0] + F)));
+        const float sym = fmaf(-R, fh[0], fmaf(-R, fh[0], feq) + feq);
+        const float asym = fmaf(R, fh[0], fmaf(-R, fh[0], feq - feq));
+        o.st0(D::enc_scaled(fmaf(hp, sym, fmaf(hm, asym, fmaf(R * D::ENC, fh[0], F)))));
     }
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
@@ -368,8 +384,10 @@ __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const E
             Fb = fmaf(ctp, B + A, ctm * (B - A));
         }
         const float ha = fh[i], hb = fh[i + 1];
-        o.st_nbr(i, fmaf(0.5f * wp, ((ea - ha) + eb) - hb, fmaf(0.5f * wm, ((ea - eb) - ha) + hb, ha + Fa)));
-        o.st_own(i, fmaf(0.5f * wp, ((eb - hb) + ea) - ha, fmaf(0.5f * wm, ((eb - ea) - hb) + ha, hb + Fb)));
+        const float sa = fmaf(-R, hb, fmaf(-R, ha, ea) + eb), sb = fmaf(-R, ha, fmaf(-R, hb, eb) + ea);
+        const float da = fmaf(R, hb, fmaf(-R, ha, ea - eb)), db = fmaf(R, ha, fmaf(-R, hb, eb - ea));
+        o.st_nbr(i, D::enc_scaled(fmaf(hp, sa, fmaf(hm, da, fmaf(R * D::ENC, ha, Fa)))));
+        o.st_own(i, D::enc_scaled(fmaf(hp, sb, fmaf(hm, db, fmaf(R * D::ENC, hb, Fb)))));
     }
 }
 
@@ -425,7 +443,7 @@ __device__ __forceinline__ void sc_cell(const DevLbm& L, const uint32_t n, const
         float rho, ux, uy, uz, fx, fy, fz;
         bool force;
         if (!electrons && eqc) { rho = L.rho[n]; ux = L.u[n]; uy = L.u[(size_t)N + n]; uz = L.u[2 * (size_t)N + n]; }
-        else moments<V>(fh, rho, ux, uy, uz);
+        else moments<V>(fh, rho, ux, uy, uz, D::RAW);
         if (electrons) {
             // electron gas: Lorentz force, Guo half-step (sim_kernels.cl:530-656)
             if constexpr (ECR) {  // SUBGRID_ECR, sim_kernels.cl:564-628 (the ionisation term is the reference's placeholder)
@@ -488,13 +506,18 @@ __device__ __forceinline__ void sc_cell(const DevLbm& L, const uint32_t n, const
                     rhoq = 0.0f;
 #pragma unroll
                     for (int i = 0; i < 7; i++) rhoq = rhoq + qhn[i];
-                    rhoq = rhoq + 1.0f;
+                    rhoq = D::RAW == 1.0f ? rhoq + 1.0f : fmaf(rhoq, D::RAW, 1.0f);
                     if constexpr (ECR) rhoq = rhoq + dq_ecr;
                     float aeq[7];
                     adv_equilibrium(rhoq, ux, uy, uz, aeq);
+                    const float wf = (1.0f - L.wq) * (D::RAW * D::ENC), we = L.wq * D::ENC;
+                    const auto dq = S.template dst<D, 7, IX>((T*)L.fqi, N, n, odd, j7, LAT_FQI);
+                    dq.st0(D::enc_scaled(fmaf(wf, qhn[0], we * aeq[0])));
 #pragma unroll
-                    for (int i = 0; i < 7; i++) qhn[i] = fmaf(1.0f - L.wq, qhn[i], L.wq * aeq[i]);
-                    ep_store_to<7>(S.template dst<D, 7, IX>((T*)L.fqi, N, n, odd, j7, LAT_FQI), qhn);
+                    for (int i = 1; i < 7; i += 2) {
+                        dq.st_nbr(i, D::enc_scaled(fmaf(wf, qhn[i], we * aeq[i])));
+                        dq.st_own(i, D::enc_scaled(fmaf(wf, qhn[i + 1], we * aeq[i + 1])));
+                    }
                 }
                 L.q[n] = rhoq - rhoe;
                 // Lorentz force on the gas
