@@ -331,16 +331,18 @@ __device__ __forceinline__ void eq_store(const DST& o, const EqState& es) {
 }
 
 // SRT collision + Esoteric-Pull store (sim_kernels.cl:714-723 / 649-656) of DDFs fh, divided by
-// D::RAW.  force: 0 = none (Fin = 0), 1 = Guo terms scaled by c_tau.
-template <class V, class DST>
+// D::RAW.  force: 0 = none (Fin = 0), 1 = Guo terms scaled by c_tau.  SELECT: eqc picks the
+// equilibrium, value by value.
+template <class V, bool SELECT, class DST>
 __device__ __forceinline__ void srt_store(const DST& o, const float* fh, const EqState& es, const ForceState& fs,
-                                          bool force, float c_tau, float w) {
+                                          bool force, float c_tau, float w, bool eqc) {
     using D = typename DST::DD;
+    auto out = [&](float feq, float f) { return D::enc_scaled(SELECT && eqc ? feq * D::ENC : f); };
     const float wf = (1.0f - w) * (D::RAW * D::ENC), we = w * D::ENC, cf = c_tau * D::ENC;
     {
         const float feq = eq_zero<V>(es);
         const float F = force ? force_dir<V>(fs, 0) * cf : 0.0f;
-        o.st0(D::enc_scaled(fmaf(wf, fh[0], fmaf(we, feq, F))));
+        o.st0(out(feq, fmaf(wf, fh[0], fmaf(we, feq, F))));
     }
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
@@ -348,8 +350,8 @@ __device__ __forceinline__ void srt_store(const DST& o, const float* fh, const E
         eq_pair<V>(es, i, fa, fb);
         const float Fa = force ? force_dir<V>(fs, i) * cf : 0.0f;
         const float Fb = force ? force_dir<V>(fs, i + 1) * cf : 0.0f;
-        o.st_nbr(i, D::enc_scaled(fmaf(wf, fh[i], fmaf(we, fa, Fa))));
-        o.st_own(i, D::enc_scaled(fmaf(wf, fh[i + 1], fmaf(we, fb, Fb))));
+        o.st_nbr(i, out(fa, fmaf(wf, fh[i], fmaf(we, fa, Fa))));
+        o.st_own(i, out(fb, fmaf(wf, fh[i + 1], fmaf(we, fb, Fb))));
     }
 }
 
@@ -358,10 +360,16 @@ template <class V, class DST>
 __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const EqState& es, const ForceState& fs,
                                           bool force, float w) {
     using D = typename DST::DD;
-    constexpr float R = D::RAW;
+    // x +- a DDF, as one addition
+    auto plus = [](float x, float h) { return D::RAW == 1.0f ? x + h : fmaf(D::RAW, h, x); };
+    auto minus = [](float x, float h) { return D::RAW == 1.0f ? x - h : fmaf(-D::RAW, h, x); };
     const float wp = w, wm = 1.0f / (0.1875f / (1.0f / w - 0.5f) + 0.5f);
     const float ctp = fmaf(wp, -0.25f, 0.5f) * D::ENC, ctm = fmaf(wm, -0.25f, 0.5f) * D::ENC;
     const float hp = 0.5f * wp * D::ENC, hm = 0.5f * wm * D::ENC;
+    auto out = [&](float sym, float asym, float h, float F) {
+        constexpr float E = D::RAW * D::ENC;
+        return D::enc_scaled(fmaf(hp, sym, fmaf(hm, asym, E == 1.0f ? h + F : fmaf(E, h, F))));
+    };
     {
         const float feq = eq_zero<V>(es);
         float F = 0.0f;
@@ -369,9 +377,7 @@ __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const E
             const float F0 = force_dir<V>(fs, 0);
             F = fmaf(ctp, F0 + F0, ctm * (F0 - F0));
         }
-        const float sym = fmaf(-R, fh[0], fmaf(-R, fh[0], feq) + feq);
-        const float asym = fmaf(R, fh[0], fmaf(-R, fh[0], feq - feq));
-        o.st0(D::enc_scaled(fmaf(hp, sym, fmaf(hm, asym, fmaf(R * D::ENC, fh[0], F)))));
+        o.st0(out(minus(minus(feq, fh[0]) + feq, fh[0]), plus(minus(feq - feq, fh[0]), fh[0]), fh[0], F));
     }
 #pragma unroll
     for (int i = 1; i < V::q; i += 2) {
@@ -384,10 +390,8 @@ __device__ __forceinline__ void trt_store(const DST& o, const float* fh, const E
             Fb = fmaf(ctp, B + A, ctm * (B - A));
         }
         const float ha = fh[i], hb = fh[i + 1];
-        const float sa = fmaf(-R, hb, fmaf(-R, ha, ea) + eb), sb = fmaf(-R, ha, fmaf(-R, hb, eb) + ea);
-        const float da = fmaf(R, hb, fmaf(-R, ha, ea - eb)), db = fmaf(R, ha, fmaf(-R, hb, eb - ea));
-        o.st_nbr(i, D::enc_scaled(fmaf(hp, sa, fmaf(hm, da, fmaf(R * D::ENC, ha, Fa)))));
-        o.st_own(i, D::enc_scaled(fmaf(hp, sb, fmaf(hm, db, fmaf(R * D::ENC, hb, Fb)))));
+        o.st_nbr(i, out(minus(minus(ea, ha) + eb, hb), plus(minus(ea - eb, ha), hb), ha, Fa));
+        o.st_own(i, out(minus(minus(eb, hb) + ea, ha), plus(minus(eb - ea, hb), ha), hb, Fb));
     }
 }
 
@@ -551,10 +555,12 @@ __device__ __forceinline__ void sc_cell(const DevLbm& L, const uint32_t n, const
         const ForceState fs = force_state<V>(ux, uy, uz, fx, fy, fz);
         const auto dst = S.template dst<D, Q, IX>(f, N, n, odd, j, lat);
         // boundary cells store the equilibrium: a branch of its own, as a select per value costs
-        // every cell of a domain without them
-        if (eqc) eq_store<V>(dst, es);
+        // every cell of a domain without them; but the SRT stencil with global stores keeps the
+        // selects (250x101x200 FP32 140.7 us, with the branch 144.9: a second set of addresses)
+        constexpr bool SELECT = !MHD && !TRT && SRC::prefetch;
+        if (!SELECT && eqc) eq_store<V>(dst, es);
         else if (TRT && !electrons) trt_store<V>(dst, fh, es, fs, force, w);
-        else srt_store<V>(dst, fh, es, fs, force, c_tau, w);
+        else srt_store<V, SELECT>(dst, fh, es, fs, force, c_tau, w, eqc);
     }
 }
 
