@@ -580,8 +580,11 @@ __device__ __forceinline__ void quad_weights(float t, float* w) {  // Lagrange w
     w[2] = 2.0f * t * (t - 0.5f);
 }
 
+// COLUMNS: a thread's cells are neighbours along z, which share their x and y and the entry of
+// the y table (bins of at least SC_CPT cells in z); else they are SC_THREADS apart in the bin
+template <bool COLUMNS>
 __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, const float4* t2, uint32_t bin, int bx,
-                                               int by, int bz, uint32_t tile, uint32_t cells, const Magic& mx,
+                                               int by, int bz, uint32_t tile, uint32_t items, const Magic& mx,
                                                const Magic& mxy);
 
 __global__ void __launch_bounds__(SC_THREADS, 3) k_surrogate_cells(const DevLbm L, const float* Y, const float* G,
@@ -625,14 +628,18 @@ __global__ void __launch_bounds__(SC_THREADS, 3) k_surrogate_cells(const DevLbm 
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < L.bsx * 9u * 8u; i += blockDim.x) {
-        const uint32_t lx = i / 72u, jk = (i / 8u) % 9u, c = i % 8u;
-        float wx[3];
+    for (uint32_t i = threadIdx.x; i < L.bsx * 9u; i += blockDim.x) {
+        const uint32_t lx = i / 9u, jk = i - 9u * lx;
+        float wx[3], v[6];
         quad_weights(L.bsx > 1 ? (float)lx / (float)(L.bsx - 1) : 0.0f, wx);
-        float v = 0.0f;
-        if (c < 6u)
-            for (int ix = 0; ix < 3; ix++) v = fmaf(wx[ix], sm.node[(ix + 3 * jk) * 6 + c], v);
-        ((float*)&sm.t1[lx][jk][0])[c] = v;
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            v[c] = 0.0f;
+#pragma unroll
+            for (int ix = 0; ix < 3; ix++) v[c] = fmaf(wx[ix], sm.node[(ix + 3 * jk) * 6 + c], v[c]);
+        }
+        sm.t1[lx][jk][0] = make_float4(v[0], v[1], v[2], v[3]);
+        sm.t1[lx][jk][1] = make_float4(v[4], v[5], 0.0f, 0.0f);
     }
     for (uint32_t i = threadIdx.x; i < 2u * Surrogate::MAX_BLOCK; i += blockDim.x) {
         const uint32_t a = i / Surrogate::MAX_BLOCK, l = i % Surrogate::MAX_BLOCK, b = a == 0u ? L.bsy : L.bsz;
@@ -645,27 +652,39 @@ __global__ void __launch_bounds__(SC_THREADS, 3) k_surrogate_cells(const DevLbm 
     // behind SurSmem in dynamic shared memory (bsx bsy rows of 3 x 8 floats, 28 apart: the eight
     // lanes of a 16-byte access then read different banks)
     float4* t2 = reinterpret_cast<float4*>(sur_smem + sizeof(SurSmem));
-    for (uint32_t i = threadIdx.x; i < L.bsx * L.bsy * 24u; i += blockDim.x) {
-        const uint32_t c = i % 8u, iz = (i / 8u) % 3u, lx = (i / 24u) % L.bsx, ly = i / (24u * L.bsx);
+    const Magic mx(L.bsx), mxy(L.bsx * L.bsy);
+    // (an entry a thread: with a value a thread the index divisions were a quarter of the kernel)
+    for (uint32_t i = threadIdx.x; i < L.bsx * L.bsy * 3u; i += blockDim.x) {
+        const uint32_t q = i / 3u, iz = i - 3u * q, ly = mx.div(q), lx = q - ly * mx.d;
         const float4 wy = sm.wyz[0][ly];
-        float v = 0.0f;
-        if (c < 6u) {
-            const float* t = (const float*)&sm.t1[lx][0][0];
-            v = fmaf(wy.x, t[(0u + 3u * iz) * 8u + c], v);
-            v = fmaf(wy.y, t[(1u + 3u * iz) * 8u + c], v);
-            v = fmaf(wy.z, t[(2u + 3u * iz) * 8u + c], v);
+        const float w[3] = {wy.x, wy.y, wy.z};
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+#pragma unroll
+        for (uint32_t iy = 0; iy < 3; iy++) {
+            const float4 p = sm.t1[lx][iy + 3u * iz][0], r = sm.t1[lx][iy + 3u * iz][1];
+            a = make_float4(fmaf(w[iy], p.x, a.x), fmaf(w[iy], p.y, a.y), fmaf(w[iy], p.z, a.z), fmaf(w[iy], p.w, a.w));
+            b.x = fmaf(w[iy], r.x, b.x);
+            b.y = fmaf(w[iy], r.y, b.y);
         }
-        ((float*)t2)[(ly * L.bsx + lx) * 28u + iz * 8u + c] = v;
+        t2[q * 7u + iz * 2u] = a;
+        t2[q * 7u + iz * 2u + 1u] = b;
     }
     __syncthreads();
 
     const uint32_t cells = L.bsx * L.bsy * L.bsz;
-    const Magic mx(L.bsx), mxy(L.bsx * L.bsy);
-    for (uint32_t tile = 0; tile * SC_CELLS < cells; tile++) surrogate_tile(L, sm, t2, bin, bx, by, bz, tile, cells, mx, mxy);
+    if (L.bsz >= SC_CPT) {
+        const uint32_t items = L.bsx * L.bsy * ((L.bsz + SC_CPT - 1u) / SC_CPT);
+        for (uint32_t tile = 0; tile * SC_THREADS < items; tile++)
+            surrogate_tile<true>(L, sm, t2, bin, bx, by, bz, tile, items, mx, mxy);
+    } else {
+        for (uint32_t tile = 0; tile * SC_CELLS < cells; tile++)
+            surrogate_tile<false>(L, sm, t2, bin, bx, by, bz, tile, cells, mx, mxy);
+    }
 }
 
+template <bool COLUMNS>
 __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, const float4* t2, uint32_t bin, int bx,
-                                               int by, int bz, uint32_t tile, uint32_t cells, const Magic& mx,
+                                               int by, int bz, uint32_t tile, uint32_t items, const Magic& mx,
                                                const Magic& mxy) {
     // cell k of this thread: local index li -> (lx, ly, lz) in the bin, kept packed
     // (10 bits each) for the tail; flags are read now and used after the near sums
@@ -676,10 +695,11 @@ __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, con
     const float4 o = L.lod_pos[bin];
 #pragma unroll
     for (uint32_t k = 0; k < SC_CPT; k++) {
-        const uint32_t li = tile * SC_CELLS + threadIdx.x + k * SC_THREADS;
-        const bool in = li < cells;
-        const uint32_t lc = in ? li : 0u;
-        const uint32_t lz = mxy.div(lc), r = lc - lz * mxy.d, ly = mx.div(r), lx = r - ly * mx.d;
+        const uint32_t li = COLUMNS ? tile * SC_THREADS + threadIdx.x : tile * SC_CELLS + threadIdx.x + k * SC_THREADS;
+        const uint32_t lc = li < items ? li : 0u;
+        const uint32_t q = mxy.div(lc), r = lc - q * mxy.d, ly = mx.div(r), lx = r - ly * mx.d;
+        const uint32_t lz = COLUMNS ? q * SC_CPT + k : q;
+        const bool in = li < items && lz < L.bsz;
         pc[k] = lx | ly << 10 | lz << 20;
         const uint32_t x = bx * L.bsx + lx, y = by * L.bsy + ly, z = bz * L.bsz + lz;
         const uint32_t m = x + (y + z * L.ny) * L.nx;
@@ -714,6 +734,14 @@ __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, con
         for (uint32_t j = 0; j < SC_CPT / 2; j++) far_fast2(cp[j], cc[j], S, fs[j]);
     }
     asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+    // triquadratic interpolation: the x and y contractions are tabulated per bin (t2)
+    float4 ta[3], tb[3];
+    auto fetch = [&](uint32_t lx, uint32_t ly) {
+        const float4* tc = t2 + (size_t)(ly * L.bsx + lx) * 7u;
+#pragma unroll
+        for (int iz = 0; iz < 3; iz++) { ta[iz] = tc[2 * iz]; tb[iz] = tc[2 * iz + 1]; }
+    };
+    if (COLUMNS) fetch(pc[0] & 1023u, (pc[0] >> 10) & 1023u);
 #pragma unroll
     for (uint32_t k = 0; k < SC_CPT; k++) {
         if ((fl[k] & F_BO) == F_S) continue;  // solid, or no cell
@@ -722,14 +750,13 @@ __device__ __forceinline__ void surrogate_tile(const DevLbm& L, SurSmem& sm, con
         const uint32_t m = (bx * L.bsx + lx) + ((by * L.bsy + ly) + (bz * L.bsz + lz) * L.ny) * L.nx;
         float e[3] = {0.0f, 0.0f, 0.0f}, b[3] = {0.0f, 0.0f, 0.0f};
         far_finish(cp[k / 2], fs[k / 2], (k & 1u) != 0, e, b);
-        // triquadratic interpolation: the x and y contractions are tabulated per bin (t2)
         const float4 wz = sm.wyz[1][lz];
         const float wz3[3] = {wz.x, wz.y, wz.z};
-        const float4* tc = t2 + (size_t)(ly * L.bsx + lx) * 7u;
+        if (!COLUMNS) fetch(lx, ly);
         float far[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int iz = 0; iz < 3; iz++) {
-            const float4 a = tc[2 * iz], b2 = tc[2 * iz + 1];
+            const float4 a = ta[iz], b2 = tb[iz];
             far[0] = fmaf(wz3[iz], a.x, far[0]); far[1] = fmaf(wz3[iz], a.y, far[1]); far[2] = fmaf(wz3[iz], a.z, far[2]);
             far[3] = fmaf(wz3[iz], a.w, far[3]); far[4] = fmaf(wz3[iz], b2.x, far[4]); far[5] = fmaf(wz3[iz], b2.y, far[5]);
         }
