@@ -45,73 +45,64 @@ __device__ __forceinline__ void add_term(const P3& p, const float4& v, float (&e
     b[0] = b[0] + v.x * bx; b[1] = b[1] + v.x * by; b[2] = b[2] + v.x * bz;
 }
 
+// What a thread sums: the R neighbouring bins i0.. along x of one in-bin offset, in bin row (iy, iz)
+struct TableItem {
+    bool valid;
+    uint32_t i0, ox, oy, oz, iy, iz;
+    int ax0;  // 2 R_x of cell 0 and source 0
+};
 template <int ND, int R, int EB>
-__global__ void __launch_bounds__(EB * (ND / R), 512 / (EB * (ND / R))) k_update_e_b_table(const DevLbm L, const FieldTable F) {
-    constexpr uint32_t THREADS = EB * (ND / R);
-    __shared__ float4 src[ND * ND];  // one z plane of sources: (q, vx, vy, vz)
+__device__ __forceinline__ TableItem table_item(const DevLbm& L) {
+    TableItem t;
     const uint32_t no = L.bsx * L.bsy * L.bsz;
     const uint32_t item = blockIdx.x * EB + threadIdx.x % EB;  // (Iz, Iy, offset)
-    const bool valid = item < no * (ND * ND);
-    const uint32_t i0 = threadIdx.x / EB * R;
-    const uint32_t it = valid ? item : 0u;
-    const uint32_t o = it % no, iy = it / no % ND, iz = it / (no * ND);
-    const uint32_t ox = o % L.bsx, oy = o / L.bsx % L.bsy, oz = o / (L.bsx * L.bsy);
-    const int ax0 = (int)(2u * (L.bsx * i0 + ox)) - (int)L.bsx;  // 2 R_x of cell 0 and source 0
-    const int first = (int)L.first_src, last = (int)min(L.n_lod_own, L.n_bins);
-    float e[R][3], b[R][3];
-#pragma unroll
-    for (int i = 0; i < R; i++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) { e[i][c] = 0.0f; b[i][c] = 0.0f; }
-    for (int jz = first / (ND * ND); jz < ND; jz++) {
-        __syncthreads();
-        for (uint32_t k = threadIdx.x; k < ND * ND; k += THREADS)
-            src[k] = reinterpret_cast<const float4*>(L.qu_lod)[jz * (ND * ND) + k];
-        __syncthreads();
-        const int az = (int)(2u * (L.bsz * iz + oz)) - (int)L.bsz - 2 * (int)L.bsz * jz;
-        const uint32_t sz = (uint32_t)az & 0x80000000u;
-#pragma unroll 1
-        for (int jy = 0; jy < ND; jy++) {
-            const int d0 = (jz * ND + jy) * ND;
-            if (d0 + ND <= first || d0 >= last) continue;
-            const int ay = (int)(2u * (L.bsy * iy + oy)) - (int)L.bsy - 2 * (int)L.bsy * jy;
-            const uint32_t sy = (uint32_t)ay & 0x80000000u;
-            const float4* row = F.T + ((size_t)((uint32_t)abs(az) >> 1) * F.ty + ((uint32_t)abs(ay) >> 1)) * F.tx;
-            auto entry = [&](int ax) -> P3 {
-                const float4 t = __ldg(row + ((uint32_t)abs(ax) >> 1));
-                return {__uint_as_float(__float_as_uint(t.x) ^ ((uint32_t)ax & 0x80000000u)),
-                        __uint_as_float(__float_as_uint(t.y) ^ sy), __uint_as_float(__float_as_uint(t.z) ^ sz)};
-            };
-            int step = 2 * (int)L.bsx;
-            asm volatile("" : "+r"(step));  // the entries' indices are formed per row, not kept
-            const bool own_row = (uint32_t)jy == iy && (uint32_t)jz == iz;
-            if (d0 >= first && d0 + ND <= last && !__any_sync(0xFFFFFFFFu, own_row)) {
-                P3 p[R + ND - 1];  // entry k: bins R - 1 - k apart
-#pragma unroll
-                for (int k = 0; k < R - 1; k++) p[k] = entry(ax0 + (R - 1 - k) * step);
-#pragma unroll
-                for (int j = 0; j < ND; j++) {
-                    p[R - 1 + j] = entry(ax0 - j * step);
-                    const float4 v = src[jy * ND + j];
-#pragma unroll
-                    for (int i = 0; i < R; i++) add_term(p[R - 1 - i + j], v, e[i], b[i]);
-                }
-            } else {  // a row with a lane's own bin, or the first row (which starts inside a row)
-#pragma unroll 1
-                for (int j = max(first - d0, 0); j < min(last - d0, ND); j++) {
-                    const float4 v = src[jy * ND + j];
-#pragma unroll
-                    for (int i = 0; i < R; i++)
-                        if (!own_row || (int)i0 + i != j) add_term(entry(ax0 + (i - j) * step), v, e[i], b[i]);
-                }
-            }
-        }
+    t.valid = item < no * (ND * ND);
+    t.i0 = threadIdx.x / EB * R;
+    const uint32_t it = t.valid ? item : 0u, o = it % no;
+    t.iy = it / no % ND;
+    t.iz = it / (no * ND);
+    t.ox = o % L.bsx;
+    t.oy = o / L.bsx % L.bsy;
+    t.oz = o / (L.bsx * L.bsy);
+    t.ax0 = (int)(2u * (L.bsx * t.i0 + t.ox)) - (int)L.bsx;
+    return t;
+}
+// the table row of source row (jy, jz), and the signs of its entries
+struct TableRow {
+    const float4* row;
+    uint32_t sy, sz;
+    __device__ __forceinline__ TableRow(const DevLbm& L, const FieldTable& F, const TableItem& t, int jy, int jz) {
+        const int ay = (int)(2u * (L.bsy * t.iy + t.oy)) - (int)L.bsy - 2 * (int)L.bsy * jy;
+        const int az = (int)(2u * (L.bsz * t.iz + t.oz)) - (int)L.bsz - 2 * (int)L.bsz * jz;
+        sy = (uint32_t)ay & 0x80000000u;
+        sz = (uint32_t)az & 0x80000000u;
+        row = F.T + ((size_t)((uint32_t)abs(az) >> 1) * F.ty + ((uint32_t)abs(ay) >> 1)) * F.tx;
     }
-    if (!valid) return;
+    __device__ __forceinline__ P3 entry(int ax) const {
+        const float4 t = __ldg(row + ((uint32_t)abs(ax) >> 1));
+        return {__uint_as_float(__float_as_uint(t.x) ^ ((uint32_t)ax & 0x80000000u)),
+                __uint_as_float(__float_as_uint(t.y) ^ sy), __uint_as_float(__float_as_uint(t.z) ^ sz)};
+    }
+};
+// a row that holds a lane's own bin, or starts or ends inside the sources
+template <int ND, int R>
+__device__ __forceinline__ void table_edge_row(const TableRow& w, const TableItem& t, const float4* src, int d0, int first,
+                                               int last, bool own_row, int step, float (&e)[R][3], float (&b)[R][3]) {
+#pragma unroll 1
+    for (int j = max(first - d0, 0); j < min(last - d0, ND); j++) {
+        const float4 v = src[j];
+#pragma unroll
+        for (int i = 0; i < R; i++)
+            if (!own_row || (int)t.i0 + i != j) add_term(w.entry(t.ax0 + (i - j) * step), v, e[i], b[i]);
+    }
+}
+template <int R>
+__device__ __forceinline__ void table_store(const DevLbm& L, const TableItem& t, const float (&e)[R][3], const float (&b)[R][3]) {
+    if (!t.valid) return;
     const size_t N = L.n;
 #pragma unroll
     for (int i = 0; i < R; i++) {
-        const uint32_t n = (i0 + i) * L.bsx + ox + ((iy * L.bsy + oy) + (iz * L.bsz + oz) * L.ny) * L.nx;
+        const uint32_t n = (t.i0 + i) * L.bsx + t.ox + ((t.iy * L.bsy + t.oy) + (t.iz * L.bsz + t.oz) * L.ny) * L.nx;
         if ((L.flags[n] & F_BO) == F_S) continue;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -122,9 +113,48 @@ __global__ void __launch_bounds__(EB * (ND / R), 512 / (EB * (ND / R))) k_update
 }
 
 template <int ND, int R, int EB>
+__global__ void __launch_bounds__(EB * (ND / R), 512 / (EB * (ND / R))) k_update_e_b_table(const DevLbm L, const FieldTable F) {
+    constexpr uint32_t THREADS = EB * (ND / R);
+    __shared__ float4 src[ND * ND];  // one z plane of sources: (q, vx, vy, vz)
+    const TableItem t = table_item<ND, R, EB>(L);
+    const int first = (int)L.first_src, last = (int)min(L.n_lod_own, L.n_bins);
+    float e[R][3] = {}, b[R][3] = {};
+    for (int jz = first / (ND * ND); jz < ND; jz++) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < ND * ND; k += THREADS)
+            src[k] = reinterpret_cast<const float4*>(L.qu_lod)[jz * (ND * ND) + k];
+        __syncthreads();
+#pragma unroll 1
+        for (int jy = 0; jy < ND; jy++) {
+            const int d0 = (jz * ND + jy) * ND;
+            if (d0 + ND <= first || d0 >= last) continue;
+            const TableRow w(L, F, t, jy, jz);
+            int step = 2 * (int)L.bsx;
+            asm volatile("" : "+r"(step));  // the entries' indices are formed per row, not kept
+            const bool own_row = (uint32_t)jy == t.iy && (uint32_t)jz == t.iz;
+            if (d0 >= first && d0 + ND <= last && !__any_sync(0xFFFFFFFFu, own_row)) {
+                P3 p[R + ND - 1];  // entry k: bins R - 1 - k apart
+#pragma unroll
+                for (int k = 0; k < R - 1; k++) p[k] = w.entry(t.ax0 + (R - 1 - k) * step);
+#pragma unroll
+                for (int j = 0; j < ND; j++) {
+                    p[R - 1 + j] = w.entry(t.ax0 - j * step);
+                    const float4 v = src[jy * ND + j];
+#pragma unroll
+                    for (int i = 0; i < R; i++) add_term(p[R - 1 - i + j], v, e[i], b[i]);
+                }
+            } else {
+                table_edge_row<ND, R>(w, t, src + jy * ND, d0, first, last, own_row, step, e, b);
+            }
+        }
+    }
+    table_store<R>(L, t, e, b);
+}
+
+template <int ND, int R, int EB>
 cudaError_t launch(const DevLbm& L, const FieldTable& F, cudaStream_t s) {
-    const uint64_t items = (uint64_t)(L.n / ND);  // cells over the bins along x
-    k_update_e_b_table<ND, R, EB><<<(unsigned)((items + EB - 1) / EB), EB * (ND / R), 0, s>>>(L, F);
+    const unsigned items = L.n / ND;  // cells over the bins along x
+    k_update_e_b_table<ND, R, EB><<<(items + EB - 1) / EB, EB * (ND / R), 0, s>>>(L, F);
     return cudaGetLastError();
 }
 
@@ -150,10 +180,12 @@ cudaError_t launch_field_table(const DevLbm& L, const FieldTable& F, cudaStream_
 }
 
 // Four cells a thread amortise the table entries and the source best (24 against 26 instructions
-// a term); below 2^18 cells two cells a thread keep more of the SMs' schedulers supplied.
+// a term); small boxes fill the schedulers better with two: with three domains in turn 32^3 149
+// us (two) against 155 us a step, 48^3 336 against 306 us, 64^3 756 against 666 us; alone 216
+// against 305, 386 against 463 and 822 against 822 us.  The line lies between 32^3 and 48^3.
 cudaError_t launch_update_e_b_table(const DevLbm& L, const FieldTable& F, cudaStream_t s) {
-    const bool wide = L.n >= (1u << 18);
-    if (L.nd == 16u) return wide ? launch<16, 4, 64>(L, F, s) : launch<16, 2, 16>(L, F, s);
+    const bool wide = L.n >= 3u << 15;
+    if (L.nd == 16u) return wide ? launch<16, 4, 32>(L, F, s) : launch<16, 2, 16>(L, F, s);
     return wide ? launch<8, 4, 64>(L, F, s) : launch<8, 2, 32>(L, F, s);
 }
 
