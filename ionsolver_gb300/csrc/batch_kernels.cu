@@ -91,7 +91,9 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, 5) k_batch_stream_rows(const
     extern __shared__ __align__(128) uint8_t rows_smem[];
     __shared__ __align__(8) uint64_t full[2], empty[2];
     __shared__ DevLbm sL[2];                            // the domain of the row in each buffer
-    __shared__ uint32_t sdom[2], srow[2], fail_flag, issued;
+    __shared__ RowGroup sgroup[2];                      // the group of rows in each buffer,
+    __shared__ uint2 scells[2];                         // its first cell and their number
+    __shared__ uint32_t sdom[2], fail_flag, issued;
     volatile uint32_t* fail = &fail_flag;
     const bool odd = odd_t != 0u;
     const uint32_t nct = blockDim.x - 32u, ncw = nct / 32u;  // compute threads and warps
@@ -115,9 +117,9 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, 5) k_batch_stream_rows(const
             auto write_back = [&](uint32_t k) {
                 const uint32_t b = k & 1u;
                 const DevLbm& L = sL[b];
-                const uint8_t* src = rows_smem + b * RB;
-                const uint32_t rb = L.nx * (uint32_t)sizeof(T);
-                for_row_streams<FT, MHD>(L, srow[b], odd, [&](uint32_t st, T* g) { bulk_s2g(g, src + st * SB, rb); });
+                const RowGroup R = sgroup[b];
+                for_group_streams<FT, MHD>(L, R, odd, rows_smem + b * RB,
+                                           [&](uint32_t st, T* g, uint8_t* at, uint32_t bytes) { bulk_s2g(g, at + st * SB, bytes); });
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             };
             uint32_t k = 0;
@@ -136,20 +138,25 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, 5) k_batch_stream_rows(const
                     sL[b] = B.doms[d];
                     sdom[b] = d;
                 }
-                srow[b] = r;
                 const DevLbm& L = sL[b];
-                const uint32_t nx = L.nx, N = L.n, own = r * nx, rb = nx * (uint32_t)sizeof(T);
+                const uint32_t N = L.n;
+                const RowGroup R(r, RS / L.nx, L.ny);
+                const uint32_t own = (R.y + R.z * L.ny) * L.nx, cells = R.rows * L.nx;
+                sgroup[b] = R;
+                scells[b] = make_uint2(own, cells);
                 uint8_t* dst = rows_smem + b * RB;
-                // (the arrive below releases the view and row index written above)
-                mbar_expect_tx(&full[b], row_streams<FT, MHD>() * rb + (MHD ? 6u * nx * 4u : 0u) + ((nx + 15u) & ~15u));
-                for_row_streams<FT, MHD>(L, r, odd, [&](uint32_t st, T* gp) { bulk_g2s(dst + st * SB, gp, rb, &full[b]); });
+                // (the arrive below releases the view and group index written above)
+                mbar_expect_tx(&full[b], cells * (row_streams<FT, MHD>() * (uint32_t)sizeof(T) + (MHD ? 24u : 0u) + 1u));
+                for_group_streams<FT, MHD>(L, R, odd, dst, [&](uint32_t st, T* gp, uint8_t* at, uint32_t bytes) {
+                    bulk_g2s(at + st * SB, gp, bytes, &full[b]);
+                });
                 if constexpr (MHD) {
                     for (uint32_t c = 0; c < 3; c++) {
-                        bulk_g2s(dst + eb_off + c * RS * 4u, L.b_dyn + (size_t)c * N + own, nx * 4u, &full[b]);
-                        bulk_g2s(dst + eb_off + (3u + c) * RS * 4u, L.e_dyn + (size_t)c * N + own, nx * 4u, &full[b]);
+                        bulk_g2s(dst + eb_off + c * RS * 4u, L.b_dyn + (size_t)c * N + own, cells * 4u, &full[b]);
+                        bulk_g2s(dst + eb_off + (3u + c) * RS * 4u, L.e_dyn + (size_t)c * N + own, cells * 4u, &full[b]);
                     }
                 }
-                bulk_g2s(dst + fl_off, L.flags + own, (nx + 15u) & ~15u, &full[b]);
+                bulk_g2s(dst + fl_off, L.flags + own, cells, &full[b]);
                 issued = k + 1u;
             }
             // the last (up to) two rows, once computed
@@ -169,13 +176,12 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, 5) k_batch_stream_rows(const
             const bool go = mbar_wait_or_fail(&full[b], (k >> 1) & 1u, fail, limit) && *fail == 0u;
             if (go) {
                 const DevLbm& L = sL[b];
-                const uint32_t nx = L.nx, r = srow[b];
+                const uint32_t own = scells[b].x, cells = scells[b].y;
                 uint8_t* buf = rows_smem + b * RB;
-                for (uint32_t x = threadIdx.x; x < nx; x += nct) {
-                    const RowSrc<T, RS, true> S{buf, nx, x, x + 1u == nx ? 0u : x + 1u, x == 0u ? nx - 1u : x - 1u,
-                                                 eb_off, fl_off};
-                    if (L.trt) sc_cell<19, FT, MHD, true, false, RowSrc<T, RS, true>, uint32_t>(L, x + r * nx, odd, S);
-                    else sc_cell<19, FT, MHD, false, false, RowSrc<T, RS, true>, uint32_t>(L, x + r * nx, odd, S);
+                for (uint32_t t = threadIdx.x; t < cells; t += nct) {
+                    const RowSrc<T, RS, true> S = group_cell<T, RS>(L, buf, t, eb_off, fl_off);
+                    if (L.trt) sc_cell<19, FT, MHD, true, false, RowSrc<T, RS, true>, uint32_t>(L, own + t, odd, S);
+                    else sc_cell<19, FT, MHD, false, false, RowSrc<T, RS, true>, uint32_t>(L, own + t, odd, S);
                 }
                 // the new DDFs (generic-proxy writes) become visible to the bulk copies
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -1346,7 +1346,7 @@ struct ion_batch {
     uint32_t* d_gated_off = nullptr;
     const uint32_t** d_gates = nullptr;  // [domains]: FftField::direct, null without a convolution
     uint32_t gated_bricks = 0;
-    uint32_t* d_row_off = nullptr;  // row-staged stencil: prefix sums of ny nz (null: tiles of cells)
+    uint32_t* d_row_off = nullptr;  // row-staged stencil: prefix sums of the groups of rows (null: tiles of cells)
     uint32_t total_rows = 0;
     uint32_t* d_err = nullptr;
     uint64_t t = 0;
@@ -1567,7 +1567,8 @@ int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out) {
     for (uint32_t i = 0; i < count; i++) {
         const DevLbm& L = domains[i]->L;
         rows_ok = rows_ok && L.nx % 16u == 0u && L.nx <= BATCH_ROW_MAX && 19ull * L.n < (1ull << 32);
-        rows[i + 1] = rows[i] + L.ny * L.nz;
+        const uint32_t K = L.nx <= BATCH_ROW_STRIDE ? BATCH_ROW_STRIDE / L.nx : 1u;  // rows a group
+        rows[i + 1] = rows[i] + (L.ny + K - 1u) / K * L.nz;
     }
     if (!rc && rows_ok) {
         b->total_rows = rows[count];

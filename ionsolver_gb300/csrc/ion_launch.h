@@ -68,7 +68,7 @@ struct BatchDev {
     const uint32_t* bin_off;   // [ndom+1] prefix sums of lod_blocks (LOD bin groups; 1 at depth 0)
     uint32_t total_bins;
     uint32_t* err;
-    const uint32_t* row_off;   // [ndom+1] prefix sums of ny nz (the row-staged stencil), or null
+    const uint32_t* row_off;   // [ndom+1] prefix sums of the groups of rows (the row-staged stencil), or null
     uint32_t total_rows;       // 0: the stencil runs in tiles of cells with global loads
 };
 // threads per block of the batch's stencil kernel (its tiles: BATCH_SC_THREADS * EB_CPT cells;

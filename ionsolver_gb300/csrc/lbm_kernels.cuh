@@ -612,11 +612,10 @@ __host__ __device__ inline uint32_t row_bytes(uint32_t nx) {
 // compute the row.  So the offsets of the seven neighbour rows are formed once, every stream is
 // unrolled, and a slot's address is two multiply-adds (19 N < 2^32: 32-bit offsets).
 template <int FT, bool MHD, class OP>
-__device__ __forceinline__ void for_row_streams(const DevLbm& L, uint32_t r, bool odd, OP&& op) {
+__device__ __forceinline__ void for_row_streams(const DevLbm& L, uint32_t y, uint32_t z, bool odd, OP&& op) {
     using V = VSet<19>;
     using T = typename Ddf<FT>::T;
     const uint32_t nx = L.nx, ny = L.ny, nz = L.nz, N = L.n;
-    const uint32_t z = r / ny, y = r - z * ny;
     const uint32_t yp = y + 1u == ny ? 0u : y + 1u, ym = y == 0u ? ny - 1u : y - 1u;
     const uint32_t zp = (z + 1u == nz ? 0u : z + 1u) * ny, zm = (z == 0u ? nz - 1u : z - 1u) * ny, z0 = z * ny;
     const uint32_t own = (y + z0) * nx;
@@ -676,7 +675,7 @@ __global__ void __launch_bounds__(256, 2) k_sc_rows(const DevLbm L, const uint32
         uint8_t* dst = rows_smem + b * RB;
         const uint32_t own = r * nx;
         mbar_expect_tx(&bar[b], RB);
-        for_row_streams<FT, MHD>(L, r, odd, [&](uint32_t st, T* g) { bulk_g2s(dst + st * rb, g, rb, &bar[b]); });
+        for_row_streams<FT, MHD>(L, r % ny, r / ny, odd, [&](uint32_t st, T* g) { bulk_g2s(dst + st * rb, g, rb, &bar[b]); });
         if constexpr (MHD) {
             for (uint32_t c = 0; c < 3; c++) {
                 bulk_g2s(dst + eb_off + c * nx * 4u, L.b_dyn + (size_t)c * N + own, nx * 4u, &bar[b]);
@@ -711,6 +710,33 @@ __global__ void __launch_bounds__(256, 2) k_sc_rows(const DevLbm L, const uint32
     }
 }
 
+// Short rows are staged several at a time: a group is up to K rows that follow each other in y,
+// which every stream holds as one stretch of memory, its neighbour rows as well, except where
+// they wrap around in y.  There the group's rows are copied one by one.
+struct RowGroup {
+    uint32_t y, z, rows;  // the first row and their number
+    bool whole;           // one copy a stream
+    RowGroup() = default;
+    __device__ __forceinline__ RowGroup(uint32_t g, uint32_t K, uint32_t ny) {
+        const uint32_t per = (ny + K - 1u) / K;
+        z = g / per;
+        y = (g - z * per) * K;
+        rows = min(K, ny - y);
+        whole = rows == 1u || (y > 0u && y + rows < ny);
+    }
+};
+__host__ __device__ inline uint32_t row_groups(uint32_t ny, uint32_t nz, uint32_t K) { return (ny + K - 1u) / K * nz; }
+// The copies of a group: op(stream, pointer in global memory, staged stretch, bytes) with the
+// stretch at `staged` (the group's buffer) or a row's share of it.
+template <int FT, bool MHD, class OP>
+__device__ __forceinline__ void for_group_streams(const DevLbm& L, const RowGroup& G, bool odd, uint8_t* staged, OP&& op) {
+    using T = typename Ddf<FT>::T;
+    const uint32_t row = L.nx * (uint32_t)sizeof(T), bytes = G.whole ? G.rows * row : row, end = G.y + (G.whole ? 1u : G.rows);
+#pragma unroll 1
+    for (uint32_t y = G.y; y < end; y++, staged += row)
+        for_row_streams<FT, MHD>(L, y, G.z, odd, [&](uint32_t st, T* g) { op(st, g, staged, bytes); });
+}
+
 // waits for an mbarrier phase; gives up after `limit` polls (setting *fail) or as soon
 // as another warp has set *fail
 __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, volatile uint32_t* fail,
@@ -726,6 +752,14 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// cell t of a staged group of rows, periodic within its row
+template <class T, uint32_t RS>
+__device__ __forceinline__ RowSrc<T, RS, true> group_cell(const DevLbm& L, uint8_t* buf, uint32_t t, uint32_t eb_off,
+                                                          uint32_t fl_off) {
+    const uint32_t nx = L.nx, x = t - L.dx.div(t) * nx;
+    return {buf, nx, t, x + 1u == nx ? t - x : t + 1u, x == 0u ? t + nx - 1u : t - 1u, eb_off, fl_off};
+}
+
 // Rows of up to 384 cells (WS_ROW): blockDim.x = compute threads + 32.  The last warp
 // stages rows and writes them back; the others compute (one cell per thread and row).
 // The row buffer has a fixed stride of RS elements per stream (the smallest of 96,
@@ -737,7 +771,7 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
 // so no other CTA touches them within the step.  The other outputs (q, the LOD
 // velocity, rho, u) are stored directly.
 constexpr uint32_t WS_ROW = 384;
-__host__ __device__ constexpr int ws_variant(uint32_t nx) { return nx <= 96u ? 0 : nx <= 128u ? 1 : nx <= 192u ? 2 : nx <= 256u ? 3 : 4; }
+__host__ __device__ constexpr uint32_t ws_rows(int v) { return v == 0 ? 96u : v == 1 ? 128u : v == 2 ? 192u : v == 3 ? 256u : 384u; }
 template <int FT, bool MHD, uint32_t RS>
 __host__ __device__ constexpr uint32_t ws_row_bytes() {
     return row_streams<FT, MHD>() * RS * (uint32_t)sizeof(typename Ddf<FT>::T) + (MHD ? 6u * RS * 4u : 0u) + RS;
@@ -757,6 +791,7 @@ __host__ __device__ constexpr int ws_min_ctas() {
 template <int FT, bool MHD, bool TRT, uint32_t RS>
 __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_t, uint32_t* err) {
     using T = typename Ddf<FT>::T;
+    const uint32_t K = RS / L.nx;  // rows a group
     constexpr uint32_t RB = ws_row_bytes<FT, MHD, RS>();
     constexpr uint32_t SB = RS * (uint32_t)sizeof(T);  // bytes per stream row
     constexpr uint32_t eb_off = row_streams<FT, MHD>() * SB, fl_off = eb_off + (MHD ? 6u * RS * 4u : 0u);
@@ -765,8 +800,7 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
     __shared__ uint32_t fail_flag, issued;  // rows the producer has staged
     volatile uint32_t* fail = &fail_flag;
     const bool odd = odd_t != 0u;
-    const uint32_t nx = L.nx, ny = L.ny, nz = L.nz, nrows = ny * nz, N = L.n;
-    const uint32_t rb = nx * (uint32_t)sizeof(T);  // bytes of one stream's row in global memory
+    const uint32_t nx = L.nx, ny = L.ny, nz = L.nz, nrows = row_groups(ny, nz, K), N = L.n;  // (groups of rows)
     const uint32_t nct = blockDim.x - 32u, ncw = nct / 32u;  // compute threads and warps
     if (threadIdx.x == 0) {
         mbar_init(&full[0], 1u);
@@ -781,18 +815,18 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
     const uint32_t my_rows = blockIdx.x < nrows ? (nrows - 1u - blockIdx.x) / gridDim.x + 1u : 0u;
     if (threadIdx.x >= nct) {
         if (threadIdx.x == nct) {
-            auto for_streams = [&](uint32_t r, auto&& op) { for_row_streams<FT, MHD>(L, r, odd, op); };
-            // row k of this CTA lives in buffer k & 1
+            // group k of this CTA lives in buffer k & 1
             auto write_back = [&](uint32_t k) {
-                const uint8_t* src = rows_smem + (k & 1u) * RB;
-                for_streams(blockIdx.x + k * gridDim.x, [&](uint32_t st, T* g) { bulk_s2g(g, src + st * SB, rb); });
+                const RowGroup R(blockIdx.x + k * gridDim.x, K, ny);
+                for_group_streams<FT, MHD>(L, R, odd, rows_smem + (k & 1u) * RB,
+                                           [&](uint32_t st, T* g, uint8_t* at, uint32_t bytes) { bulk_s2g(g, at + st * SB, bytes); });
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             };
             uint32_t k = 0;
             for (; k < my_rows; k++) {
-                const uint32_t b = k & 1u, r = blockIdx.x + k * gridDim.x;
+                const uint32_t b = k & 1u;
                 if (k >= 2) {
-                    // row k - 2 computed: copy it back, and wait until the copies have read the buffer
+                    // group k - 2 computed: copy it back, and wait until the copies have read the buffer
                     if (!mbar_wait_or_fail(&empty[b], ((k - 2) >> 1) & 1u, fail, L.wait_limit)) break;
                     if (*fail) break;
                     write_back(k - 2u);
@@ -800,16 +834,19 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
                 }
                 if (*fail) break;
                 uint8_t* dst = rows_smem + b * RB;
-                const uint32_t y = r % ny, z = r / ny, own = (y + z * ny) * nx;
-                mbar_expect_tx(&full[b], row_streams<FT, MHD>() * rb + (MHD ? 6u * nx * 4u : 0u) + ((nx + 15u) & ~15u));
-                for_streams(r, [&](uint32_t st, T* g) { bulk_g2s(dst + st * SB, g, rb, &full[b]); });
+                const RowGroup R(blockIdx.x + k * gridDim.x, K, ny);
+                const uint32_t own = (R.y + R.z * ny) * nx, cells = R.rows * nx;
+                mbar_expect_tx(&full[b], cells * (row_streams<FT, MHD>() * (uint32_t)sizeof(T) + (MHD ? 24u : 0u) + 1u));
+                for_group_streams<FT, MHD>(L, R, odd, dst, [&](uint32_t st, T* g, uint8_t* at, uint32_t bytes) {
+                    bulk_g2s(at + st * SB, g, bytes, &full[b]);
+                });
                 if constexpr (MHD) {
                     for (uint32_t c = 0; c < 3; c++) {
-                        bulk_g2s(dst + eb_off + c * RS * 4u, L.b_dyn + (size_t)c * N + own, nx * 4u, &full[b]);
-                        bulk_g2s(dst + eb_off + (3u + c) * RS * 4u, L.e_dyn + (size_t)c * N + own, nx * 4u, &full[b]);
+                        bulk_g2s(dst + eb_off + c * RS * 4u, L.b_dyn + (size_t)c * N + own, cells * 4u, &full[b]);
+                        bulk_g2s(dst + eb_off + (3u + c) * RS * 4u, L.e_dyn + (size_t)c * N + own, cells * 4u, &full[b]);
                     }
                 }
-                bulk_g2s(dst + fl_off, L.flags + own, (nx + 15u) & ~15u, &full[b]);
+                bulk_g2s(dst + fl_off, L.flags + own, cells, &full[b]);
                 issued = k + 1u;
             }
             // the last (up to) two rows, once computed
@@ -825,15 +862,15 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
     } else {
         const uint32_t lane = threadIdx.x & 31u;
         for (uint32_t k = 0; k < my_rows; k++) {
-            const uint32_t b = k & 1u, r = blockIdx.x + k * gridDim.x;
+            const uint32_t b = k & 1u;
             const bool go = mbar_wait_or_fail(&full[b], (k >> 1) & 1u, fail, L.wait_limit) && *fail == 0u;
             if (go) {
                 uint8_t* buf = rows_smem + b * RB;
-                const uint32_t y = r % ny, z = r / ny;
-                for (uint32_t x = threadIdx.x; x < nx; x += nct) {
-                    const RowSrc<T, RS, true> S{buf, nx, x, x + 1u == nx ? 0u : x + 1u, x == 0u ? nx - 1u : x - 1u,
-                                                 eb_off, fl_off};
-                    sc_cell<19, FT, MHD, TRT, false, RowSrc<T, RS, true>, uint32_t>(L, x + (y + z * ny) * nx, odd, S);
+                const RowGroup R(blockIdx.x + k * gridDim.x, K, ny);
+                const uint32_t own = (R.y + R.z * ny) * nx, cells = R.rows * nx;
+                for (uint32_t t = threadIdx.x; t < cells; t += nct) {
+                    const RowSrc<T, RS, true> S = group_cell<T, RS>(L, buf, t, eb_off, fl_off);
+                    sc_cell<19, FT, MHD, TRT, false, RowSrc<T, RS, true>, uint32_t>(L, own + t, odd, S);
                 }
                 // the new DDFs (generic-proxy writes) become visible to the bulk copies
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -852,58 +889,97 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
     }
 }
 
+// How the row kernels run on a grid: the kernel (a row stride of k_sc_rows_ws, or k_sc_rows), the
+// rows of a group, the block and the blocks per SM.
+struct RowPlan {
+    uint32_t nx, ny, nz;  // the grid it was made for
+    int v;
+    uint32_t K, threads, smem;
+    int per_sm;           // 0: the rows do not fit
+};
+
+// The smallest stride that holds a row, or, with 16-bit storage and without MHD, a wider one
+// that stages several short rows at a time: the one thread that issues the copies then has
+// fewer, longer ones.  It is taken where it keeps at least 5% more cells on an SM and the
+// groups still feed every resident block at least twice (four times without MHD).  MHD
+// FP16S, one stride against the wider: 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31
+// us; plain FP32 112^3 41 -> 37 us, FP16S 128^3 51 -> 46 us.  FP32 MHD holds its SMs' shared
+// memory with the smallest stride already (64 to 128 cells: within 2%).
+template <int FT, bool MHD, bool TRT>
+RowPlan make_row_plan(const DevLbm& L, int sms) {
+    using Kern = void (*)(const DevLbm, const uint32_t, uint32_t*);
+    static const Kern kern[6] = {k_sc_rows_ws<FT, MHD, TRT, 96u>,  k_sc_rows_ws<FT, MHD, TRT, 128u>,
+                                 k_sc_rows_ws<FT, MHD, TRT, 192u>, k_sc_rows_ws<FT, MHD, TRT, 256u>,
+                                 k_sc_rows_ws<FT, MHD, TRT, 384u>, k_sc_rows<FT, MHD, TRT>};
+    static constexpr uint32_t bytes[5] = {ws_row_bytes<FT, MHD, 96u>(), ws_row_bytes<FT, MHD, 128u>(), ws_row_bytes<FT, MHD, 192u>(),
+                                          ws_row_bytes<FT, MHD, 256u>(), ws_row_bytes<FT, MHD, 384u>()};
+    static_assert(2u * ws_row_bytes<ION_FP32, true, WS_ROW>() <= 200u * 1024u, "two row buffers of the widest form");
+    RowPlan best{L.nx, L.ny, L.nz, 0, 0u, 0u, 0u, 0};
+    const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
+    for (int v = ws ? 0 : 5; v < 6; v++) {
+        RowPlan p = best;
+        p.v = v;
+        if (v < 5) {
+            if (ws_rows(v) < L.nx) continue;
+            p.K = ws_rows(v) / L.nx;
+            p.smem = 2u * bytes[v];
+            p.threads = (p.K * L.nx + 31u) / 32u * 32u + 32u;
+        } else {
+            if (ws) break;
+            p.K = 1u;
+            p.smem = 2u * row_bytes<FT, MHD>(L.nx);
+            p.threads = ((L.nx + ((L.nx + 255u) / 256u) - 1u) / ((L.nx + 255u) / 256u) + 31u) / 32u * 32u;
+        }
+        p.per_sm = 0;
+        if (p.smem > 200u * 1024u ||
+            cudaFuncSetAttribute(kern[v], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p.per_sm, kern[v], (int)p.threads, p.smem) != cudaSuccess || p.per_sm < 1)
+            continue;
+        if (best.per_sm == 0) {
+            best = p;
+            if (FT == ION_FP32 && MHD) break;
+        } else if ((uint64_t)p.per_sm * p.K * 100u > (uint64_t)best.per_sm * best.K * 105u &&
+                   row_groups(L.ny, L.nz, p.K) >= (MHD ? 2u : 4u) * (uint32_t)(p.per_sm * sms)) {
+            best = p;
+        }
+    }
+    return best;
+}
+
 // the row kernels when the domain's rows can be copied as whole 16-byte-aligned
 // streams and two buffers fit in shared memory; false: use k_stream_collide
 template <int FT, bool MHD, bool TRT>
 bool launch_sc_rows(const DevLbm& L, uint32_t o, uint32_t* err, cudaStream_t s) {
-    // whole 16-byte rows, two buffers in shared memory, and 32-bit slot offsets (19 N < 2^32)
-    const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
-    const int v = ws ? ws_variant(L.nx) : 5;
-    static_assert(2u * ws_row_bytes<ION_FP32, true, WS_ROW>() <= 200u * 1024u, "two row buffers of the widest form");
-    const uint32_t smem = 2u * (v == 0   ? ws_row_bytes<FT, MHD, 96u>()
-                                : v == 1 ? ws_row_bytes<FT, MHD, 128u>()
-                                : v == 2 ? ws_row_bytes<FT, MHD, 192u>()
-                                : v == 3 ? ws_row_bytes<FT, MHD, 256u>()
-                                : v == 4 ? ws_row_bytes<FT, MHD, 384u>()
-                                         : row_bytes<FT, MHD>(L.nx));
-    if (L.nx % 16u || smem > 200u * 1024u || 19ull * L.n >= (1ull << 32)) return false;
-    const uint32_t threads =
-        ws ? (L.nx + 31u) / 32u * 32u + 32u : ((L.nx + ((L.nx + 255u) / 256u) - 1u) / ((L.nx + 255u) / 256u) + 31u) / 32u * 32u;
-    auto kern = v == 0   ? k_sc_rows_ws<FT, MHD, TRT, 96u>
-                : v == 1 ? k_sc_rows_ws<FT, MHD, TRT, 128u>
-                : v == 2 ? k_sc_rows_ws<FT, MHD, TRT, 192u>
-                : v == 3 ? k_sc_rows_ws<FT, MHD, TRT, 256u>
-                : v == 4 ? k_sc_rows_ws<FT, MHD, TRT, 384u>
-                         : k_sc_rows<FT, MHD, TRT>;
-    // the shared-memory opt-in and the occupancy of the last shape, per instantiation
-    // (handles may step on several host threads)
-    static std::mutex mu;
-    static bool attr[6] = {};
-    static int per_sm_of[6] = {};
-    static uint32_t for_smem[6] = {}, for_threads[6] = {};
-    int per_sm = 0;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!attr[v]) {
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-                return false;
-            attr[v] = true;
-        }
-        if (for_smem[v] != smem || for_threads[v] != threads) {
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_of[v], kern, (int)threads, smem) != cudaSuccess ||
-                per_sm_of[v] < 1)
-                return false;
-            for_smem[v] = smem;
-            for_threads[v] = threads;
-        }
-        per_sm = per_sm_of[v];
-    }
+    // whole 16-byte rows and 32-bit slot offsets (19 N < 2^32)
+    if (L.nx % 16u || 19ull * L.n >= (1ull << 32)) return false;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t rows = L.ny * L.nz;
-    const uint32_t grid = std::min<uint32_t>(rows, (uint32_t)(per_sm * sms));
-    kern<<<grid, threads, smem, s>>>(L, o, err);
+    // the plans of the last few grids, per instantiation (handles may step on several host threads)
+    static std::mutex mu;
+    static RowPlan plans[8] = {};
+    static uint32_t next = 0;
+    RowPlan p{};
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const RowPlan* hit = nullptr;
+        for (const RowPlan& q : plans)
+            if (q.nx == L.nx && q.ny == L.ny && q.nz == L.nz) hit = &q;
+        if (!hit) {
+            plans[next] = make_row_plan<FT, MHD, TRT>(L, sms);
+            hit = &plans[next];
+            next = (next + 1u) % 8u;
+        }
+        p = *hit;
+    }
+    if (p.per_sm < 1) return false;
+    const uint32_t grid = std::min<uint32_t>(row_groups(L.ny, L.nz, p.K), (uint32_t)(p.per_sm * sms));
+    if (p.v == 0) k_sc_rows_ws<FT, MHD, TRT, 96u><<<grid, p.threads, p.smem, s>>>(L, o, err);
+    else if (p.v == 1) k_sc_rows_ws<FT, MHD, TRT, 128u><<<grid, p.threads, p.smem, s>>>(L, o, err);
+    else if (p.v == 2) k_sc_rows_ws<FT, MHD, TRT, 192u><<<grid, p.threads, p.smem, s>>>(L, o, err);
+    else if (p.v == 3) k_sc_rows_ws<FT, MHD, TRT, 256u><<<grid, p.threads, p.smem, s>>>(L, o, err);
+    else if (p.v == 4) k_sc_rows_ws<FT, MHD, TRT, 384u><<<grid, p.threads, p.smem, s>>>(L, o, err);
+    else k_sc_rows<FT, MHD, TRT><<<grid, p.threads, p.smem, s>>>(L, o, err);
     return true;
 }
 
