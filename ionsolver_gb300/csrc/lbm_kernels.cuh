@@ -756,7 +756,7 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity
 template <class T, uint32_t RS>
 __device__ __forceinline__ RowSrc<T, RS, true> group_cell(const DevLbm& L, uint8_t* buf, uint32_t t, uint32_t eb_off,
                                                           uint32_t fl_off) {
-    const uint32_t nx = L.nx, x = t - L.dx.div(t) * nx;
+    const uint32_t nx = L.nx, x = t < nx ? t : t - L.dx.div(t) * nx;
     return {buf, nx, t, x + 1u == nx ? t - x : t + 1u, x == 0u ? t + nx - 1u : t - 1u, eb_off, fl_off};
 }
 
@@ -797,7 +797,8 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
     constexpr uint32_t eb_off = row_streams<FT, MHD>() * SB, fl_off = eb_off + (MHD ? 6u * RS * 4u : 0u);
     extern __shared__ __align__(128) uint8_t rows_smem[];
     __shared__ __align__(8) uint64_t full[2], empty[2];
-    __shared__ uint32_t fail_flag, issued;  // rows the producer has staged
+    __shared__ uint2 group[2];              // first cell and cells of the group in each buffer
+    __shared__ uint32_t fail_flag, issued;  // groups the producer has staged
     volatile uint32_t* fail = &fail_flag;
     const bool odd = odd_t != 0u;
     const uint32_t nx = L.nx, ny = L.ny, nz = L.nz, nrows = row_groups(ny, nz, K), N = L.n;  // (groups of rows)
@@ -836,6 +837,7 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
                 uint8_t* dst = rows_smem + b * RB;
                 const RowGroup R(blockIdx.x + k * gridDim.x, K, ny);
                 const uint32_t own = (R.y + R.z * ny) * nx, cells = R.rows * nx;
+                group[b] = make_uint2(own, cells);  // (released by the arrive below)
                 mbar_expect_tx(&full[b], cells * (row_streams<FT, MHD>() * (uint32_t)sizeof(T) + (MHD ? 24u : 0u) + 1u));
                 for_group_streams<FT, MHD>(L, R, odd, dst, [&](uint32_t st, T* g, uint8_t* at, uint32_t bytes) {
                     bulk_g2s(at + st * SB, g, bytes, &full[b]);
@@ -866,8 +868,7 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
             const bool go = mbar_wait_or_fail(&full[b], (k >> 1) & 1u, fail, L.wait_limit) && *fail == 0u;
             if (go) {
                 uint8_t* buf = rows_smem + b * RB;
-                const RowGroup R(blockIdx.x + k * gridDim.x, K, ny);
-                const uint32_t own = (R.y + R.z * ny) * nx, cells = R.rows * nx;
+                const uint32_t own = group[b].x, cells = group[b].y;
                 for (uint32_t t = threadIdx.x; t < cells; t += nct) {
                     const RowSrc<T, RS, true> S = group_cell<T, RS>(L, buf, t, eb_off, fl_off);
                     sc_cell<19, FT, MHD, TRT, false, RowSrc<T, RS, true>, uint32_t>(L, own + t, odd, S);
@@ -901,9 +902,9 @@ struct RowPlan {
 // The smallest stride that holds a row, or, with 16-bit storage and without MHD, a wider one
 // that stages several short rows at a time: the one thread that issues the copies then has
 // fewer, longer ones.  It is taken where it keeps at least 5% more cells on an SM and the
-// groups still feed every resident block at least twice (four times without MHD).  MHD
-// FP16S, one stride against the wider: 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31
-// us; plain FP32 112^3 41 -> 37 us, FP16S 128^3 51 -> 46 us.  FP32 MHD holds its SMs' shared
+// groups still feed every resident block at least twice.  The smallest stride against the
+// wider: MHD FP16S 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31 us; plain FP32 112^3
+// 41 -> 37 us, FP16S 128^3 51 -> 46 us, 64^3 FP32 6.6 -> 6.0 us (three domains in turn).  FP32 MHD holds its SMs' shared
 // memory with the smallest stride already (64 to 128 cells: within 2%).
 template <int FT, bool MHD, bool TRT>
 RowPlan make_row_plan(const DevLbm& L, int sms) {
@@ -939,7 +940,7 @@ RowPlan make_row_plan(const DevLbm& L, int sms) {
             best = p;
             if (FT == ION_FP32 && MHD) break;
         } else if ((uint64_t)p.per_sm * p.K * 100u > (uint64_t)best.per_sm * best.K * 105u &&
-                   row_groups(L.ny, L.nz, p.K) >= (MHD ? 2u : 4u) * (uint32_t)(p.per_sm * sms)) {
+                   row_groups(L.ny, L.nz, p.K) >= 2u * (uint32_t)(p.per_sm * sms)) {
             best = p;
         }
     }
