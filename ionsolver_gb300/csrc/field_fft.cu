@@ -9,8 +9,7 @@
 // operations per cell where the direct sum (field_kernels.cuh, eb_tile) takes 56,000.
 // The sources are the direct sum's: bins [first_src, 8^D), (q, q v) with q v rounded first.
 //
-//   k_fft_plan  once per grid shape: spectra of R/|R|^3 (64-bit sums and transforms,
-//               rounded to 32 bits).  An offset o and its mirror image b - o have spectra
+//   k_fft_plan  once per grid shape: spectra of R/|R|^3.  An offset o and its mirror image b - o have spectra
 //               that differ by the sign of a wave number and of a component, so
 //               (b/2 + 1) of b offsets per axis are kept.
 //   k_fft_src   spectra of the sources, 4 (nd + 1) blocks; block 0 also looks at the range
@@ -20,8 +19,8 @@
 //               shared memory.
 //   k_fft_put   the sums to the cells, x-rows at a time: E_stat + KE e, B_stat + KMU b.
 //
-// Rounding: a 32-bit transform's error is about 1.5e-7 of the field's norm (the direct
-// 32-bit sums: 1.1e-6), spread evenly over the lattice.  An infinite bin would leave NaN
+// Rounding: the field's error against 64 bits is 1.6e-7 to 2.2e-7 of its norm from 8^3 to 256^3
+// cells (the direct 32-bit sums: 2.6e-7 to 8.6e-7), spread evenly over the lattice.  An infinite bin would leave NaN
 // where the direct sum keeps the sign, and sums near the ends of the exponent range would
 // over- or underflow at other places; so for sources that are infinite, or whose largest value
 // lies outside [1e-28, 1e25], `direct` is set and k_update_e_b_gated runs instead (a NaN
@@ -54,51 +53,47 @@ __constant__ float2 c_tw[32] = {  // exp(2 pi i j / 32)
 #undef ION_TW
 
 // ---------------------------------------------------------------------------
-// spectra of R/|R|^3: one block per distinct offset and kx
+// spectra of R/|R|^3: one block per distinct offset and kx.  In 32 bits: |2 R|^2 is exact, and
+// the transforms' error adds to that of the step's (together 2e-7 of the field's norm).  A
+// 256^3 grid's plan takes 0.58 ms; in 64 bits, at 1/64 of the rate, it took 21 ms
 // ---------------------------------------------------------------------------
 template <int ND>
 __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField F) {
-    constexpr int M = 2 * ND;
-    extern __shared__ __align__(16) uint8_t plan_smem[];
-    C2<double>* a = reinterpret_cast<C2<double>*>(plan_smem);  // [component][mz][my], rows of M + 1
-    __shared__ C2<double> tw[M];
-    constexpr int ROW = M + 1;
+    constexpr int M = 2 * ND, ROW = M + 1;
+    __shared__ C2<float> a[3 * M * ROW];  // [component][mz][my], rows of M + 1
+    __shared__ C2<float> tw[M];
     const uint32_t kx = blockIdx.x % (ND + 1u), u = blockIdx.x / (ND + 1u);
     const uint32_t ox = u % F.ux, oy = (u / F.ux) % F.uy, oz = u / (F.ux * F.uy);
     if (threadIdx.x < M) {
-        const int j = (int)((threadIdx.x * kx) % M) * (32 / M);
-        tw[threadIdx.x] = {cospi(j / 16.0), -sinpi(j / 16.0)};
+        const float2 w = c_tw[((threadIdx.x * kx) % M) * (32 / M)];
+        tw[threadIdx.x] = {w.x, -w.y};
     }
     __syncthreads();
-    const double bx = L.bsx, by = L.bsy, bz = L.bsz;
-    const double sx = ox - 0.5 * bx, sy = oy - 0.5 * by, sz = oz - 0.5 * bz;
+    const float bx = L.bsx, by = L.bsy, bz = L.bsz;
+    const float sx = ox - 0.5f * bx, sy = oy - 0.5f * by, sz = oz - 0.5f * bz;
     for (int t = threadIdx.x; t < M * M; t += blockDim.x) {
         const int my = t % M, mz = t / M;
-        C2<double> g[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        C2<float> g[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
         if (my != ND && mz != ND) {
-            const double ry = by * (my < ND ? my : my - M) + sy, rz = bz * (mz < ND ? mz : mz - M) + sz;
+            const float ry = by * (my < ND ? my : my - M) + sy, rz = bz * (mz < ND ? mz : mz - M) + sz;
             for (int mx = 0; mx < M; mx++) {
                 if (mx == ND || (mx | my | mz) == 0) continue;  // outside the bin lattice, the own bin
-                const double rx = bx * (mx < ND ? mx : mx - M) + sx;
-                const double r2 = rx * rx + ry * ry + rz * rz;
-                // 1/sqrt(r2): two Newton steps double the digits of the 32-bit value twice
-                double y = (double)rsqrtf((float)r2);
-                y = y * fma(-0.5 * r2 * y, y, 1.5);
-                y = y * fma(-0.5 * r2 * y, y, 1.5);
-                const double i3 = y * y * y;
-                const C2<double> w = tw[mx];
-                const double vx = rx * i3, vy = ry * i3, vz = rz * i3;
-                g[0] = {fma(vx, w.x, g[0].x), fma(vx, w.y, g[0].y)};
-                g[1] = {fma(vy, w.x, g[1].x), fma(vy, w.y, g[1].y)};
-                g[2] = {fma(vz, w.x, g[2].x), fma(vz, w.y, g[2].y)};
+                const float rx = bx * (mx < ND ? mx : mx - M) + sx;
+                const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+                const float i3 = 1.0f / (r2 * sqrtf(r2));
+                const C2<float> w = tw[mx];
+                const float vx = rx * i3, vy = ry * i3, vz = rz * i3;
+                g[0] = {fmaf(vx, w.x, g[0].x), fmaf(vx, w.y, g[0].y)};
+                g[1] = {fmaf(vy, w.x, g[1].x), fmaf(vy, w.y, g[1].y)};
+                g[2] = {fmaf(vz, w.x, g[2].x), fmaf(vz, w.y, g[2].y)};
             }
         }
         for (int c = 0; c < 3; c++) a[(c * M + mz) * ROW + my] = g[c];
     }
     __syncthreads();
     if (threadIdx.x < 3u * M) {  // along y, a row per thread
-        C2<double>* row = a + threadIdx.x * ROW;
-        C2<double> v[M];
+        C2<float>* row = a + threadIdx.x * ROW;
+        C2<float> v[M];
 #pragma unroll
         for (int k = 0; k < M; k++) v[k] = row[k];
         fft_regs<M, -1>(v);
@@ -108,13 +103,13 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
     __syncthreads();
     if (threadIdx.x < 3u * M) {  // along z, a column per thread
         const int c = threadIdx.x / M, ky = threadIdx.x % M;
-        C2<double> v[M];
+        C2<float> v[M];
 #pragma unroll
         for (int k = 0; k < M; k++) v[k] = a[(c * M + k) * ROW + ky];
         fft_regs<M, -1>(v);
         float2* out = F.G + ((((size_t)u * (ND + 1u) + kx) * 3u + c) * M) * M + ky;
 #pragma unroll
-        for (int k = 0; k < M; k++) out[k * M] = make_float2((float)v[k].x, (float)v[k].y);
+        for (int k = 0; k < M; k++) out[k * M] = make_float2(v[k].x, v[k].y);
     }
 }
 
@@ -469,11 +464,9 @@ __global__ void __launch_bounds__(PUT_THREADS) k_fft_put_batch(const FftBatch B,
 
 template <int ND>
 cudaError_t prepare_kernels() {
-    const int plan = 3 * 2 * ND * (2 * ND + 1) * 16;
     cudaError_t e = cudaFuncSetAttribute(k_fft_sum<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem(ND));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_fft_sum_batch<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem(ND));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fft_plan<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, plan);
     return e;
 }
 
@@ -540,8 +533,8 @@ cudaError_t launch_fft_plan(const DevLbm& L, const FftField& F, cudaStream_t s) 
     const cudaError_t e = L.nd == 16u ? prepare_kernels<16>() : prepare_kernels<8>();
     if (e != cudaSuccess) return e;
     const uint32_t blocks = F.ux * F.uy * F.uz * (L.nd + 1u);
-    if (L.nd == 16u) k_fft_plan<16><<<blocks, 256, 3 * 32 * 33 * 16, s>>>(L, F);
-    else k_fft_plan<8><<<blocks, 256, 3 * 16 * 17 * 16, s>>>(L, F);
+    if (L.nd == 16u) k_fft_plan<16><<<blocks, 256, 0, s>>>(L, F);
+    else k_fft_plan<8><<<blocks, 256, 0, s>>>(L, F);
     return cudaGetLastError();
 }
 
