@@ -25,6 +25,8 @@
 // over- or underflow at other places; so for sources that are infinite, or whose largest value
 // lies outside [1e-28, 1e25], `direct` is set and k_update_e_b_gated runs instead (a NaN
 // charge leaves NaN in every cell either way).
+#include <algorithm>
+
 #include "field_fft.h"
 #include "fft_regs.cuh"
 #include "ion_device.cuh"
@@ -42,7 +44,10 @@ __host__ __device__ constexpr uint32_t stage_elems(uint32_t nd) { return planes(
 __host__ __device__ constexpr uint32_t sum_smem(uint32_t nd) { return ((nd - planes(nd)) * slot_elems(nd) + stage_elems(nd)) * 8u; }
 static_assert(planes(16) * slot_elems(16) <= stage_elems(16) && planes(8) * slot_elems(8) <= stage_elems(8),
               "the last planes' slots lie inside the staging area");
-constexpr uint32_t SUM_THREADS = 128, SUM_BLOCKS = 5, SRC_THREADS = 512, PUT_THREADS = 256, PUT_X = 128;
+constexpr uint32_t SUM_THREADS = 128, SRC_THREADS = 512, PUT_THREADS = 256, PUT_X = 128;
+// k_fft_sum's blocks per SM: 96 registers at nd = 16 (with six it spills: 122 -> 155 us at 128^3),
+// half the line at nd = 8
+__host__ __device__ constexpr int sum_blocks(int nd) { return nd == 16 ? 5 : 8; }
 
 #define ION_TW(j) {(float)cos32(j), (float)sin32(j)}
 __constant__ float2 c_tw[32] = {  // exp(2 pi i j / 32)
@@ -393,7 +398,7 @@ __global__ void __launch_bounds__(SRC_THREADS) k_fft_src(const DevLbm L, const F
     fft_src<ND>(L, F, blockIdx.x);
 }
 template <int ND>
-__global__ void __launch_bounds__(SUM_THREADS, SUM_BLOCKS) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0,
+__global__ void __launch_bounds__(SUM_THREADS, sum_blocks(ND)) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0,
                                                                      const uint32_t* gate, const uint32_t blocks) {
     extern __shared__ __align__(16) float2 sum_sm[];
     if ((gate && *gate == 0u) || *F.direct) return;
@@ -443,7 +448,7 @@ __global__ void __launch_bounds__(SRC_THREADS) k_fft_src_batch(const FftBatch B)
     fft_src<ND>(L, F, block);
 }
 template <int ND>
-__global__ void __launch_bounds__(SUM_THREADS, SUM_BLOCKS) k_fft_sum_batch(const FftBatch B, const uint32_t pass) {
+__global__ void __launch_bounds__(SUM_THREADS, sum_blocks(ND)) k_fft_sum_batch(const FftBatch B, const uint32_t pass) {
     extern __shared__ __align__(16) float2 sum_sm[];
     __shared__ DevLbm L;
     __shared__ FftField F;
@@ -482,7 +487,7 @@ uint32_t launch_field_nd(const DevLbm& L, const FftField& F, const uint32_t* gat
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        resident = SUM_BLOCKS * (uint32_t)(sms > 0 ? sms : 1);
+        resident = (uint32_t)sum_blocks(ND) * (uint32_t)(sms > 0 ? sms : 1);
     }
     k_fft_src<ND><<<fft_src_blocks(L), SRC_THREADS, 0, s>>>(L, F, gate);
     for (uint32_t p = 0; p < fft_passes(L, F); p++) {
@@ -524,8 +529,8 @@ void fft_field_sizes(const DevLbm& L, FftField& F, size_t* g_bytes, size_t* s_by
     *g_bytes = (size_t)F.ux * F.uy * F.uz * (L.nd + 1u) * 3u * plane;
     *s_bytes = (L.nd + 1u) * 4u * plane;
     const size_t per = 6u * sizeof(float) * (size_t)(L.n / L.bsz);  // one in-bin z offset
-    const size_t fit = FFT_OUT_BYTES / per;
-    F.chunk = fit < 1 ? 1u : fit < L.bsz ? (uint32_t)fit : L.bsz;
+    const uint32_t fit = (uint32_t)std::min<size_t>(std::max<size_t>(FFT_OUT_BYTES / per, 1), L.bsz);
+    F.chunk = (L.bsz + (L.bsz + fit - 1u) / fit - 1u) / ((L.bsz + fit - 1u) / fit);  // passes of about equal length
     *out_bytes = per * F.chunk;
 }
 

@@ -20,7 +20,7 @@ struct FftField {
 };
 
 // bytes of the sums that are held at once (a few in-bin z offsets of a large grid)
-constexpr size_t FFT_OUT_BYTES = 256ull << 20;
+constexpr size_t FFT_OUT_BYTES = 48ull << 20;
 
 // whether a domain's FAST field runs as the convolution, and its sizes in bytes
 bool fft_field_fits(const DevLbm& L);

@@ -33,20 +33,22 @@ struct Magic {
     __device__ __forceinline__ uint32_t div(uint32_t n) const { return d > 1u ? __umulhi(n, m) : n; }
 };
 
-// LOD bins, LB_BINS neighbours along x per thread block: warps 1.. stream the bins' cells
-// (ascending cell index, LB_SLAB of each bin at a time, double-buffered) through shared memory,
-// laid out so that the 32 lanes of warp 0 -- lane = bin + LB_BINS component -- each add the
+// LOD bins, nb neighbours along x per thread block: warps 1.. stream the bins' cells
+// (ascending cell index, a slab of each bin at a time, double-buffered) through shared memory,
+// laid out so that the 4 nb lanes of warp 0 -- lane = bin + nb component -- each add the
 // next cell of their sum in one load and one addition.  A cell outside the fluid is stored as -0.0f, which leaves every float (+0
 // included) unchanged under round-to-nearest addition, so the sums need no branch.
 // Bound by memory (17 bytes a cell) for large bins and by the additions, 4 cycles each, for
 // small ones: 12.3 us at 128^3, 67 us at 256^3 (4.2 TB/s).  A block per bin with four summing
 // lanes took 21.7 and 97 us (a quarter of the bins resident at a time); lanes across the bins
 // instead of along the row 16.5 and 103 us (8 sectors of 16 bytes a load).
-constexpr uint32_t LB_THREADS = 288, LB_SLAB = 128;
-// cells 34 floats apart: the 32 lanes of a store (4 cells apart, 8 bins) write 32 different banks
-constexpr uint32_t LB_CELL = 34;
+constexpr uint32_t LB_THREADS = 288;
+// cells 4 nb + 2 floats apart: with eight bins the 32 lanes of a store (4 cells apart) write 32
+// different banks
+__device__ __forceinline__ constexpr uint32_t lb_cell(uint32_t nb) { return 4u * nb + 2u; }
+__device__ __forceinline__ constexpr uint32_t lb_slab(uint32_t nb) { return nb == 8u ? 128u : 512u; }
 struct LodSmem {
-    float v[2][LB_SLAB * LB_CELL];  // [buffer][cell][component][bin]
+    float v[2][512u * (4u * 2u + 2u)];  // [buffer][cell][component][bin]
 };
 template <uint32_t V> struct LodVec;
 template <> struct LodVec<1> { using F = float; using B = uint8_t; };
@@ -54,7 +56,7 @@ template <> struct LodVec<2> { using F = float2; using B = uchar2; };
 template <> struct LodVec<4> { using F = float4; using B = uchar4; };
 
 // cells of slab `base` of the block's bins to shared memory (warps 1..), V neighbours a thread.
-// Lanes run along the bins' common x-row (bins of up to LB_SLAB cells an edge), so a warp's
+// Lanes run along the bins' common x-row (bins of up to a slab's cells an edge), so a warp's
 // loads are contiguous.
 template <uint32_t V>
 __device__ __forceinline__ void lod_load(const DevLbm& L, float* const buf, uint32_t x0, uint32_t y0, uint32_t z0,
@@ -94,23 +96,24 @@ __device__ __forceinline__ void lod_load(const DevLbm& L, float* const buf, uint
 #pragma unroll
         for (uint32_t u = 0; u < V; u++) {
             const bool fluid = (reinterpret_cast<const uint8_t*>(&f)[u] & F_BO) != F_S;
-            float* const o = buf + (j + u) * LB_CELL + b;
+            float* const o = buf + (j + u) * lb_cell(nb) + b;
 #pragma unroll
-            for (uint32_t c = 0; c < 4; c++) o[c * LB_BINS] = fluid ? reinterpret_cast<const float*>(&a[c])[u] : -0.0f;
+            for (uint32_t c = 0; c < 4; c++) o[c * nb] = fluid ? reinterpret_cast<const float*>(&a[c])[u] : -0.0f;
         }
     }
 }
 
 __device__ __forceinline__ void lod_bins_block(const DevLbm& L, const uint32_t block, LodSmem& sm) {
-    const uint32_t nd = L.nd, groups = (nd + LB_BINS - 1u) / LB_BINS, nb = min(nd, LB_BINS);
-    const uint32_t bx0 = block % groups * LB_BINS, by = block / groups % nd, bz = block / (groups * nd);
+    const uint32_t nd = L.nd, nb = lod_bins_per_block(nd), groups = nd / nb;
+    const uint32_t bx0 = block % groups * nb, by = block / groups % nd, bz = block / (groups * nd);
     if (block == 0u)  // bins of the lower LOD levels stay zero (single domain)
         for (uint32_t i = L.n_bins * 4u + threadIdx.x; i < L.n_lod_own * 4u; i += LB_THREADS) L.qu_lod[i] = 0.0f;
     const uint32_t cells = L.bsx * L.bsy * L.bsz;
-    const bool rows = L.bsx <= LB_SLAB;  // whole rows a slab
+    const uint32_t room = lb_slab(nb);
+    const bool rows = L.bsx <= room;  // whole rows a slab
     // neighbours a thread; rows of n bins, so a multiple of V cells keeps every access aligned
     const uint32_t vec = !rows ? 1u : L.bsx % 4u == 0u ? 4u : L.bsx % 2u == 0u ? 2u : 1u;
-    const uint32_t slab = rows ? LB_SLAB / L.bsx * L.bsx : LB_SLAB, nslabs = (cells + slab - 1u) / slab;
+    const uint32_t slab = rows ? room / L.bsx * L.bsx : room, nslabs = (cells + slab - 1u) / slab;
     const Magic mx(L.bsx), mxy(L.bsx * L.bsy), mq(L.bsx / vec);
     const bool magic = (uint64_t)cells * (L.bsx * L.bsy) < (1ull << 32);  // Magic's bound (bins of <= ~2^16 cells)
     auto load = [&](uint32_t k) {
@@ -129,21 +132,22 @@ __device__ __forceinline__ void lod_bins_block(const DevLbm& L, const uint32_t b
             if (k + 1u < nslabs) load(k + 1u);
         } else {
             const uint32_t cnt = min(slab, cells - k * slab);
-            const float* v = sm.v[k & 1u] + threadIdx.x;
+            const float* v = sm.v[k & 1u] + (threadIdx.x < 4u * nb ? threadIdx.x : 0u);
+            const uint32_t cell = lb_cell(nb);
             uint32_t i = 0;
             for (; i + 16u <= cnt; i += 16u) {  // loads first, then the dependent additions
                 float a[16];
 #pragma unroll
-                for (uint32_t u = 0; u < 16u; u++) a[u] = v[(i + u) * LB_CELL];
+                for (uint32_t u = 0; u < 16u; u++) a[u] = v[(i + u) * cell];
 #pragma unroll
                 for (uint32_t u = 0; u < 16u; u++) acc = acc + a[u];
             }
-            for (; i < cnt; i++) acc = acc + v[i * LB_CELL];
+            for (; i < cnt; i++) acc = acc + v[i * cell];
         }
         __syncthreads();
     }
-    const uint32_t bin = threadIdx.x % LB_BINS, c = threadIdx.x / LB_BINS;
-    if (threadIdx.x < 32u && bin < nb) L.qu_lod[(size_t)(bx0 + bin + (by + bz * nd) * nd) * 4u + c] = acc;
+    const uint32_t bin = threadIdx.x % nb, c = threadIdx.x / nb;
+    if (threadIdx.x < 4u * nb) L.qu_lod[(size_t)(bx0 + bin + (by + bz * nd) * nd) * 4u + c] = acc;
 }
 
 static __global__ void __launch_bounds__(LB_THREADS) k_lod_bins(const DevLbm L) {
