@@ -33,10 +33,10 @@ Metric: MLUPs/s = cells * steps / seconds / 1e6.
   e2e         : the same job through the C ABI with host buffers: upload of
                 the inputs from pinned memory, initialize, K steps (CUDA graph),
                 download of the result fields, inside the timed region.
-  roofline    : the dominant kernel -- the E/B update, FP32-bound -- against
-                the measured FP32 FMA peak (ion_probe_fp32_peak); the plain
-                workloads' dominant kernel is stream_collide against the
-                measured HBM bandwidth (MEASURED_PEAKS.json).
+  roofline    : the dominant kernel -- the E/B update against the measured
+                FP32 FMA peak (ion_probe_fp32_peak), or stream_collide against
+                the measured HBM bandwidth (MEASURED_PEAKS.json); the other one
+                is in roofline_field or roofline_stencil.
   cpu_baseline: the reference's kernels compiled for the host (or the C
                 restatement when the reference copy is absent), all host cores,
                 a bounded sample of the same workload.
@@ -65,6 +65,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 FLOP_PER_INTERACTION = 34  # one source's E and B: 34 FLOP + 1 sqrt (sim_kernels.cl:950-954)
+FLOP_PER_TABLE_TERM = 21   # the same with R/|R|^3 from the table (k_update_e_b_table)
 # kernel-time results of one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum per launch);
 # the summaries with the commands that produced them are in profiles/
 # (rings384: the rings192 capture of k_sc_rows_ws scaled by the cell count, (384/192)^3; every
@@ -202,6 +203,23 @@ def field_interactions(cfg: dict, flags: np.ndarray) -> int:
     own = bx + (by + bz * nd) * nd
     fluid = int(fl.sum())
     return fluid * (nd ** 3 - first) - int((fl & (own >= first)).sum())
+
+
+def laid_out_field(cfg: dict) -> bool:
+    """Whether the exact field runs in its laid-out form (a convolution with FAST, a table with BITWISE)."""
+    D = int(cfg["mhd_lod_depth"])
+    return D in (3, 4) and all(cfg[k] // (1 << (1 << D)) <= 1 and cfg[k] < 65536 for k in ("n_x", "n_y", "n_z"))
+
+
+def convolution_flops(cfg: dict) -> int:
+    """FLOPs of the FAST field's convolution: per in-bin offset the products of spectra (8 a value for E, 14
+    for B) and six inverse transforms, the usual 5 M log2 M a complex line of M = 2 nd points, half of that
+    a real one."""
+    nd = 1 << int(cfg["mhd_lod_depth"])
+    M = 2 * nd
+    offsets = cfg["n_x"] * cfg["n_y"] * cfg["n_z"] // nd ** 3
+    lines = nd * (M + nd) + nd * nd / 2
+    return int(offsets * (6 * lines * 5 * M * (M.bit_length() - 1) + 3 * (8 + 14) * nd * M * M))
 
 
 # ---------------------------------------------------------------------------
@@ -645,19 +663,32 @@ def main():
         sur.update(checks_in_run=st["checks"], fallbacks_in_run=st["fallbacks"],
                    nonfinite_checks_in_run=st["nonfinite"])
     elif mhd:
-        inter = sum(field_interactions(c["config"], d.read("flags")) for c, d in zip(cases, doms))
+        laid = [laid_out_field(c["config"]) for c in cases]
+        conv = a.field_mode != "bitwise"
+        inter = [field_interactions(c["config"], d.read("flags")) for c, d in zip(cases, doms)]
+        # a batch's BITWISE domains take the direct sum
+        per_term = FLOP_PER_TABLE_TERM if not conv and batch is None else FLOP_PER_INTERACTION
+        flop = sum((convolution_flops(c["config"]) if conv else n * per_term) if l and (conv or batch is None)
+                   else n * FLOP_PER_INTERACTION for c, n, l in zip(cases, inter, laid))
+        form = ("k_fft_src + k_fft_sum + k_fft_put" if conv else "k_update_e_b_table") if all(laid) else \
+            "k_update_e_b_fast" if conv else "k_update_e_b_exact"
         if batch is None:
             avg = eb_ms / max(eb_n, 1)
-            kname = "k_update_e_b_exact" if a.field_mode == "bitwise" else "k_update_e_b_fast"
+            kname = form
         else:
             avg = ms / a.steps
             kname = (f"k_batch_stream{'_rows' if all(c['config']['n_x'] % 16 == 0 and c['config']['n_x'] <= 96 for c in cases) else ''}"
-                     f" + k_batch_field<{a.field_mode}> (whole step; FLOPs of its E/B phase)")
-        tflops = inter * FLOP_PER_INTERACTION / (avg * 1e-3) / 1e12
-        roofline = {"bound": "fp32", "achieved": tflops, "peak": tf.value, "unit": "TFLOP/s",
-                    "frac": tflops / tf.value, "traffic": NCU_TRAFFIC.get((a.workload, kname)), "kernel": kname,
-                    "flop_per_launch": inter * FLOP_PER_INTERACTION, "interactions_per_launch": inter,
-                    "avg_launch_ms": avg, "peak_source": "measured FP32 FMA throughput (ion_probe_fp32_peak)"}
+                     f" + k_batch_lod + {form if conv and all(laid) else 'k_batch_field<' + a.field_mode + '>'}"
+                     " (whole step; FLOPs of its E/B phase)")
+        tflops = flop / (avg * 1e-3) / 1e12
+        roof_field = {"bound": "fp32", "achieved": tflops, "peak": tf.value, "unit": "TFLOP/s",
+                      "frac": tflops / tf.value, "traffic": NCU_TRAFFIC.get((a.workload, kname)), "kernel": kname,
+                      "flop_per_launch": flop, "interactions_per_launch": sum(inter),
+                      "avg_launch_ms": avg, "peak_source": "measured FP32 FMA throughput (ion_probe_fp32_peak)"}
+        roofline = roof_field
+        if batch is None and sc_ms > eb_ms:
+            roofline = roof_stencil
+            extra["roofline_field"] = roof_field
     if batch is not None:
         extra["autotuner"] = {"chosen": batch.chosen(), "trials": batch.tuning()}
     if sur is not None:
