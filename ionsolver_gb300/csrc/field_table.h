@@ -8,10 +8,12 @@ namespace ion {
 
 struct DevLbm;
 
-// R/|R|^3 of every distance |2 R| between a cell and a bin centre: [z][y][x], (x, y, z, 0)
+// R/|R|^3 between cells and bin centres, (x, y, z, 0): of every distance |2 R|, [z][y][x]; or, in
+// bins, of every difference D of two bins and in-bin offset, [Dz][Dy][Dx][offset]
 struct FieldTable {
     float4* T = nullptr;
     uint32_t tx = 0, ty = 0, tz = 0;
+    bool in_bins = false;
 };
 
 bool field_table_fits(const DevLbm& L);
