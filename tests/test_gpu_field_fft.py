@@ -77,7 +77,7 @@ def _cells(shape, seed=1):
                                          ((48, 16, 80), 4), ((144, 16, 16), 4), ((136, 8, 16), 3), ((256, 256, 256), 4)])
 def test_convolution_against_float64(shape, depth):
     """Bins of 1, 2, 3, 5, 7, 9, 16 and 17 cells an edge; rows of one and of two tiles; the sums
-    of 256^3 go in two passes."""
+    of 256^3 go in several passes."""
     lod = _bins(depth, 5)
     e, b, k = _field(shape, depth, lod)
     cells = _cells(shape)
