@@ -1,7 +1,7 @@
 // setup_kernels.cu -- geometry and static-field kernels, FP64 reductions.
 //
-//   voxelize  : IonSolver src/kernels/sim_kernels.cl:1150-1231 (one warp
-//               per bounding-box column, Moeller-Trumbore in both ray
+//   voxelize  : IonSolver src/kernels/sim_kernels.cl:1150-1231 (one thread
+//               or warp per bounding-box column, Moeller-Trumbore in both ray
 //               directions, 16-bit hit distances, parity with correction).
 //   psi / B   : sim_kernels.cl:1234-1276.  The reference loops over all N
 //               cells for each of the (N+2)^3 potential points and tests the
@@ -10,6 +10,9 @@
 //               work) and staged through shared memory.
 //   static E  : sim_kernels.cl:1278-1300, same compaction over charged cells.
 //   FP64 sums : deterministic two-pass tree reductions of decoded DDFs.
+#include <algorithm>
+#include <cmath>
+
 #include "ion_device.cuh"
 #include "ion_launch.h"
 #include "reduce_f64.cuh"
@@ -25,12 +28,81 @@ __device__ __forceinline__ V3 vcross(V3 a, V3 b) { return {a.y * b.z - a.z * b.y
 __device__ __forceinline__ float vdot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ int iclamp(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
-// A warp per column: the lanes take the triangles side by side and file their hits in triangle
-// order (a thread per column left most SMs with a few warps, each waiting on one triangle's
-// divide after another: 150 us for 128 triangles at 128^3).
-constexpr uint32_t VOX_WARPS = 4, VOX_HITS = 64;
+constexpr uint32_t VOX_WARPS = 4, VOX_THREADS = 128, VOX_HITS = 64;
 
-__global__ void __launch_bounds__(VOX_WARPS * 32) k_voxelize(const DevLbm L, VoxArgs A) {
+// a thread per column
+__global__ void __launch_bounds__(VOX_THREADS) k_voxelize(const DevLbm L, VoxArgs A) {
+    const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= A.columns) return;
+    const int nx = (int)L.nx, ny = (int)L.ny, nz = (int)L.nz;
+    const int dir = A.direction;
+    uint32_t c[3];
+    if (dir == 0) { c[0] = (uint32_t)iclamp((int)A.x0, 0, nx - 1); c[1] = a % L.ny; c[2] = a / L.ny; }
+    else if (dir == 1) { c[0] = a / L.nz; c[1] = (uint32_t)iclamp((int)A.y0, 0, ny - 1); c[2] = a % L.nz; }
+    else { c[0] = a % L.nx; c[1] = a / L.nx; c[2] = (uint32_t)iclamp((int)A.z0, 0, nz - 1); }
+    const V3 org = {(((float)c[0] + 0.5f) - 0.5f * (float)nx) + (0.5f * (float)nx - 0.5f),
+                    (((float)c[1] + 0.5f) - 0.5f * (float)ny) + (0.5f * (float)ny - 0.5f),
+                    (((float)c[2] + 0.5f) - 0.5f * (float)nz) + (0.5f * (float)nz - 0.5f)};
+    bool outside;
+    if (dir == 0) outside = org.y < A.y0 || org.z < A.z0 || org.y >= A.y1 || org.z >= A.z1;
+    else if (dir == 1) outside = org.x < A.x0 || org.z < A.z0 || org.x >= A.x1 || org.z >= A.z1;
+    else outside = org.x < A.x0 || org.y < A.y0 || org.x >= A.x1 || org.y >= A.y1;
+    if (outside) return;
+    const V3 rdir = {(float)(dir == 0), (float)(dir == 1), (float)(dir == 2)};
+    uint16_t dist[64];
+    for (int i = 0; i < 64; i++) dist[i] = 0;
+    uint32_t hits = 0, back = 0;
+    for (uint32_t i = 0; i < A.ntri; i++) {
+        const V3 P0 = {A.p0[3 * i], A.p0[3 * i + 1], A.p0[3 * i + 2]};
+        const V3 P1 = {A.p1[3 * i], A.p1[3 * i + 1], A.p1[3 * i + 2]};
+        const V3 P2 = {A.p2[3 * i], A.p2[3 * i + 1], A.p2[3 * i + 2]};
+        const V3 e1 = vsub(P1, P0), e2 = vsub(P2, P0), s0 = vsub(org, P0);
+        const V3 pv = vcross(rdir, e2), qv = vcross(s0, e1);
+        const float inv = 1.0f / vdot(e1, pv);
+        const float su = inv * vdot(s0, pv), sv = inv * vdot(rdir, qv), sd = inv * vdot(e2, qv);
+        if (su >= 0.0f && su < 1.0f && sv >= 0.0f && su + sv < 1.0f) {
+            if (sd > 0.0f) {
+                if (hits < 64u && sd < 65536.0f) dist[hits] = (uint16_t)sd;
+                hits++;
+            } else {
+                back++;
+            }
+        }
+    }
+    const uint32_t ns = hits < 64u ? hits : 64u;
+    for (uint32_t i = 1; i < ns; i++) {
+        const uint16_t key = dist[i];
+        int k = (int)i - 1;
+        while (k >= 0 && dist[k] > key) { dist[k + 1] = dist[k]; k--; }
+        dist[k + 1] = key;
+    }
+    bool inside = (hits % 2u) && (back % 2u);
+    uint32_t next = (hits % 2u) != (back % 2u);
+    const uint32_t h0 = c[dir];
+    const uint32_t hmax = dir == 0 ? (uint32_t)iclamp((int)A.x1, 0, nx) : dir == 1 ? (uint32_t)iclamp((int)A.y1, 0, ny)
+                                                                                  : (uint32_t)iclamp((int)A.z1, 0, nz);
+    const uint32_t last = hits - 1u < 63u ? hits - 1u : 63u;
+    const uint32_t hmesh = h0 + (uint32_t)dist[last];
+    const size_t N = L.n;
+    for (uint32_t hh = h0; hh < hmax; hh++) {
+        while (next < hits && hh > h0 + (uint32_t)dist[next < 63u ? next : 63u]) { inside = !inside; next++; }
+        inside = inside && (next < hits && hh < hmesh);
+        uint32_t cc[3] = {c[0], c[1], c[2]};
+        cc[dir] = hh;
+        const uint32_t n = cc[0] + (cc[1] + cc[2] * L.ny) * L.nx;
+        if (inside) {
+            L.flags[n] = (uint8_t)((L.flags[n] & ~F_BO) | A.flag);
+            if (L.ext_mhd) {
+                if (A.flag & F_M) { L.b_dyn[n] = A.mx; L.b_dyn[N + n] = A.my; L.b_dyn[2 * N + n] = A.mz; }
+                else if ((A.flag & F_F) || (A.flag & F_C)) L.b_dyn[n] = A.mx;
+            }
+        }
+    }
+}
+
+// a warp per column: the lanes take the triangles side by side and file their hits in triangle
+// order
+__global__ void __launch_bounds__(VOX_WARPS * 32) k_voxelize_warp(const DevLbm L, VoxArgs A) {
     __shared__ uint16_t s_dist[VOX_WARPS][VOX_HITS], s_sorted[VOX_WARPS][VOX_HITS];
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t a = blockIdx.x * VOX_WARPS + wid;
@@ -113,8 +185,25 @@ __global__ void __launch_bounds__(VOX_WARPS * 32) k_voxelize(const DevLbm L, Vox
     }
 }
 
+// A thread per column leaves most SMs with a few warps, each waiting on one triangle's divide
+// after another, until there are many columns; a warp per column repeats the walk in every lane.
+// us a call, thread / warp: 64^3 with 48 triangles 39 / 20, 128^3 with 224 on 14,209 columns
+// 110 / 77, 192^3 with 12 on 10,000 columns 37 / 52, 512^3 with 12 on 216,039 columns 299 /
+// 3,440 and with 3,968 3,766 / 5,199.  The forms cross near 9,000 columns at 12 triangles,
+// 22,000 at 224, 45,000 at 960 and 85,000 at 3,968: a square root of the triangles.
+static bool voxelize_by_warps(uint64_t columns, uint32_t ntri) {
+    return columns <= 8192u || columns * columns <= 1800000ull * ntri;
+}
+
 void launch_voxelize(const DevLbm& L, const VoxArgs& A, cudaStream_t s) {
-    k_voxelize<<<grid_for(A.columns, VOX_WARPS), VOX_WARPS * 32, 0, s>>>(L, A);
+    const uint32_t edge[3] = {L.nx, L.ny, L.nz};
+    const float lo[3] = {A.x0, A.y0, A.z0}, hi[3] = {A.x1, A.y1, A.z1};
+    uint64_t columns = 1;  // inside the mesh's bounds
+    for (int a = 0; a < 3; a++)
+        if (a != A.direction)
+            columns *= (uint64_t)std::max(0.0, std::min((double)edge[a], std::ceil((double)hi[a])) - std::max(0.0, std::ceil((double)lo[a])));
+    if (voxelize_by_warps(columns, A.ntri)) k_voxelize_warp<<<grid_for(A.columns, VOX_WARPS), VOX_WARPS * 32, 0, s>>>(L, A);
+    else k_voxelize<<<grid_for(A.columns, VOX_THREADS), VOX_THREADS, 0, s>>>(L, A);
 }
 
 // ---------------------------------------------------------------------------

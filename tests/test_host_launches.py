@@ -1,0 +1,25 @@
+"""What the host code launches and keeps, on a CUDA runtime without a device (_fake_cuda.py)."""
+import numpy as np
+import pytest
+
+import ionsolver_gb300 as I
+from tests._fake_cuda import fake  # noqa: F401
+
+
+def _box(lo, hi):
+    v = np.array([[x, y, z] for z in (lo, hi) for y in (lo, hi) for x in (lo, hi)], np.float32)
+    f = np.array([[0, 2, 1], [1, 2, 3], [4, 5, 6], [5, 7, 6], [0, 1, 4], [1, 5, 4], [2, 6, 3], [3, 6, 7], [0, 4, 2], [2, 4, 6],
+                  [1, 3, 5], [3, 7, 5]])
+    return tuple(np.ascontiguousarray(v[f[:, k]]) for k in range(3))
+
+
+@pytest.mark.parametrize("n,form", [(40, "k_voxelize_warp"), (91, "k_voxelize_warp"), (96, "k_voxelizeE"), (200, "k_voxelizeE")])
+def test_voxeliser_form_by_columns(fake, n, form):  # noqa: F811
+    """Twelve triangles: a warp per column up to 8192 columns inside the mesh's bounds, then a
+    thread (a warp each took 3,440 us where a thread each takes 299)."""
+    lbm = I.Lbm(I.LbmConfig(velocity_set=2, float_type=0, n_x=n, n_y=n, n_z=n, nu=1 / 30))
+    mesh = lbm.add_mesh(*_box(2.5, n - 2.5))
+    fake.lib.fake_clear()
+    lbm.voxelise_mesh(mesh, I.ModelType.Solid())
+    assert fake.kernel("k_voxelize")["name"].startswith(form)
+    lbm.close()
