@@ -20,11 +20,14 @@
 //   k_fft_put   the sums to the cells, x-rows at a time: E_stat + KE e, B_stat + KMU b.
 //
 // Rounding: the field's error against 64 bits is 1.6e-7 to 2.2e-7 of its norm from 8^3 to 256^3
-// cells (the direct 32-bit sums: 2.6e-7 to 8.6e-7), spread evenly over the lattice.  An infinite bin would leave NaN
-// where the direct sum keeps the sign, and sums near the ends of the exponent range would
-// over- or underflow at other places; so for sources that are infinite, or whose largest value
-// lies outside [1e-28, 1e25], `direct` is set and k_update_e_b_gated runs instead (a NaN
-// charge leaves NaN in every cell either way).
+// cells (the direct 32-bit sums: 2.6e-7 to 8.6e-7).  The transforms spread it evenly over the
+// lattice, where the direct sum's is relative to a cell's own terms: with the charge in a few
+// bins the weakest cells would be up to 1e-4 of their field off (one bin 1.3e-5, the direct sum
+// 4.5e-7).  So k_fft_src compares the two (see `concentrated`), and where the convolution's error would
+// be the larger one, `direct` is set and k_update_e_b_gated runs instead.  It also runs for
+// sources that are infinite, where the convolution would leave NaN and the direct sum keeps the
+// sign, or whose largest value lies outside [1e-28, 1e25], where sums could over- or underflow (a
+// NaN charge leaves NaN in every cell either way).
 #include <algorithm>
 
 #include "field_fft.h"
@@ -121,41 +124,101 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
 // ---------------------------------------------------------------------------
 // spectra of the sources: block = component + 4 kx
 // ---------------------------------------------------------------------------
+
+// Whether a component w_J of the sources (s, scaled by a power of two to below 1) is too
+// concentrated for the convolution.  Its error is about the same in every cell, of the size
+// |w| kappa: |w|^2 = sum w_J^2, kappa^2 = the mean of 1/|R|^4 over the padded lattice.  The direct
+// sum's is relative to the cell's own sum of |w_J|/|R|^2, least far from the sources: estimated over
+// 4^3 groups of bins, each at the distance of its centre and half a group an axis (within 15% of
+// the cells' least sum on boxes of even edges).  Both errors against 64 bits, per cell relative
+// to that sum, root mean square, 2,800 distributions in 22 box shapes: with the least sum above
+// 4 |w| kappa at nd = 16 and 2.75 |w| kappa at nd = 8 the convolution's is at most 0.88 and 1.08 of the
+// direct sum's; at half the line of nd = 16 it reaches 2.  Charges and currents spread over the box, as in
+// all the configurations, lie at 5 to 10 and at 3 to 5 (one charged bin: 0.1).  Bins twice as
+// long as wide lie lower, eight times as long below the line.  F.spread holds the square of the
+// line times kappa.  (All of it in fixed order: a batch decides as its domains do alone.)
+template <int ND>
+__device__ __forceinline__ bool concentrated(const DevLbm& L, const FftField& F, const float* s, const float scale) {
+    constexpr uint32_t G = ND / 4;  // bins a group and axis
+    __shared__ float s_sum[64], s_sq[64], s_inv[64];
+    __shared__ uint32_t s_min;
+    const uint32_t g = threadIdx.x / 8u, sub = threadIdx.x % 8u;  // eight lanes a group
+    static_assert(SRC_THREADS == 512u, "64 groups of eight lanes");
+    float sum = 0.0f, sq = 0.0f;
+#pragma unroll
+    for (uint32_t k = sub; k < G * G * G; k += 8u) {
+        const uint32_t x = g % 4u * G + k % G, y = g / 4u % 4u * G + k / G % G, z = g / 16u * G + k / (G * G);
+        const float v = fabsf(s[(z * ND + y) * (ND + 1) + x]) * scale;
+        sum = sum + v;
+        sq = fmaf(v, v, sq);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        sum = sum + __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        sq = sq + __shfl_xor_sync(0xFFFFFFFFu, sq, o);
+    }
+    if (sub == 0u) { s_sum[g] = sum; s_sq[g] = sq; }
+    if (threadIdx.x < 64u) {  // 1/|R|^2 of groups (x, y, z) apart
+        const float rx = ((threadIdx.x % 4u) + 0.5f) * (float)(G * L.bsx), ry = ((threadIdx.x / 4u % 4u) + 0.5f) * (float)(G * L.bsy),
+                    rz = ((threadIdx.x / 16u) + 0.5f) * (float)(G * L.bsz);
+        s_inv[threadIdx.x] = 1.0f / fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+    }
+    if (threadIdx.x == 0u) s_min = 0x7F800000u;
+    __syncthreads();
+    float a = 0.0f, q = 0.0f;
+#pragma unroll
+    for (uint32_t j = sub; j < 64u; j += 8u) {
+        const uint32_t dx = abs((int)(j % 4u) - (int)(g % 4u)), dy = abs((int)(j / 4u % 4u) - (int)(g / 4u % 4u)),
+                       dz = abs((int)(j / 16u) - (int)(g / 16u));
+        a = fmaf(s_sum[j], s_inv[dx + 4u * dy + 16u * dz], a);
+        q = q + s_sq[j];
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        a = a + __shfl_xor_sync(0xFFFFFFFFu, a, o);
+        q = q + __shfl_xor_sync(0xFFFFFFFFu, q, o);
+    }
+    if (sub == 0u) atomicMin(&s_min, __float_as_uint(a));  // (in any order; a >= 0)
+    __syncthreads();
+    const float least = __uint_as_float(s_min);
+    return least * least < F.spread * q;
+}
+
 template <int ND>
 __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, const uint32_t block) {
     constexpr uint32_t M = 2u * ND, NB = ND * ND * ND;
     __shared__ float s[ND * ND * (ND + 1)];  // [z][y][x], rows of ND + 1
     __shared__ float2 a[ND][ND], b[ND][M], tw[M];
-    __shared__ uint32_t s_max[4], s_bad;
+    __shared__ uint32_t s_max[2];
     const uint32_t c = block % 4u, kx = block / 4u;
     const uint32_t first = L.first_src, last = min(L.n_lod_own, L.n_bins);
-    if (threadIdx.x < 4u) s_max[threadIdx.x] = 0u;
-    if (threadIdx.x == 0u) s_bad = 0u;
+    if (threadIdx.x < 2u) s_max[threadIdx.x] = 0u;
     if (threadIdx.x < M) tw[threadIdx.x] = c_tw[threadIdx.x * (32u / M)];  // the lanes index it apart
     __syncthreads();
-    uint32_t m[4] = {0u, 0u, 0u, 0u};
+    uint32_t m[2] = {0u, 0u};  // the largest charge and value of the component: NaN > Inf > finite
 #pragma unroll
     for (uint32_t d = threadIdx.x; d < NB; d += SRC_THREADS) {
         const float4 v = d >= first && d < last ? reinterpret_cast<const float4*>(L.qu_lod)[d] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float w[4] = {v.x, v.x * v.y, v.x * v.z, v.x * v.w};
-        s[d / ND * (ND + 1) + d % ND] = c == 0u ? w[0] : c == 1u ? w[1] : c == 2u ? w[2] : w[3];
-        if (block == 0u) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) m[k] = max(m[k], __float_as_uint(w[k]) & 0x7FFFFFFFu);  // NaN > Inf > finite
-        }
+        const float w = c == 0u ? v.x : c == 1u ? v.x * v.y : c == 2u ? v.x * v.z : v.x * v.w;
+        s[d / ND * (ND + 1) + d % ND] = w;
+        m[0] = max(m[0], __float_as_uint(v.x) & 0x7FFFFFFFu);
+        m[1] = max(m[1], __float_as_uint(w) & 0x7FFFFFFFu);
     }
-    if (block == 0u) {
+    if (kx == 0u) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < 2; k++) {
             const uint32_t v = __reduce_max_sync(0xFFFFFFFFu, m[k]);
             if ((threadIdx.x & 31u) == 0u) atomicMax(&s_max[k], v);
         }
     }
     __syncthreads();
-    if (block == 0u && threadIdx.x < 4u) {
-        const uint32_t v = s_max[threadIdx.x];
-        // a NaN charge makes every cell's E and B NaN either way
-        if (s_max[0] <= 0x7F800000u && v != 0u && !(v >= __float_as_uint(1e-28f) && v <= __float_as_uint(1e25f))) atomicExch(&s_bad, 1u);
+    if (kx == 0u) {  // the component's block decides for it
+        const uint32_t v = s_max[1];
+        bool bad = false;
+        if (s_max[0] <= 0x7F800000u && v != 0u)  // a NaN charge makes every cell's E and B NaN either way
+            bad = !(v >= __float_as_uint(1e-28f) && v <= __float_as_uint(1e25f)) ||
+                  concentrated<ND>(L, F, s, __uint_as_float(0x7E800000u - (v & 0x7F800000u)));
+        if (threadIdx.x == 0u) F.direct[c] = bad;
     }
     // along x at this kx
     for (uint32_t t = threadIdx.x; t < ND * ND; t += SRC_THREADS) {
@@ -170,7 +233,6 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
         a[t / ND][t % ND] = acc;
     }
     __syncthreads();
-    if (block == 0u && threadIdx.x == 0u) *F.direct = s_bad;
     // along y, then along z
     for (uint32_t t = threadIdx.x; t < ND * M; t += SRC_THREADS) {
         const uint32_t ky = t % M, z = t / M;
@@ -402,7 +464,7 @@ template <int ND>
 __global__ void __launch_bounds__(SUM_THREADS, sum_blocks(ND)) k_fft_sum(const DevLbm L, const FftField F, const uint32_t oz0,
                                                                      const uint32_t* gate, const uint32_t blocks) {
     extern __shared__ __align__(16) float2 sum_sm[];
-    if ((gate && *gate == 0u) || *F.direct) return;
+    if ((gate && *gate == 0u) || any_of(F.direct)) return;
     for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
         fft_sum<ND>(L, F, b, oz0, sum_sm);
         if (gate) __syncthreads();
@@ -411,7 +473,7 @@ __global__ void __launch_bounds__(SUM_THREADS, sum_blocks(ND)) k_fft_sum(const D
 template <int ND>
 __global__ void __launch_bounds__(PUT_THREADS) k_fft_put(const DevLbm L, const FftField F, const uint32_t oz0,
                                                          const uint32_t* gate, const uint32_t blocks) {
-    if ((gate && *gate == 0u) || *F.direct) return;
+    if ((gate && *gate == 0u) || any_of(F.direct)) return;
     for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
         fft_put<ND>(L, F, b, oz0);
         if (gate) __syncthreads();
@@ -455,7 +517,7 @@ __global__ void __launch_bounds__(SUM_THREADS, sum_blocks(ND)) k_fft_sum_batch(c
     __shared__ FftField F;
     __shared__ uint32_t e;
     const uint32_t block = batch_entry(B, B.sum_off, L, F, e);
-    if (*F.direct) return;
+    if (any_of(F.direct)) return;
     fft_sum<ND>(L, F, block, pass * F.chunk, sum_sm);
 }
 template <int ND>
@@ -464,7 +526,7 @@ __global__ void __launch_bounds__(PUT_THREADS) k_fft_put_batch(const FftBatch B,
     __shared__ FftField F;
     __shared__ uint32_t e;
     const uint32_t block = batch_entry(B, B.put_off, L, F, e);
-    if (*F.direct) return;
+    if (any_of(F.direct)) return;
     fft_put<ND>(L, F, block, pass * F.chunk);
 }
 
@@ -533,6 +595,27 @@ void fft_field_sizes(const DevLbm& L, FftField& F, size_t* g_bytes, size_t* s_by
     const uint32_t fit = (uint32_t)std::min<size_t>(std::max<size_t>(FFT_OUT_BYTES / per, 1), L.bsz);
     F.chunk = (L.bsz + (L.bsz + fit - 1u) / fit - 1u) / ((L.bsz + fit - 1u) / fit);  // passes of about equal length
     *out_bytes = per * F.chunk;
+}
+
+// The line of `concentrated`: (4 kappa)^2 or (2.75 kappa)^2.  kappa^2 is taken over the bins up to
+// four apart (1/|R|^4 falls fast) and up to four offsets an axis.
+float fft_field_spread(const DevLbm& L) {
+    const uint32_t bs[3] = {L.bsx, L.bsy, L.bsz};
+    double r2[3][4][9], sum = 0.0;  // squares along an axis, [offset][difference of the bins]
+    for (int a = 0; a < 3; a++)
+        for (uint32_t i = 0; i < 4; i++)
+            for (int d = -4; d <= 4; d++) {
+                const double r = (double)bs[a] * d + (2u * i + 1u) * bs[a] / 8u - 0.5 * bs[a];
+                r2[a][i][d + 4] = r * r;
+            }
+    for (int o = 0; o < 64; o++)
+        for (int d = 0; d < 729; d++) {
+            if (d == 364) continue;  // the own bin
+            const double r = r2[0][o % 4][d % 9] + r2[1][o / 4 % 4][d / 9 % 9] + r2[2][o / 16][d / 81];
+            sum += 1.0 / (r * r);
+        }
+    const double M = 2.0 * L.nd, line = L.nd == 16u ? 4.0 : 2.75;
+    return (float)(line * line * sum / (64.0 * M * M * M));
 }
 
 cudaError_t launch_fft_plan(const DevLbm& L, const FftField& F, cudaStream_t s) {

@@ -593,13 +593,13 @@ __device__ __forceinline__ bool eb_tile(const DevLbm& L, const uint32_t brick, c
     return true;
 }
 
-// The exact update, run only when *gate != 0 (and, where given, *gate2 != 0: the surrogate's
-// fallback decision, sources that the convolution does not take): resident blocks walk the
+// The direct sums, run only when *gate != 0 (where given: the surrogate's fallback decision) and a
+// word of direct is set (where given: sources that the convolution does not take): resident blocks walk the
 // bricks, so that a closed gate costs one wave of blocks that leave at once (a block per brick:
 // 7.3 us at 192^3)
 static __global__ void __launch_bounds__(256, 2) k_update_e_b_gated(const DevLbm L, uint32_t* err, const uint32_t* gate,
-                                                                    const uint32_t* gate2, const uint32_t bricks) {
-    if (*gate == 0u || (gate2 && *gate2 == 0u)) return;
+                                                                    const uint32_t* direct, const uint32_t bricks) {
+    if ((gate && *gate == 0u) || (direct && !any_of(direct))) return;
     __shared__ __align__(16) EbSmem<true> sm;
     eb_init(sm);
     uint32_t uses[2] = {0u, 0u};

@@ -274,7 +274,7 @@ int setup_field(ion_lbm* h) {
     // (SURROGATE handles fall back to the FAST field)
     if (h->fft.G || h->cfg.field_mode == ION_FIELD_BITWISE || !fft_field_fits(h->L)) return ION_OK;
     FftField F;
-    size_t bytes[4] = {0, 0, 0, 4};
+    size_t bytes[4] = {0, 0, 0, 16};
     fft_field_sizes(h->L, F, &bytes[0], &bytes[1], &bytes[2]);
     void** const ptr[4] = {(void**)&F.G, (void**)&F.S, (void**)&F.out, (void**)&F.direct};
     for (int i = 0; i < 4; i++) {
@@ -285,7 +285,8 @@ int setup_field(ion_lbm* h) {
         }
     }
     for (auto* q : ptr) h->allocs.push_back(*q);
-    CK(cudaMemsetAsync(F.direct, 0, 4, h->stream));
+    F.spread = fft_field_spread(h->L);
+    CK(cudaMemsetAsync(F.direct, 0, 16, h->stream));
     CK(launch_fft_plan(h->L, F, h->stream));
     g_launches++;
     h->fft = F;
@@ -295,7 +296,7 @@ int setup_field(ion_lbm* h) {
 int launch_field(ion_lbm* h) {
     if (h->cfg.field_mode != ION_FIELD_BITWISE && h->fft.G) {
         g_launches += launch_fft_field(h->L, h->fft, nullptr, h->stream) + 1;
-        launch_update_e_b_gated(h->L, h->d_err, h->fft.direct, nullptr, h->stream);
+        launch_update_e_b_gated(h->L, h->d_err, nullptr, h->fft.direct, h->stream);
         CKL();
         return ION_OK;
     }

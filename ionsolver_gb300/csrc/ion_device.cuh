@@ -144,6 +144,12 @@ __host__ __device__ __forceinline__ float fp16c_raw(uint16_t x) {
 }
 __host__ __device__ __forceinline__ float fp16c_decode(uint16_t x) { return fp16c_raw(x) * 5.192296858534828e33f; }
 
+// whether one of four words (16-byte aligned) is set
+__device__ __forceinline__ bool any_of(const uint32_t* w) {
+    const uint4 v = *reinterpret_cast<const uint4*>(w);
+    return (v.x | v.y | v.z | v.w) != 0u;
+}
+
 // Packed FP32 pairs (PTX add/sub/mul/fma .f32x2, sm_100 and later): one
 // instruction does the same IEEE round-to-nearest operation on the two halves
 // of a 64-bit register (each instruction checked against the scalar one on the
