@@ -1738,8 +1738,9 @@ static int ensure_surrogate(ion_lbm* h) {
     const uint32_t big = 1u << h->L.nd;
     if (h->L.depth < 2 || h->L.nx / big > 1 || h->L.ny / big > 1 || h->L.nz / big > 1)
         return fail(ION_E_CONFIG, "the learned far field needs LOD depth >= 2 and an empty reference near field");
-    if (h->L.bsx > (uint32_t)ion::Surrogate::MAX_BLOCK)
-        return fail(ION_E_CONFIG, "the learned far field needs LOD blocks of at most %d cells along x",
+    // (the per-cell kernel's tables hold MAX_BLOCK entries an axis)
+    if (std::max({h->L.bsx, h->L.bsy, h->L.bsz}) > (uint32_t)ion::Surrogate::MAX_BLOCK)
+        return fail(ION_E_CONFIG, "the learned far field needs LOD blocks of at most %d cells an edge",
                     ion::Surrogate::MAX_BLOCK);
     if (h->sur) return ION_OK;
     h->sur.reset(new ion::Surrogate());

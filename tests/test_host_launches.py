@@ -23,3 +23,27 @@ def test_voxeliser_form_by_columns(fake, n, form):  # noqa: F811
     lbm.voxelise_mesh(mesh, I.ModelType.Solid())
     assert fake.kernel("k_voxelize")["name"].startswith(form)
     lbm.close()
+
+
+def _mhd(shape, depth, mode=0, **changes):
+    c = I.LbmConfig(velocity_set=2, float_type=2, n_x=shape[0], n_y=shape[1], n_z=shape[2], nu=1 / 30, ext_volume_force=True,
+                    ext_magneto_hydro=True, mhd_lod_depth=depth, field_mode=mode)
+    for k, v in changes.items():
+        setattr(c, k, v)
+    return I.Lbm(c)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("edge,accepted", [(32, True), (33, False)])
+def test_learned_field_bins_of_at_most_32_cells_an_edge(fake, axis, edge, accepted):  # noqa: F811
+    """k_surrogate_cells' tables hold 32 cells an axis (a larger bin read past them)."""
+    shape = [16, 16, 16]
+    shape[axis] = 8 * edge
+    lbm = _mhd(shape, 3)
+    if accepted:
+        lbm.set_field_mode(2)
+    else:
+        with pytest.raises(I.IonError) as e:
+            lbm.set_field_mode(2)
+        assert e.value.code == -2
+    lbm.close()
