@@ -893,7 +893,8 @@ __global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>())
 // How the row kernels run on a grid: the kernel (a row stride of k_sc_rows_ws, or k_sc_rows), the
 // rows of a group, the block and the blocks per SM.
 struct RowPlan {
-    uint32_t nx, ny, nz;  // the grid it was made for
+    int device;
+    uint32_t nx, ny, nz;  // the device and grid it was made for
     int v;
     uint32_t K, threads, smem;
     int per_sm;           // 0: the rows do not fit
@@ -906,8 +907,9 @@ struct RowPlan {
 // wider: MHD FP16S 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31 us; plain FP32 112^3
 // 41 -> 37 us, FP16S 128^3 51 -> 46 us, 64^3 FP32 6.6 -> 6.0 us (three domains in turn).  FP32 MHD holds its SMs' shared
 // memory with the smallest stride already (64 to 128 cells: within 2%).
+// failed: a runtime call did (its error is taken here); such a plan serves one launch and is not kept.
 template <int FT, bool MHD, bool TRT>
-RowPlan make_row_plan(const DevLbm& L, int sms) {
+RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
     using Kern = void (*)(const DevLbm, const uint32_t, uint32_t*);
     static const Kern kern[6] = {k_sc_rows_ws<FT, MHD, TRT, 96u>,  k_sc_rows_ws<FT, MHD, TRT, 128u>,
                                  k_sc_rows_ws<FT, MHD, TRT, 192u>, k_sc_rows_ws<FT, MHD, TRT, 256u>,
@@ -915,7 +917,8 @@ RowPlan make_row_plan(const DevLbm& L, int sms) {
     static constexpr uint32_t bytes[5] = {ws_row_bytes<FT, MHD, 96u>(), ws_row_bytes<FT, MHD, 128u>(), ws_row_bytes<FT, MHD, 192u>(),
                                           ws_row_bytes<FT, MHD, 256u>(), ws_row_bytes<FT, MHD, 384u>()};
     static_assert(2u * ws_row_bytes<ION_FP32, true, WS_ROW>() <= 200u * 1024u, "two row buffers of the widest form");
-    RowPlan best{L.nx, L.ny, L.nz, 0, 0u, 0u, 0u, 0};
+    RowPlan best{device, L.nx, L.ny, L.nz, 0, 0u, 0u, 0u, 0};
+    failed = false;
     const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
     for (int v = ws ? 0 : 5; v < 6; v++) {
         RowPlan p = best;
@@ -932,10 +935,14 @@ RowPlan make_row_plan(const DevLbm& L, int sms) {
             p.threads = ((L.nx + ((L.nx + 255u) / 256u) - 1u) / ((L.nx + 255u) / 256u) + 31u) / 32u * 32u;
         }
         p.per_sm = 0;
-        if (p.smem > 200u * 1024u ||
-            cudaFuncSetAttribute(kern[v], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p.per_sm, kern[v], (int)p.threads, p.smem) != cudaSuccess || p.per_sm < 1)
+        if (p.smem > 200u * 1024u) continue;
+        if (cudaFuncSetAttribute(kern[v], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p.per_sm, kern[v], (int)p.threads, p.smem) != cudaSuccess) {
+            cudaGetLastError();
+            failed = true;
             continue;
+        }
+        if (p.per_sm < 1) continue;
         if (best.per_sm == 0) {
             best = p;
             if (FT == ION_FP32 && MHD) break;
@@ -956,22 +963,28 @@ bool launch_sc_rows(const DevLbm& L, uint32_t o, uint32_t* err, cudaStream_t s) 
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // the plans of the last few grids, per instantiation (handles may step on several host threads)
+    // the plans of the last grids, per instantiation and device (the shared-memory opt-in and the
+    // SM count are the device's; handles may step on several host threads)
+    constexpr uint32_t KEPT = 32;
     static std::mutex mu;
-    static RowPlan plans[8] = {};
+    static RowPlan plans[KEPT] = {};
     static uint32_t next = 0;
     RowPlan p{};
     {
         std::lock_guard<std::mutex> lock(mu);
         const RowPlan* hit = nullptr;
         for (const RowPlan& q : plans)
-            if (q.nx == L.nx && q.ny == L.ny && q.nz == L.nz) hit = &q;
-        if (!hit) {
-            plans[next] = make_row_plan<FT, MHD, TRT>(L, sms);
-            hit = &plans[next];
-            next = (next + 1u) % 8u;
+            if (q.nx == L.nx && q.ny == L.ny && q.nz == L.nz && q.device == dev) hit = &q;
+        if (hit) {
+            p = *hit;
+        } else {
+            bool failed;
+            p = make_row_plan<FT, MHD, TRT>(L, dev, sms, failed);
+            if (!failed) {
+                plans[next] = p;
+                next = (next + 1u) % KEPT;
+            }
         }
-        p = *hit;
     }
     if (p.per_sm < 1) return false;
     const uint32_t grid = std::min<uint32_t>(row_groups(L.ny, L.nz, p.K), (uint32_t)(p.per_sm * sms));

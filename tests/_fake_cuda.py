@@ -51,8 +51,12 @@ def fake(tmp_path, monkeypatch):
     objects = sorted(str(p) for p in B.OUT.glob("*.o"))
     include = Path(B.nvcc()).resolve().parent.parent / "include"
     out = tmp_path / "libionsolver_fake.so"
+    # only these names leave the library: the static variables of inline functions would be one in
+    # the whole process, and this copy's runtime is not the others'
+    names = tmp_path / "names.map"
+    names.write_text("{ global: ion_*; fake_*; local: *; };\n")
     subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-shared", "-fPIC", f"-I{include}", str(SOURCE), *objects, "-Wl,-Bsymbolic",
-                    "-o", str(out)], check=True)
+                    f"-Wl,--version-script={names}", "-o", str(out)], check=True)
     lib = C.CDLL(str(out))
     for name, (res, args) in N._SIGS.items():
         f = getattr(lib, name)

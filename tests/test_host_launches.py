@@ -47,3 +47,35 @@ def test_learned_field_bins_of_at_most_32_cells_an_edge(fake, axis, edge, accept
             lbm.set_field_mode(2)
         assert e.value.code == -2
     lbm.close()
+
+
+def _plain(shape, ft=2):
+    lbm = I.Lbm(I.LbmConfig(velocity_set=2, float_type=ft, n_x=shape[0], n_y=shape[1], n_z=shape[2], nu=1 / 30))
+    lbm.initialize()
+    return lbm
+
+
+def test_row_plan_belongs_to_its_device(fake):  # noqa: F811
+    """The opt-in for more than 48 KB of shared memory is per device: the same grid on a second
+    device gets one of its own."""
+    shape = (384, 16, 16)
+    for device in (0, 1, 0):
+        assert fake.lib.ion_select_device(device) == 0
+        lbm = _plain(shape)
+        lbm.do_time_step()
+        k = fake.kernel("k_sc_rows_ws")
+        assert k["device"] == device and k["smem"] > 48 * 1024
+        lbm.close()
+
+
+@pytest.mark.parametrize("call", ["cudaFuncSetAttribute", "cudaOccupancy"])
+def test_row_plan_that_failed_is_not_kept(fake, call):  # noqa: F811
+    """A runtime call that fails once costs one step the row kernels, and its error is not the
+    fallback's."""
+    lbm = _plain((320, 16, 16))
+    fake.fail(call)
+    lbm.do_time_step()
+    assert fake.launches()[-1]["name"].startswith("k_stream_collide")
+    lbm.do_time_step()
+    assert fake.launches()[-1]["name"].startswith("k_sc_rows_ws")
+    lbm.close()
