@@ -789,9 +789,8 @@ __host__ __device__ constexpr int ws_min_ctas() {
     return RS == 384u ? ((MHD && TRT) ? 1 : 2) : ((MHD && TRT) ? 576 : 896) / ws_threads<RS>();
 }
 template <int FT, bool MHD, bool TRT, uint32_t RS>
-__global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_t, uint32_t* err) {
+__global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_t, const uint32_t K, uint32_t* err) {  // K: rows a group
     using T = typename Ddf<FT>::T;
-    const uint32_t K = RS / L.nx;  // rows a group
     constexpr uint32_t RB = ws_row_bytes<FT, MHD, RS>();
     constexpr uint32_t SB = RS * (uint32_t)sizeof(T);  // bytes per stream row
     constexpr uint32_t eb_off = row_streams<FT, MHD>() * SB, fl_off = eb_off + (MHD ? 6u * RS * 4u : 0u);
@@ -900,9 +899,12 @@ struct RowPlan {
     int per_sm;           // 0: the rows do not fit
 };
 
-// The smallest stride that holds a row, or, with 16-bit storage and without MHD, a wider one
-// that stages several short rows at a time: the one thread that issues the copies then has
-// fewer, longer ones.  It is taken where it keeps at least 5% more cells on an SM and the
+// The smallest stride that holds a row, with as many rows a group as the resident blocks leave it (a
+// group's copies are issued by one thread, row by row where a neighbour row wraps around: with six
+// rows a group 16^3 took 8.3 us plain and 16.5 us with MHD, with one 5.2 and 10.4; 16x96x96 with
+// one 15.4 and 39.0 us, with four or six 9.4 to 12.3 and 24.8 to 28.8).  Or, but for FP32 with
+// MHD, a wider stride that stages several short rows at a time: the one thread that issues the
+// copies then has fewer, longer ones.  It is taken where it keeps at least 5% more cells on an SM and the
 // groups still feed every resident block at least twice.  The smallest stride against the
 // wider: MHD FP16S 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31 us; plain FP32 112^3
 // 41 -> 37 us, FP16S 128^3 51 -> 46 us, 64^3 FP32 6.6 -> 6.0 us (three domains in turn).  FP32 MHD holds its SMs' shared
@@ -910,10 +912,10 @@ struct RowPlan {
 // failed: a runtime call did (its error is taken here); such a plan serves one launch and is not kept.
 template <int FT, bool MHD, bool TRT>
 RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
-    using Kern = void (*)(const DevLbm, const uint32_t, uint32_t*);
-    static const Kern kern[6] = {k_sc_rows_ws<FT, MHD, TRT, 96u>,  k_sc_rows_ws<FT, MHD, TRT, 128u>,
-                                 k_sc_rows_ws<FT, MHD, TRT, 192u>, k_sc_rows_ws<FT, MHD, TRT, 256u>,
-                                 k_sc_rows_ws<FT, MHD, TRT, 384u>, k_sc_rows<FT, MHD, TRT>};
+    static const void* const kern[6] = {
+        (const void*)k_sc_rows_ws<FT, MHD, TRT, 96u>,  (const void*)k_sc_rows_ws<FT, MHD, TRT, 128u>,
+        (const void*)k_sc_rows_ws<FT, MHD, TRT, 192u>, (const void*)k_sc_rows_ws<FT, MHD, TRT, 256u>,
+        (const void*)k_sc_rows_ws<FT, MHD, TRT, 384u>, (const void*)k_sc_rows<FT, MHD, TRT>};
     static constexpr uint32_t bytes[5] = {ws_row_bytes<FT, MHD, 96u>(), ws_row_bytes<FT, MHD, 128u>(), ws_row_bytes<FT, MHD, 192u>(),
                                           ws_row_bytes<FT, MHD, 256u>(), ws_row_bytes<FT, MHD, 384u>()};
     static_assert(2u * ws_row_bytes<ION_FP32, true, WS_ROW>() <= 200u * 1024u, "two row buffers of the widest form");
@@ -923,24 +925,36 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
     for (int v = ws ? 0 : 5; v < 6; v++) {
         RowPlan p = best;
         p.v = v;
+        auto set_rows = [&](uint32_t K) {
+            p.K = K;
+            p.threads = (K * L.nx + 31u) / 32u * 32u + 32u;
+        };
         if (v < 5) {
             if (ws_rows(v) < L.nx) continue;
-            p.K = ws_rows(v) / L.nx;
             p.smem = 2u * bytes[v];
-            p.threads = (p.K * L.nx + 31u) / 32u * 32u + 32u;
+            set_rows(best.per_sm == 0 ? 1u : ws_rows(v) / L.nx);
         } else {
             if (ws) break;
             p.K = 1u;
             p.smem = 2u * row_bytes<FT, MHD>(L.nx);
             p.threads = ((L.nx + ((L.nx + 255u) / 256u) - 1u) / ((L.nx + 255u) / 256u) + 31u) / 32u * 32u;
         }
-        p.per_sm = 0;
         if (p.smem > 200u * 1024u) continue;
-        if (cudaFuncSetAttribute(kern[v], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p.per_sm, kern[v], (int)p.threads, p.smem) != cudaSuccess) {
+        auto occupancy = [&]() {
+            p.per_sm = 0;
+            if (cudaFuncSetAttribute(kern[v], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p.per_sm, kern[v], (int)p.threads, p.smem) == cudaSuccess)
+                return;
             cudaGetLastError();
             failed = true;
-            continue;
+            p.per_sm = 0;
+        };
+        occupancy();
+        if (v < 5 && best.per_sm == 0 && p.per_sm > 0 && ws_rows(v) / L.nx > 1u) {
+            // more rows a group only where a row each would give the resident blocks more than one
+            const uint32_t resident = (uint32_t)(p.per_sm * sms);
+            set_rows(std::min(ws_rows(v) / L.nx, (L.ny * L.nz + resident - 1u) / resident));
+            occupancy();
         }
         if (p.per_sm < 1) continue;
         if (best.per_sm == 0) {
@@ -988,11 +1002,11 @@ bool launch_sc_rows(const DevLbm& L, uint32_t o, uint32_t* err, cudaStream_t s) 
     }
     if (p.per_sm < 1) return false;
     const uint32_t grid = std::min<uint32_t>(row_groups(L.ny, L.nz, p.K), (uint32_t)(p.per_sm * sms));
-    if (p.v == 0) k_sc_rows_ws<FT, MHD, TRT, 96u><<<grid, p.threads, p.smem, s>>>(L, o, err);
-    else if (p.v == 1) k_sc_rows_ws<FT, MHD, TRT, 128u><<<grid, p.threads, p.smem, s>>>(L, o, err);
-    else if (p.v == 2) k_sc_rows_ws<FT, MHD, TRT, 192u><<<grid, p.threads, p.smem, s>>>(L, o, err);
-    else if (p.v == 3) k_sc_rows_ws<FT, MHD, TRT, 256u><<<grid, p.threads, p.smem, s>>>(L, o, err);
-    else if (p.v == 4) k_sc_rows_ws<FT, MHD, TRT, 384u><<<grid, p.threads, p.smem, s>>>(L, o, err);
+    if (p.v == 0) k_sc_rows_ws<FT, MHD, TRT, 96u><<<grid, p.threads, p.smem, s>>>(L, o, p.K, err);
+    else if (p.v == 1) k_sc_rows_ws<FT, MHD, TRT, 128u><<<grid, p.threads, p.smem, s>>>(L, o, p.K, err);
+    else if (p.v == 2) k_sc_rows_ws<FT, MHD, TRT, 192u><<<grid, p.threads, p.smem, s>>>(L, o, p.K, err);
+    else if (p.v == 3) k_sc_rows_ws<FT, MHD, TRT, 256u><<<grid, p.threads, p.smem, s>>>(L, o, p.K, err);
+    else if (p.v == 4) k_sc_rows_ws<FT, MHD, TRT, 384u><<<grid, p.threads, p.smem, s>>>(L, o, p.K, err);
     else k_sc_rows<FT, MHD, TRT><<<grid, p.threads, p.smem, s>>>(L, o, err);
     return true;
 }

@@ -79,3 +79,27 @@ def test_row_plan_that_failed_is_not_kept(fake, call):  # noqa: F811
     lbm.do_time_step()
     assert fake.launches()[-1]["name"].startswith("k_sc_rows_ws")
     lbm.close()
+
+
+@pytest.mark.parametrize("shape,ft", [((16, 16, 16), 2), ((16, 16, 2), 0), ((32, 16, 16), 1), ((48, 12, 12), 2)])
+@pytest.mark.parametrize("mhd", [False, True])
+def test_few_short_rows_are_staged_one_by_one(fake, shape, ft, mhd):  # noqa: F811
+    """A row a block while the resident blocks hold all of them (in groups of three to six 16^3
+    took 8.4 us instead of 5.2)."""
+    if mhd:
+        shape = tuple(max(16, s) for s in shape)
+        lbm = _mhd(shape, 2, float_type=ft)
+        lbm.initialize()
+    else:
+        lbm = _plain(shape, ft)
+    lbm.do_time_step()
+    k = fake.kernel("k_sc_rows_ws")
+    assert k["grid"] == shape[1] * shape[2] and k["block"] == (shape[0] + 31) // 32 * 32 + 32
+    lbm.close()
+
+
+def test_many_short_rows_are_staged_in_groups(fake):  # noqa: F811
+    lbm = _plain((16, 96, 96))
+    lbm.do_time_step()
+    assert fake.kernel("k_sc_rows_ws")["block"] >= 4 * 16 + 32
+    lbm.close()
