@@ -909,6 +909,10 @@ struct RowPlan {
 // wider: MHD FP16S 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31 us; plain FP32 112^3
 // 41 -> 37 us, FP16S 128^3 51 -> 46 us, 64^3 FP32 6.6 -> 6.0 us (three domains in turn).  FP32 MHD holds its SMs' shared
 // memory with the smallest stride already (64 to 128 cells: within 2%).
+// FP32 SRT lattices that do not stay in L2, in rows of 96 cells and more, run slower with more than
+// about 720 cells of the plain stencil or 400 of the MHD one staged on an SM: us a step with the
+// blocks that fit and with the bound (at least three blocks), 128^3 63.1 / 60.4, 160^3 119.7 / 112, 224x160x160
+// 166 / 156; MHD 96x128x128 116.7 / 113.5.  The other forms gain from every block.
 // failed: a runtime call did (its error is taken here); such a plan serves one launch and is not kept.
 template <int FT, bool MHD, bool TRT>
 RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
@@ -922,6 +926,7 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
     RowPlan best{device, L.nx, L.ny, L.nz, 0, 0u, 0u, 0u, 0};
     failed = false;
     const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
+    const bool bounded = FT == ION_FP32 && !TRT && L.nx >= 96u && (uint64_t)L.n * ((MHD ? 45u : 19u) * 4u) > 96ull << 20;  // (L2: 129 MB)
     for (int v = ws ? 0 : 5; v < 6; v++) {
         RowPlan p = best;
         p.v = v;
@@ -957,9 +962,10 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
             occupancy();
         }
         if (p.per_sm < 1) continue;
+        if (v < 5 && bounded) p.per_sm = std::min(p.per_sm, std::max(3, (int)((MHD ? 400u : 720u) / L.nx)));
         if (best.per_sm == 0) {
             best = p;
-            if (FT == ION_FP32 && MHD) break;
+            if ((FT == ION_FP32 && MHD) || bounded) break;
         } else if ((uint64_t)p.per_sm * p.K * 100u > (uint64_t)best.per_sm * best.K * 105u &&
                    row_groups(L.ny, L.nz, p.K) >= 2u * (uint32_t)(p.per_sm * sms)) {
             best = p;

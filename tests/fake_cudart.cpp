@@ -101,7 +101,7 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v) {
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int threads, size_t smem, unsigned) {
     if (failing("cudaOccupancy")) return result(cudaErrorUnknown);
-    const int by_smem = (int)((227u * 1024u) / (smem + 1024u)), by_regs = 65536 / (72 * threads);
+    const int by_smem = (int)((227u * 1024u) / (smem + 1024u)), by_regs = 65536 / (64 * threads);
     *n = by_smem < by_regs ? by_smem : by_regs;
     return cudaSuccess;
 }

@@ -103,3 +103,15 @@ def test_many_short_rows_are_staged_in_groups(fake):  # noqa: F811
     lbm.do_time_step()
     assert fake.kernel("k_sc_rows_ws")["block"] >= 4 * 16 + 32
     lbm.close()
+
+
+@pytest.mark.parametrize("shape,mhd,blocks", [((160, 128, 128), False, 4), ((224, 128, 128), False, 3), ((128, 128, 128), False, 5),
+                                              ((160, 64, 64), False, 5), ((96, 96, 96), True, 4)])
+def test_fp32_rows_beyond_l2_are_staged_on_fewer_blocks(fake, shape, mhd, blocks):  # noqa: F811
+    """At most 720 cells of the plain stencil and 400 of the MHD one on an SM (160^3 took 119.7 us with
+    the five blocks that fit, 112 with four); a lattice inside L2 keeps them all."""
+    lbm = _mhd(shape, 2) if mhd else _plain(shape)
+    lbm.initialize()
+    lbm.do_time_step()
+    assert fake.kernel("k_sc_rows_ws")["grid"] == blocks * 152
+    lbm.close()
