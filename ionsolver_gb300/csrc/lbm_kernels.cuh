@@ -784,12 +784,16 @@ __host__ __device__ constexpr uint32_t ws_row_bytes() {
 // registers), one for MHD with TRT.
 template <uint32_t RS>
 __host__ __device__ constexpr int ws_threads() { return (int)RS + 32; }
-template <uint32_t RS, bool MHD, bool TRT>
+// (MHD with TRT at 128 in FP32 and FP16S: 96 registers, four blocks of 112 or 128 cells; with 128 registers three,
+// FP32 112x128x128 130 -> 144 us, FP16S 32x128x128 64 -> 100 us.  FP16C needs the 128: there 157 us, 177 with 96.)
+template <int FT, uint32_t RS, bool MHD, bool TRT>
+__host__ __device__ constexpr int ws_bound() { return MHD && TRT && RS == 128u && FT != ION_FP16C ? 288 : ws_threads<RS>(); }
+template <int FT, uint32_t RS, bool MHD, bool TRT>
 __host__ __device__ constexpr int ws_min_ctas() {
-    return RS == 384u ? ((MHD && TRT) ? 1 : 2) : ((MHD && TRT) ? 576 : 896) / ws_threads<RS>();
+    return RS == 384u ? ((MHD && TRT) ? 1 : 2) : ((MHD && TRT) ? 576 : 896) / ws_bound<FT, RS, MHD, TRT>();
 }
 template <int FT, bool MHD, bool TRT, uint32_t RS>
-__global__ void __launch_bounds__(ws_threads<RS>(), ws_min_ctas<RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_t, const uint32_t K, uint32_t* err) {  // K: rows a group
+__global__ void __launch_bounds__(ws_bound<FT, RS, MHD, TRT>(), ws_min_ctas<FT, RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_t, const uint32_t K, uint32_t* err) {  // K: rows a group
     using T = typename Ddf<FT>::T;
     constexpr uint32_t RB = ws_row_bytes<FT, MHD, RS>();
     constexpr uint32_t SB = RS * (uint32_t)sizeof(T);  // bytes per stream row
@@ -909,10 +913,11 @@ struct RowPlan {
 // wider: MHD FP16S 128^3 121 -> 102 us, 112^3 94 -> 74 us, 80^3 39 -> 31 us; plain FP32 112^3
 // 41 -> 37 us, FP16S 128^3 51 -> 46 us, 64^3 FP32 6.6 -> 6.0 us (three domains in turn).  FP32 MHD holds its SMs' shared
 // memory with the smallest stride already (64 to 128 cells: within 2%).
-// FP32 SRT lattices that do not stay in L2, in rows of 96 cells and more, run slower with more than
+// FP32 lattices that do not stay in L2 (SRT, and TRT with MHD), in rows of 96 cells and more, run slower with more than
 // about 720 cells of the plain stencil or 400 of the MHD one staged on an SM: us a step with the
 // blocks that fit and with the bound (at least three blocks), 128^3 63.1 / 60.4, 160^3 119.7 / 112, 224x160x160
-// 166 / 156; MHD 96x128x128 116.7 / 113.5.  The other forms gain from every block.
+// 166 / 156; MHD 96x128x128 116.7 / 113.5.  MHD with TRT: 450 cells, 128^3 154 / 148.  The other forms
+// gain from every block.
 // failed: a runtime call did (its error is taken here); such a plan serves one launch and is not kept.
 template <int FT, bool MHD, bool TRT>
 RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
@@ -926,7 +931,7 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
     RowPlan best{device, L.nx, L.ny, L.nz, 0, 0u, 0u, 0u, 0};
     failed = false;
     const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
-    const bool bounded = FT == ION_FP32 && !TRT && L.nx >= 96u && (uint64_t)L.n * ((MHD ? 45u : 19u) * 4u) > 96ull << 20;  // (L2: 129 MB)
+    const bool bounded = FT == ION_FP32 && (MHD || !TRT) && L.nx >= 96u && (uint64_t)L.n * ((MHD ? 45u : 19u) * 4u) > 96ull << 20;  // (L2: 129 MB)
     for (int v = ws ? 0 : 5; v < 6; v++) {
         RowPlan p = best;
         p.v = v;
@@ -962,7 +967,7 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
             occupancy();
         }
         if (p.per_sm < 1) continue;
-        if (v < 5 && bounded) p.per_sm = std::min(p.per_sm, std::max(3, (int)((MHD ? 400u : 720u) / L.nx)));
+        if (v < 5 && bounded) p.per_sm = std::min(p.per_sm, std::max(3, (int)((!MHD ? 720u : TRT ? 450u : 400u) / L.nx)));
         if (best.per_sm == 0) {
             best = p;
             if ((FT == ION_FP32 && MHD) || bounded) break;

@@ -115,3 +115,16 @@ def test_fp32_rows_beyond_l2_are_staged_on_fewer_blocks(fake, shape, mhd, blocks
     lbm.do_time_step()
     assert fake.kernel("k_sc_rows_ws")["grid"] == blocks * 152
     lbm.close()
+
+
+@pytest.mark.parametrize("ft", [0, 2])
+def test_mhd_trt_rows_of_128_keep_four_blocks(ft):
+    """At most 102 registers, so that four blocks of 160 threads fit (with 128 registers three: FP32
+    112x128x128 144 us instead of 130)."""
+    from ionsolver_gb300 import build as B
+    log = (B.OUT / "ptxas.log").read_text()
+    name = f"k_sc_rows_wsILi{ft}ELb1ELb1ELj128E"
+    if name not in log:
+        pytest.skip("the stencil was not compiled by the last build")
+    used = log[log.index(name):].split("Used ")[1].split()[0]
+    assert int(used) <= 102
