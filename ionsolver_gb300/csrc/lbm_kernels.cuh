@@ -564,10 +564,14 @@ __device__ __forceinline__ void sc_cell(const DevLbm& L, const uint32_t n, const
     }
 }
 
-// Blocks per SM: six for D2Q9 (its nine loads leave registers for 48 warps; 2048^2 FP32 74 ->
-// 68 us, FP16S 69 -> 62 us against four), four for the others without MHD
+// Blocks per SM without MHD: four, but for D2Q9 in FP32, whose nine loads leave registers for six
+// (2000x1000 38.9 -> 33.8 us) or with TRT five (42.0 -> 39.0 us; six spill).  With 16-bit codes six spill
+// as well and gain nothing: FP16S 400^2 5.2 -> 6.2 us, 1024^2 TRT 19.5 -> 20.6, FP16C 2000x1000
+// TRT 40.0 -> 42.0.
+template <int Q, int FT, bool TRT>
+__host__ __device__ constexpr int sc_blocks() { return Q == 9 && FT == ION_FP32 ? (TRT ? 5 : 6) : 4; }
 template <int Q, int FT, bool MHD, bool TRT, bool ECR = false>
-__global__ void __launch_bounds__(256, MHD ? 2 : Q == 9 ? 6 : 4) k_stream_collide(const DevLbm L, const uint32_t odd_t) {
+__global__ void __launch_bounds__(256, MHD ? 2 : sc_blocks<Q, FT, TRT>()) k_stream_collide(const DevLbm L, const uint32_t odd_t) {
     const bool odd = odd_t != 0u;
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < L.n; n += gridDim.x * blockDim.x)
         sc_cell<Q, FT, MHD, TRT, ECR>(L, n, odd);

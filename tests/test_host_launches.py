@@ -128,3 +128,19 @@ def test_mhd_trt_rows_of_128_keep_four_blocks(ft):
         pytest.skip("the stencil was not compiled by the last build")
     used = log[log.index(name):].split("Used ")[1].split()[0]
     assert int(used) <= 102
+
+
+def test_d2q9_stencils_do_not_spill():
+    """(bounded to six blocks an SM the 16-bit ones did: FP16S 700^2 10.1 us instead of 9.3)"""
+    import re
+    from ionsolver_gb300 import build as B
+    log = (B.OUT / "ptxas.log").read_text()
+    found = 0
+    for ft in range(3):
+        for trt in range(2):
+            name = f"k_stream_collideILi9ELi{ft}ELb0ELb{trt}ELb0E"
+            if name in log:
+                found += 1
+                assert int(re.search(r"(\d+) bytes spill stores", log[log.index(name):]).group(1)) == 0, name
+    if not found:
+        pytest.skip("the stencil was not compiled by the last build")
