@@ -190,6 +190,7 @@ struct ion_lbm {
     uint32_t* d_tiles = nullptr;
     uint32_t* d_list = nullptr;
     uint32_t* d_count = nullptr;
+    ion::PsiInfo* psi_info = nullptr;  // pinned: written by the device, read by the host (null: no table)
     void* psi_ws = nullptr;  // terms and runs of the magnets' potential (kept up to PSI_KEEP bytes)
     size_t psi_ws_bytes = 0;
     float *d_p0 = nullptr, *d_p1 = nullptr, *d_p2 = nullptr;
@@ -232,6 +233,7 @@ void destroy_handle(ion_lbm* h) {
     if (h->graph) cudaGraphExecDestroy(h->graph);
     for (void* p : h->allocs) cudaFree(p);
     cudaFree(h->psi_ws);
+    cudaFreeHost(h->psi_info);
     for (auto& e : h->ev) if (e) cudaEventDestroy(e);
     for (auto& e : h->kev) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
     for (auto e : h->ev_pool) cudaEventDestroy(e);
@@ -627,6 +629,10 @@ int ion_lbm_create(const ion_config* cfg, ion_lbm** out) {
     }
     rc = setup_field(h);
     if (rc) { destroy_handle(h); return rc; }
+    if (mhd && cudaHostAlloc((void**)&h->psi_info, sizeof(PsiInfo), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        h->psi_info = nullptr;
+    }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) { destroy_handle(h); return fail(ION_E_CUDA, "create: stream sync failed"); }
     for (auto& e : h->ev) cudaEventCreate(&e);
     *out = h;
@@ -960,24 +966,24 @@ static int ensure_compaction(ion_lbm* h) {
     return ION_OK;
 }
 
-// The tabulated form of the magnets' potential (P.T null: the direct sum runs): the runs of the
-// compacted list, read back for the table's size, and the table's memory.  The part of E_dyn
-// that the potential will overwrite holds the runs (8 bytes each) until their number is known.  Below 64 cells the direct sum costs less than the table.
-static int psi_table(ion_lbm* h, PsiTable& P, uint32_t& kinds) {
-    if (h->L.n >= 1u << 30) return ION_OK;  // a run keeps its magnetisation in the index's top bits
+// The tabulated form of the magnets' potential (P.T null: the direct sum runs), of lists of `from`
+// cells and more: the runs of the compacted list, their number and bounds written to pinned memory, and
+// the table's memory.  The part of E_dyn that the potential will overwrite holds the runs (8 bytes
+// each) until their number is known.
+static int psi_table(ion_lbm* h, uint32_t from, PsiTable& P, uint32_t& kinds) {
     uint2* const runs = (uint2*)h->L.e_dyn;
-    PsiInfo* const d_info = (PsiInfo*)h->d_partials;
-    PsiInfo info;
+    PsiInfo& info = *h->psi_info;
     const size_t npsi = (size_t)(h->L.nx + 2) * (h->L.ny + 2) * (h->L.nz + 2);
-    launch_psi_runs(h->L, h->d_list, h->d_count, runs, (uint32_t)(npsi / 2 - 1), d_info, h->stream);
+    launch_psi_runs(h->L, h->d_list, h->d_count, runs, (uint32_t)(npsi / 2 - 1), from, h->psi_info, h->stream);
     g_launches++;
     CKL();
-    CK(cudaMemcpyAsync(&info, d_info, sizeof info, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    if (info.count < 64u || info.kinds > PSI_KINDS) return ION_OK;
+    if (info.count < from || info.kinds > PSI_KINDS) return ION_OK;
     const size_t bytes = psi_table_size(h->L, info, P), run_bytes = sizeof(uint2) * ((size_t)info.runs + 1);
     const size_t at = (bytes + 255) / 256 * 256;
-    if ((uint64_t)P.tx * P.ny >= 1ull << 32 || (uint64_t)P.tz * info.kinds > 65535u) return ION_OK;
+    if ((uint64_t)P.tx * P.ny >= 1ull << 32 || (uint64_t)P.tz * info.kinds > 65535u ||
+        !psi_table_pays(h->L, info, bytes / sizeof(float)))
+        return ION_OK;
     if (h->psi_ws_bytes < at + run_bytes) {
         cudaFree(h->psi_ws);
         h->psi_ws_bytes = 0;
@@ -1004,13 +1010,24 @@ int ion_lbm_precompute_b(ion_lbm* h) {
     g_launches += 3;
     PsiTable P{};
     uint32_t kinds = 0;
-    rc = psi_table(h, P, kinds);
-    if (rc) return rc;
+    const uint32_t from = h->psi_info ? psi_table_from(h->L) : 0xFFFFFFFFu;
+    bool done = false;
+    if (from != 0xFFFFFFFFu && (uint64_t)(h->L.nx + 2) * (h->L.ny + 2) * (h->L.nz + 2) < PSI_FEW_POINTS) {
+        launch_psi_static_b(h->L, h->d_list, h->d_count, from, h->psi_info, h->stream);
+        g_launches += 2;
+        CKL();
+        CK(cudaStreamSynchronize(h->stream));
+        done = h->psi_info->count < from;
+    }
+    if (!done && from != 0xFFFFFFFFu) {
+        rc = psi_table(h, from, P, kinds);
+        if (rc) return rc;
+    }
     if (P.T) {
-        launch_psi_table_static_b(h->L, P, kinds, h->stream);
+        launch_psi_table_static_b(h->L, P, kinds, h->d_count, h->stream);
         g_launches += 3;
-    } else {
-        launch_psi_static_b(h->L, h->d_list, h->d_count, h->stream);
+    } else if (!done) {
+        launch_psi_static_b(h->L, h->d_list, h->d_count, 0xFFFFFFFFu, nullptr, h->stream);
         g_launches += 2;
     }
     CKL();

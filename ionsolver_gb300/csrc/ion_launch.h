@@ -25,6 +25,10 @@ struct VoxArgs {
 
 // a list of magnet cells as runs along x (setup_kernels.cu, k_psi_runs)
 constexpr uint32_t PSI_KINDS = 4;  // distinct magnetisations with a table of their own
+// On fewer points a wait costs a short list more than two launches for nothing a long one: the direct
+// sum of short lists is launched before the host knows the length (32^3 without cells 41 us; with a look at the
+// list 57).
+constexpr uint32_t PSI_FEW_POINTS = 1u << 18;
 struct PsiInfo {
     uint32_t count, runs, kinds;   // kinds > PSI_KINDS: not tabulated
     uint32_t lo[3], hi[3];         // bounds of the cells
@@ -104,12 +108,18 @@ void launch_div_check(uint64_t samples, uint64_t seed, unsigned long long* bad, 
 void launch_update_e_b_gated(const DevLbm& L, uint32_t* err, const uint32_t* gate, const uint32_t* direct, cudaStream_t s);
 void launch_voxelize(const DevLbm& L, const VoxArgs& A, cudaStream_t s);
 void launch_compact(const DevLbm& L, uint8_t mask, uint32_t* tiles, uint32_t* list, uint32_t* total, cudaStream_t s);
-void launch_psi_static_b(const DevLbm& L, const uint32_t* mags, const uint32_t* count, cudaStream_t s);
+// the potential summed directly and the static field, of a list of fewer than `below` cells; its length to
+// info->count (where given)
+void launch_psi_static_b(const DevLbm& L, const uint32_t* mags, const uint32_t* count, uint32_t below, PsiInfo* info,
+                         cudaStream_t s);
 // runs of the list; the table's size for them; the table, the potential and the static field
 void launch_psi_runs(const DevLbm& L, const uint32_t* list, const uint32_t* count, uint2* runs, uint32_t max_runs,
-                     PsiInfo* info, cudaStream_t s);
+                     uint32_t from, PsiInfo* info, cudaStream_t s);
+// the length from which a list's runs are worth a look, and whether they pay for the table (of `entries` terms)
+uint32_t psi_table_from(const DevLbm& L);
+bool psi_table_pays(const DevLbm& L, const PsiInfo& I, size_t entries);
 size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P);
-void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, cudaStream_t s);
+void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, const uint32_t* count, cudaStream_t s);
 void launch_static_e(const DevLbm& L, const uint32_t* list, const uint32_t* count, float* E, cudaStream_t s);
 void launch_sum_f64(const void* x, int ft, uint64_t count, double* partials, uint32_t nparts, double* out,
                     cudaStream_t s);

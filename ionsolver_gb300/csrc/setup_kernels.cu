@@ -264,7 +264,10 @@ void launch_compact(const DevLbm& L, uint8_t mask, uint32_t* tiles, uint32_t* li
 // ---------------------------------------------------------------------------
 constexpr uint32_t MAG_TILE = 256;
 
-__global__ void __launch_bounds__(256) k_psi(const DevLbm L, const uint32_t* mags, const uint32_t* count, float* psi) {
+// On few points k_psi and k_static_b are launched for lists of fewer than `below` cells before the host
+// knows the length, which k_static_b reports.
+__global__ void __launch_bounds__(256) k_psi(const DevLbm L, const uint32_t* mags, const uint32_t* count, const uint32_t below,
+                                             float* psi) {
     __shared__ float4 s_p[MAG_TILE];  // (x+1, y+1, z+1) as float
     __shared__ float4 s_m[MAG_TILE];  // magnetisation
     const uint32_t l0 = L.nx + 2, l1 = L.ny + 2;
@@ -273,6 +276,7 @@ __global__ void __launch_bounds__(256) k_psi(const DevLbm L, const uint32_t* mag
     const uint32_t t = i % (l0 * l1);
     const float cx = (float)(t % l0), cy = (float)(t / l0), cz = (float)(i / (l0 * l1));
     const uint32_t nm = *count;
+    if (nm >= below) return;
     const size_t N = L.n;
     float acc = 0.0f;
     for (uint32_t base = 0; base < nm; base += MAG_TILE) {
@@ -298,9 +302,11 @@ __global__ void __launch_bounds__(256) k_psi(const DevLbm L, const uint32_t* mag
     if (i < np) psi[i] = (float)((double)acc / (4.0 * 3.14159265358979323846));
 }
 
-__global__ void __launch_bounds__(256) k_static_b(const DevLbm L, const float* psi) {
+__global__ void __launch_bounds__(256) k_static_b(const DevLbm L, const uint32_t* count, const uint32_t below, PsiInfo* info,
+                                                  const float* psi) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= L.n || (L.flags[n] & F_S) == F_S) return;
+    if (info && n == 0u) info->count = *count;
+    if (*count >= below || n >= L.n || (L.flags[n] & F_S) == F_S) return;
     uint32_t x, y, z;
     cell_xyz(L, n, x, y, z);
     const uint32_t l0 = L.nx + 2, l1 = L.ny + 2;
@@ -331,13 +337,19 @@ __global__ void __launch_bounds__(256) k_static_b(const DevLbm L, const float* p
 // ---------------------------------------------------------------------------
 constexpr uint32_t PSI_R = 16, PSI_THREADS = 256, RUN_THREADS = 1024;
 
-// one block, the list in tiles: distinct magnetisations, bounds and runs, in list order.
+// one block, the list in tiles: distinct magnetisations, bounds and runs, in list order (of a list
+// of fewer than `from` cells the length only).
 // runs[r] = (first list entry, its cell | magnetisation << 30), runs[number of runs] = (list length, 0)
 __global__ void __launch_bounds__(RUN_THREADS) k_psi_runs(const DevLbm L, const uint32_t* list, const uint32_t* count,
-                                                          uint2* runs, const uint32_t max_runs, PsiInfo* info) {
+                                                          uint2* runs, const uint32_t max_runs, const uint32_t from,
+                                                          PsiInfo* info) {
     __shared__ uint32_t s_m[PSI_KINDS][3], s_kinds, s_first, s_warp[RUN_THREADS / 32], s_lo[3], s_hi[3];
     const uint32_t nm = *count, t = threadIdx.x, lane = t & 31u;
     const size_t N = L.n;
+    if (nm < from) {
+        if (t == 0) info->count = nm;
+        return;
+    }
     if (t == 0) s_kinds = 0u;
     if (t < 3) { s_lo[t] = 0xFFFFFFFFu; s_hi[t] = 0u; }
     uint32_t nruns = 0;
@@ -488,9 +500,28 @@ __global__ void __launch_bounds__(PSI_THREADS, 4) k_psi_runs_sum(const DevLbm L,
     }
 }
 
-void launch_psi_runs(const DevLbm& L, const uint32_t* list, const uint32_t* count, uint2* runs, uint32_t max_runs,
+void launch_psi_runs(const DevLbm& L, const uint32_t* list, const uint32_t* count, uint2* runs, uint32_t max_runs, uint32_t from,
                      PsiInfo* info, cudaStream_t s) {
-    k_psi_runs<<<1, RUN_THREADS, 0, s>>>(L, list, count, runs, max_runs, info);
+    k_psi_runs<<<1, RUN_THREADS, 0, s>>>(L, list, count, runs, max_runs, from, info);
+}
+
+// Estimates in us, from calls on 16^3 to 256^3 cells with 1 to 2,000 magnet cells, scattered or
+// in a block; both forms take 42 us besides.  A cell costs the direct sum a divide per point (or
+// its latency, on few points); the table costs a host read-back and a term per entry, then
+// per point an addition a cell and some seven a run.  The lines are crossed near 460 cells at 32^3, 130 at 64^3 and
+// 40 at 128^3 (in one block): direct / table, us, 32^3 with 100 scattered cells 53 / 106, in a
+// block 55 / 82; 128^3 with 64 scattered 232 / 470, in a block 234 / 163.
+static double psi_points(const DevLbm& L) { return (double)(L.nx + 2u) * (L.ny + 2u) * (L.nz + 2u); }
+static double psi_direct_us(const DevLbm& L, double cells) { return cells * std::max(0.13, 0.07 + 1.2e-6 * psi_points(L)); }
+uint32_t psi_table_from(const DevLbm& L) {
+    if (L.n >= 1u << 30) return 0xFFFFFFFFu;  // a run keeps its magnetisation in the index's top bits
+    const double np = psi_points(L);
+    return (uint32_t)(((np < PSI_FEW_POINTS ? 60.0 : 45.0) + 2.5e-5 * np) / psi_direct_us(L, 1.0));
+}
+bool psi_table_pays(const DevLbm& L, const PsiInfo& I, size_t entries) {
+    const double np = psi_points(L);
+    return psi_direct_us(L, I.count) >
+           20.0 + 1.6e-5 * (double)entries + I.runs * std::max(0.12, 3.2e-7 * np) + I.count * std::max(0.05, 2.6e-8 * np);
 }
 
 size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P) {
@@ -510,7 +541,7 @@ size_t psi_table_size(const DevLbm& L, const PsiInfo& I, PsiTable& P) {
     return (size_t)I.kinds * P.tz * P.tx * P.ty * sizeof(float);
 }
 
-void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, cudaStream_t s) {
+void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kinds, const uint32_t* count, cudaStream_t s) {
     k_psi_terms<<<dim3((P.tx * P.ny + 255u) / 256u, P.tz * kinds), 256, 0, s>>>(P);
     const uint64_t rows = (uint64_t)(L.ny + 2) * (L.nz + 2), nxb = (L.nx + 2u + PSI_R - 1u) / PSI_R;
     const unsigned grid = grid_for((rows + 31u) / 32u * nxb * 32u, PSI_THREADS);
@@ -519,13 +550,13 @@ void launch_psi_table_static_b(const DevLbm& L, const PsiTable& P, uint32_t kind
     else if (P.ty == 192u) k_psi_runs_sum<192><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
     else if (P.ty == 256u) k_psi_runs_sum<256><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
     else k_psi_runs_sum<0><<<grid, PSI_THREADS, 0, s>>>(L, P, L.e_dyn);
-    k_static_b<<<grid_for(L.n, 256), 256, 0, s>>>(L, L.e_dyn);
+    k_static_b<<<grid_for(L.n, 256), 256, 0, s>>>(L, count, 0xFFFFFFFFu, nullptr, L.e_dyn);
 }
 
-void launch_psi_static_b(const DevLbm& L, const uint32_t* mags, const uint32_t* count, cudaStream_t s) {
+void launch_psi_static_b(const DevLbm& L, const uint32_t* mags, const uint32_t* count, uint32_t below, PsiInfo* info, cudaStream_t s) {
     const uint64_t np = (uint64_t)(L.nx + 2) * (L.ny + 2) * (L.nz + 2);
-    k_psi<<<grid_for(np, 256), 256, 0, s>>>(L, mags, count, L.e_dyn);
-    k_static_b<<<grid_for(L.n, 256), 256, 0, s>>>(L, L.e_dyn);
+    k_psi<<<grid_for(np, 256), 256, 0, s>>>(L, mags, count, below, L.e_dyn);
+    k_static_b<<<grid_for(L.n, 256), 256, 0, s>>>(L, count, below, info, L.e_dyn);
 }
 
 // static E from charged solids (charge per cell held in B_dyn.x by the voxeliser) into E:

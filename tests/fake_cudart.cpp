@@ -121,6 +121,8 @@ cudaError_t cudaFree(void* p) {
     if (p) { used_memory -= blocks[p]; blocks.erase(p); free(p); }
     return cudaSuccess;
 }
+cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) { *p = calloc(bytes, 1); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *t = total_memory; *f = total_memory - used_memory; return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
