@@ -209,6 +209,7 @@ struct ion_lbm {
     std::unique_ptr<ion::Surrogate> sur;  // learned far field (field_mode SURROGATE)
     ion::FftField fft;         // FAST field as a convolution over the bins; fft.G null: the direct sum
     ion::FieldTable table;     // BITWISE field: R/|R|^3 of the grid; table.T null: the direct sum
+    size_t fft_bytes = 0, table_bytes = 0;
 };
 
 namespace {
@@ -227,11 +228,16 @@ int dmalloc(ion_lbm* h, void** p, size_t bytes) {
 
 size_t ddf_bytes(int ft) { return ft == ION_FP32 ? 4 : 2; }
 
+void drop_table(ion_lbm* h);
+void drop_plan(ion_lbm* h);
+
 void destroy_handle(ion_lbm* h) {
     if (!h) return;
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     for (void* p : h->allocs) cudaFree(p);
+    drop_table(h);
+    drop_plan(h);
     cudaFree(h->psi_ws);
     cudaFreeHost(h->psi_info);
     for (auto& e : h->ev) if (e) cudaEventDestroy(e);
@@ -256,42 +262,84 @@ int launch_stream_collide(ion_lbm* h, uint64_t t) {
     return ION_OK;
 }
 
-// Lays out what a handle's field mode keeps per grid shape, the FAST field's convolution or the
-// BITWISE field's table (once; launches work on the handle's stream and allocates, so it runs
-// when a handle is created or switched to a mode, never inside a step).  Where the device has
-// no memory left for it the direct sum stays.
-int setup_field(ion_lbm* h) {
+// Memory that handles can do without (the FAST field's plan, the BITWISE field's table): at most an
+// eighth of the device in all, and only while another eighth stays free, so that handles whose own
+// buffers need up to 7/8 of the device fit as they would without.  What does not get it runs the
+// direct sum.
+std::atomic<size_t> g_optional{0};
+bool optional_malloc(void** p, size_t bytes) {
+    *p = nullptr;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (g_optional.fetch_add(bytes) + bytes <= total / 8 && bytes + total / 8 <= free_bytes) {
+        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+    }
+    g_optional.fetch_sub(bytes);
+    return false;
+}
+void optional_free(void* p, size_t bytes) {
+    if (!p) return;
+    cudaFree(p);
+    g_optional.fetch_sub(bytes);
+}
+void drop_table(ion_lbm* h) {
+    optional_free(h->table.T, h->table_bytes);
+    h->table = FieldTable{};
+    h->table_bytes = 0;
+}
+void drop_plan(ion_lbm* h) {  // (one allocation, from G on)
+    optional_free(h->fft.G, h->fft_bytes);
+    h->fft = FftField{};
+    h->fft_bytes = 0;
+}
+
+// Lays out what a field mode keeps per grid shape, the FAST field's convolution or the BITWISE
+// field's table (once; launches work on the handle's stream and allocates, so it runs when a
+// handle is created or switched to a mode, never inside a step).  Where the device has no memory
+// to spare for it the direct sum stays.
+int setup_field(ion_lbm* h, int mode) {
     if (!h->cfg.ext_magneto_hydro) return ION_OK;
-    if (h->cfg.field_mode == ION_FIELD_BITWISE && !h->table.T && field_table_fits(h->L)) {
+    if (mode == ION_FIELD_BITWISE) {
+        if (h->table.T || !field_table_fits(h->L)) return ION_OK;
         FieldTable T;
-        if (cudaMalloc((void**)&T.T, field_table_size(h->L, T)) != cudaSuccess) {
-            cudaGetLastError();
-            return ION_OK;
-        }
-        h->allocs.push_back(T.T);
-        CK(launch_field_table(h->L, T, h->stream));
-        g_launches++;
+        const size_t bytes = field_table_size(h->L, T);
+        if (!optional_malloc((void**)&T.T, bytes)) return ION_OK;
         h->table = T;
+        h->table_bytes = bytes;
+        g_launches++;
+        if (const cudaError_t e = launch_field_table(h->L, T, h->stream)) {
+            drop_table(h);
+            return fail(ION_E_CUDA, "field table: %s", cudaGetErrorString(e));
+        }
+        return ION_OK;
     }
     // (SURROGATE handles fall back to the FAST field)
-    if (h->fft.G || h->cfg.field_mode == ION_FIELD_BITWISE || !fft_field_fits(h->L)) return ION_OK;
+    if (h->fft.G || !fft_field_fits(h->L)) return ION_OK;
     FftField F;
-    size_t bytes[4] = {0, 0, 0, 16};
+    size_t bytes[4] = {0, 0, 0, 16}, at[5] = {0, 0, 0, 0, 0};
     fft_field_sizes(h->L, F, &bytes[0], &bytes[1], &bytes[2]);
-    void** const ptr[4] = {(void**)&F.G, (void**)&F.S, (void**)&F.out, (void**)&F.direct};
-    for (int i = 0; i < 4; i++) {
-        if (cudaMalloc(ptr[i], bytes[i]) != cudaSuccess) {
-            cudaGetLastError();
-            while (i-- > 0) cudaFree(*ptr[i]);
-            return ION_OK;
-        }
-    }
-    for (auto* q : ptr) h->allocs.push_back(*q);
+    for (int i = 0; i < 4; i++) at[i + 1] = at[i] + (bytes[i] + 255) / 256 * 256;
+    char* base;
+    if (!optional_malloc((void**)&base, at[4])) return ION_OK;
+    F.G = (float2*)base;
+    F.S = (float2*)(base + at[1]);
+    F.out = (float*)(base + at[2]);
+    F.direct = (uint32_t*)(base + at[3]);
     F.spread = fft_field_spread(h->L);
-    CK(cudaMemsetAsync(F.direct, 0, 16, h->stream));
-    CK(launch_fft_plan(h->L, F, h->stream));
-    g_launches++;
     h->fft = F;
+    h->fft_bytes = at[4];
+    g_launches++;
+    cudaError_t e = cudaMemsetAsync(F.direct, 0, 16, h->stream);
+    if (e == cudaSuccess) e = launch_fft_plan(h->L, F, h->stream);
+    if (e != cudaSuccess) {
+        drop_plan(h);
+        return fail(ION_E_CUDA, "field plan: %s", cudaGetErrorString(e));
+    }
     return ION_OK;
 }
 
@@ -627,12 +675,8 @@ int ion_lbm_create(const ion_config* cfg, ion_lbm** out) {
             return fail(ION_E_CUDA, "upload of LOD centres failed");
         }
     }
-    rc = setup_field(h);
+    rc = setup_field(h, cfg->field_mode);
     if (rc) { destroy_handle(h); return rc; }
-    if (mhd && cudaHostAlloc((void**)&h->psi_info, sizeof(PsiInfo), cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        h->psi_info = nullptr;
-    }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) { destroy_handle(h); return fail(ION_E_CUDA, "create: stream sync failed"); }
     for (auto& e : h->ev) cudaEventCreate(&e);
     *out = h;
@@ -963,6 +1007,10 @@ static int ensure_compaction(ion_lbm* h) {
     rc = dmalloc(h, &p, sizeof(uint32_t) * (size_t)h->L.n);
     if (rc) return rc;
     h->d_list = (uint32_t*)p;
+    if (cudaHostAlloc((void**)&h->psi_info, sizeof(PsiInfo), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        h->psi_info = nullptr;
+    }
     return ION_OK;
 }
 
@@ -1885,7 +1933,13 @@ int ion_lbm_set_field_mode(ion_lbm* h, int mode) {
     }
     h->cfg.field_mode = (uint8_t)mode;
     h->graph_dirty = true;
-    return setup_field(h);
+    const int rc = setup_field(h, mode);
+    if (rc) return rc;
+    if (mode != ION_FIELD_BITWISE && h->table.T) {  // (a batch uses no table; it may use the plan, which stays)
+        CK(cudaStreamSynchronize(h->stream));
+        drop_table(h);
+    }
+    return ION_OK;
 }
 
 // ---- device selection and the FP32 peak probe ---------------------------------

@@ -33,8 +33,7 @@ class Fake:
         g, b, s, d = C.c_uint(), C.c_uint(), C.c_size_t(), C.c_int()
         for i in range(self.lib.fake_launches()):
             name = self.lib.fake_launch(i, C.byref(g), C.byref(b), C.byref(s), C.byref(d)).decode()
-            out.append(dict(name=re.sub(r"^_ZN3ion(?:12_GLOBAL__N_1)?\d+", "", name), grid=g.value, block=b.value,
-                            smem=s.value, device=d.value))
+            out.append(dict(name=re.sub(r"^.*?\d(?=k_)", "", name), grid=g.value, block=b.value, smem=s.value, device=d.value))
         return out
 
     def kernel(self, prefix: str) -> dict:

@@ -144,3 +144,47 @@ def test_d2q9_stencils_do_not_spill():
                 assert int(re.search(r"(\d+) bytes spill stores", log[log.index(name):]).group(1)) == 0, name
     if not found:
         pytest.skip("the stencil was not compiled by the last build")
+
+
+def _fill(fake, mode, depth):
+    """Handles of 64^3 until one does not fit."""
+    out = []
+    try:
+        while len(out) < 64:
+            out.append(_mhd((64, 64, 64), depth, mode))
+    except I.IonError as e:
+        assert e.code == -4
+    return out
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_handles_that_fit_without_field_tables_fit_with_them(fake, mode):  # noqa: F811
+    """Tables and plans take at most an eighth of the device and leave another free: as many handles
+    as 7/8 of it hold are created (with a table each 11 of 14)."""
+    plain = _mhd((64, 64, 64), 2, mode)  # depth 2: neither table nor plan
+    bytes_each = fake.lib.fake_used()
+    plain.close()
+    assert fake.lib.fake_used() == 0
+    fake.lib.fake_memory(1 << 30)
+    for _ in range(2):  # what the first handles gave back serves the next ones
+        handles = _fill(fake, mode, 4)
+        assert len(handles) >= (7 << 27) // bytes_each
+        kernel = "k_field_table" if mode == 0 else "k_fft_plan"
+        assert sum(x["name"].startswith(kernel) for x in fake.launches()) >= 1
+        for h in handles:
+            h.close()
+        assert fake.lib.fake_used() == 0
+        fake.lib.fake_clear()
+
+
+def test_the_table_goes_with_its_mode(fake):  # noqa: F811
+    lbm = _mhd((64, 64, 64), 4, 1)
+    fast = fake.lib.fake_used()
+    lbm.close()
+    lbm = _mhd((64, 64, 64), 4, 0)
+    lbm.set_field_mode(1)
+    assert fake.lib.fake_used() == fast
+    lbm.set_field_mode(0)
+    lbm.initialize()
+    assert fake.kernel("k_update_e_b_table")
+    lbm.close()
