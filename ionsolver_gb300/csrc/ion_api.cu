@@ -1931,10 +1931,10 @@ int ion_lbm_set_field_mode(ion_lbm* h, int mode) {
         int rc = ensure_surrogate(h);
         if (rc) return rc;
     }
+    const int rc = setup_field(h, mode);
+    if (rc) return rc;  // (the mode stays)
     h->cfg.field_mode = (uint8_t)mode;
     h->graph_dirty = true;
-    const int rc = setup_field(h, mode);
-    if (rc) return rc;
     if (mode != ION_FIELD_BITWISE && h->table.T) {  // (a batch uses no table; it may use the plan, which stays)
         CK(cudaStreamSynchronize(h->stream));
         drop_table(h);

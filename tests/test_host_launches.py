@@ -188,3 +188,22 @@ def test_the_table_goes_with_its_mode(fake):  # noqa: F811
     lbm.initialize()
     assert fake.kernel("k_update_e_b_table")
     lbm.close()
+
+
+@pytest.mark.parametrize("before,after,setup,step", [(0, 1, "k_fft_plan", "k_update_e_b_table"), (1, 0, "k_field_table", "k_fft_sum")])
+def test_a_switch_that_failed_leaves_the_mode(fake, before, after, setup, step):  # noqa: F811
+    lbm = _mhd((32, 32, 32), 4, before)
+    lbm.initialize()
+    used = fake.lib.fake_used()
+    fake.fail(setup)
+    with pytest.raises(I.IonError):
+        lbm.set_field_mode(after)
+    assert fake.lib.fake_used() == used
+    fake.lib.fake_clear()
+    lbm.do_time_step()
+    assert fake.kernel(step)
+    lbm.set_field_mode(after)
+    fake.lib.fake_clear()
+    lbm.do_time_step()
+    assert not any(x["name"].startswith(step) for x in fake.launches())
+    lbm.close()
