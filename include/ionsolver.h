@@ -354,7 +354,8 @@ int ion_batch_finish(ion_batch* b, int timeout_ms);
  * used: the phases of a step are launches of their own, no grid barrier waits */
 #define ION_BARRIER_LIMIT_DEFAULT 67108864u
 int ion_batch_set_wait_limits(ion_batch* b, uint32_t barrier_polls, uint32_t tile_polls);
-/* autotuner record i (block, grid, ms per step); i = 0xFFFFFFFF: the chosen shape */
+/* autotuner record i (block, grid, ms per step); i = 0xFFFFFFFF: the chosen shape.
+ * No records where every domain's FAST field is a convolution: nothing to tune */
 int ion_batch_tuning(ion_batch* b, uint32_t i, uint32_t* block, uint32_t* grid, float* ms_per_step);
 int ion_batch_record_event(ion_batch* b, int slot);
 int ion_batch_event_elapsed(ion_batch* b, int start, int end, float* ms);

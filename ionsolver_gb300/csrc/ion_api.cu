@@ -1660,8 +1660,15 @@ int ion_batch_destroy(ion_batch* b) {
 // Autotuner: on the first run every launch shape (threads per block x blocks
 // per SM that fit on the SM) advances the batch by two real steps, timed with
 // CUDA events; the fastest shape is kept.  Results do not depend on the shape,
-// so the tuning steps are ordinary steps of the simulation.
+// so the tuning steps are ordinary steps of the simulation.  (The shape is that of the direct field sums'
+// launch; without one there is nothing to tune.)
 static int batch_autotune(ion_batch* b, uint64_t& steps) {
+    if (b->mhd && b->total_bricks[0] == 0u) {  // every field is a convolution: no launch has this shape
+        b->block = 256;
+        b->grid = 2u * (uint32_t)b->sms;
+        b->tuned = true;
+        return ION_OK;
+    }
     float best = 1e30f;
     for (uint32_t block : kBatchBlocks) {
         const int maxb = batch_max_blocks_per_sm(b->ft, b->mhd, b->fast, b->total_rows > 0u, (int)block);

@@ -207,3 +207,16 @@ def test_a_switch_that_failed_leaves_the_mode(fake, before, after, setup, step):
     lbm.do_time_step()
     assert not any(x["name"].startswith(step) for x in fake.launches())
     lbm.close()
+
+
+@pytest.mark.parametrize("depth,tuned", [(2, True), (4, False)])
+def test_batch_tunes_only_what_it_launches(fake, depth, tuned):  # noqa: F811
+    """The shape that the autotuner tries is the direct field sums'; where every field is a convolution
+    it timed the same launches several times and reported one of them."""
+    doms = [_mhd((32, 32, 32), depth, 1) for _ in range(2)]
+    b = I.Batch(doms)
+    b.run(40)
+    assert bool(b.tuning()) == tuned and b.chosen()[0] in (128, 256)
+    b.close()
+    for d in doms:
+        d.close()
