@@ -68,8 +68,8 @@ __constant__ float2 c_tw[32] = {  // exp(2 pi i j / 32)
 template <int ND>
 __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField F) {
     constexpr int M = 2 * ND, ROW = M + 1;
-    __shared__ C2<float> a[3 * M * ROW];  // [component][mz][my], rows of M + 1
-    __shared__ C2<float> tw[M];
+    __shared__ C2 a[3 * M * ROW];  // [component][mz][my], rows of M + 1
+    __shared__ C2 tw[M];
     const uint32_t kx = blockIdx.x % (ND + 1u), u = blockIdx.x / (ND + 1u);
     const uint32_t ox = u % F.ux, oy = (u / F.ux) % F.uy, oz = u / (F.ux * F.uy);
     if (threadIdx.x < M) {
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
     const float sx = ox - 0.5f * bx, sy = oy - 0.5f * by, sz = oz - 0.5f * bz;
     for (int t = threadIdx.x; t < M * M; t += blockDim.x) {
         const int my = t % M, mz = t / M;
-        C2<float> g[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+        C2 g[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
         if (my != ND && mz != ND) {
             const float ry = by * (my < ND ? my : my - M) + sy, rz = bz * (mz < ND ? mz : mz - M) + sz;
             for (int mx = 0; mx < M; mx++) {
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
                 const float rx = bx * (mx < ND ? mx : mx - M) + sx;
                 const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
                 const float i3 = 1.0f / (r2 * sqrtf(r2));
-                const C2<float> w = tw[mx];
+                const C2 w = tw[mx];
                 const float vx = rx * i3, vy = ry * i3, vz = rz * i3;
                 g[0] = {fmaf(vx, w.x, g[0].x), fmaf(vx, w.y, g[0].y)};
                 g[1] = {fmaf(vy, w.x, g[1].x), fmaf(vy, w.y, g[1].y)};
@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
     }
     __syncthreads();
     if (threadIdx.x < 3u * M) {  // along y, a row per thread
-        C2<float>* row = a + threadIdx.x * ROW;
-        C2<float> v[M];
+        C2* row = a + threadIdx.x * ROW;
+        C2 v[M];
 #pragma unroll
         for (int k = 0; k < M; k++) v[k] = row[k];
         fft_regs<M, -1>(v);
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
     __syncthreads();
     if (threadIdx.x < 3u * M) {  // along z, a column per thread
         const int c = threadIdx.x / M, ky = threadIdx.x % M;
-        C2<float> v[M];
+        C2 v[M];
 #pragma unroll
         for (int k = 0; k < M; k++) v[k] = a[(c * M + k) * ROW + ky];
         fft_regs<M, -1>(v);
@@ -263,10 +263,10 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
 // ---------------------------------------------------------------------------
 // the sums of one offset: block = (((oz - oz0) bsy + oy) bsx + ox) 6 + (0..2: E, 3..5: B)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ C2<float> cmul(const float2 a, const float2 b) {
+__device__ __forceinline__ C2 cmul(const float2 a, const float2 b) {
     return {fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x)};
 }
-__device__ __forceinline__ C2<float> cmul_sub(const C2<float> s, const float2 a, const float2 b) {
+__device__ __forceinline__ C2 cmul_sub(const C2 s, const float2 a, const float2 b) {
     return {fmaf(-a.x, b.x, fmaf(a.y, b.y, s.x)), fmaf(-a.x, b.y, fmaf(-a.y, b.x, s.y))};
 }
 
@@ -277,14 +277,14 @@ __device__ __forceinline__ C2<float> cmul_sub(const C2<float> s, const float2 a,
 // exchange, fused into the additions of half as many points (k_fft_sum at 128^3 121 -> 111 us
 // against turning the upper lane's points before it, which leaves the lower lane waiting).
 template <int N>
-__device__ __forceinline__ void fft_pair(C2<float> (&v)[N], const bool upper) {
+__device__ __forceinline__ void fft_pair(C2 (&v)[N], const bool upper) {
     fft_regs<N, 1, true>(v, upper ? -1.0f : 1.0f);
 #pragma unroll
     for (int n = 0; n < N / 2; n++) {  // even + w^n odd; w^(N/2) = i
-        const C2<float> own = v[n], got = {__shfl_xor_sync(0xFFFFFFFFu, v[n + N / 2].x, 16),
+        const C2 own = v[n], got = {__shfl_xor_sync(0xFFFFFFFFu, v[n + N / 2].x, 16),
                                            __shfl_xor_sync(0xFFFFFFFFu, v[n + N / 2].y, 16)};
-        const C2<float> even = {upper ? got.x : own.x, upper ? got.y : own.y};
-        const C2<float> odd = {upper ? -own.y : got.x, upper ? own.x : got.y};
+        const C2 even = {upper ? got.x : own.x, upper ? got.y : own.y};
+        const C2 odd = {upper ? -own.y : got.x, upper ? own.x : got.y};
         v[n] = add_twist<1>(even, odd, n * (16 / N));
     }
 }
@@ -310,7 +310,7 @@ __device__ __forceinline__ void fft_sum(const DevLbm& L, const FftField& F, cons
     const float2* const G = F.G + (size_t)u * (ND + 1u) * 3u * M * M + gy;
     const float2* const S = F.S + par * M + ky;
     auto flip = [](float v, uint32_t m) { return __uint_as_float(__float_as_uint(v) ^ m); };
-    auto gather = [&](uint32_t kx, C2<float>(&v)[ND], auto&& put) {
+    auto gather = [&](uint32_t kx, C2(&v)[ND], auto&& put) {
         const float2* g = G + (size_t)kx * 3u * M * M;
         const float2* s = S + (size_t)kx * 4u * M * M;
         // kz = 2 k + par, or M - kz; the row's address is formed at each load (an opaque step:
@@ -342,10 +342,10 @@ __device__ __forceinline__ void fft_sum(const DevLbm& L, const FftField& F, cons
 #pragma unroll 1
     for (uint32_t p0 = 0; p0 < (uint32_t)ND; p0 += PL) {
         float2* stage = sm + p0 * SLOT;  // [plane][z][ky], rows of M + 1
-        C2<float> v[ND];
-        gather(p0 + pl, v, [](C2<float>& d, const C2<float> p) { d = p; });
+        C2 v[ND];
+        gather(p0 + pl, v, [](C2& d, const C2 p) { d = p; });
         // the transforms of kx = 0 and kx = nd are real: one complex line holds both
-        if (p0 + pl == 0u) gather(ND, v, [](C2<float>& d, const C2<float> p) { d = {d.x - p.y, d.y + p.x}; });
+        if (p0 + pl == 0u) gather(ND, v, [](C2& d, const C2 p) { d = {d.x - p.y, d.y + p.x}; });
         fft_pair<ND>(v, par != 0u);
         float2* w = stage + (pl * ND + par * (ND / 2u)) * ROW + ky;
 #pragma unroll
@@ -374,13 +374,13 @@ __device__ __forceinline__ void fft_sum(const DevLbm& L, const FftField& F, cons
     for (uint32_t line = t; line < SLOT; line += SUM_THREADS) {
         const uint32_t y = line % ND, z = line / ND;
         const float2* r = sm + z * ND + (y + z) % ND;
-        C2<float> v[ND];
+        C2 v[ND];
         v[0] = {r[0].x + r[0].y, r[0].x - r[0].y};
 #pragma unroll
         for (uint32_t k = 1; k <= (uint32_t)ND / 2u; k++) {
             const float2 p = r[k * SLOT], q = r[(ND - k) * SLOT];
-            const C2<float> sum = {p.x + q.x, p.y - q.y}, dif = {p.x - q.x, p.y + q.y};
-            const C2<float> a = twist<1>(dif, k * (16 / ND) + 8);  // i w^k dif
+            const C2 sum = {p.x + q.x, p.y - q.y}, dif = {p.x - q.x, p.y + q.y};
+            const C2 a = twist<1>(dif, k * (16 / ND) + 8);  // i w^k dif
             v[k] = {sum.x + a.x, sum.y + a.y};
             // k -> h - k: sum -> conj sum, dif -> -conj dif, i w^k -> conj (i w^k)
             if (2u * k < (uint32_t)ND) v[ND - k] = {sum.x - a.x, a.y - sum.y};
