@@ -232,7 +232,7 @@ static __global__ void __launch_bounds__(256, 2) k_batch_field_gated(const Batch
     __shared__ DevLbm sL;
     __shared__ uint32_t s_dom, s_gate;
     int any = 0;
-    for (uint32_t d = threadIdx.x; d < B.ndom; d += blockDim.x) any |= gates[d] != nullptr && any_of(gates[d]);
+    for (uint32_t d = threadIdx.x; d < B.ndom; d += blockDim.x) any |= gates[d] != nullptr && field_direct(gates[d]);
     if (!__syncthreads_or(any)) return;
     eb_init(sm);
     uint32_t uses[2] = {0u, 0u};
@@ -240,7 +240,7 @@ static __global__ void __launch_bounds__(256, 2) k_batch_field_gated(const Batch
         __syncthreads();
         if (threadIdx.x == 0) {
             s_dom = find_domain(B.brick_off, B.ndom, t);
-            s_gate = any_of(gates[s_dom]);
+            s_gate = field_direct(gates[s_dom]);
             if (s_gate) sL = B.doms[s_dom];
         }
         __syncthreads();

@@ -12,8 +12,8 @@
 //   k_fft_plan  once per grid shape: spectra of R/|R|^3.  An offset o and its mirror image b - o have spectra
 //               that differ by the sign of a wave number and of a component, so
 //               (b/2 + 1) of b offsets per axis are kept.
-//   k_fft_src   spectra of the sources, 4 (nd + 1) blocks; block 0 also looks at the range
-//               of the sources (see below).
+//   k_fft_src   spectra of the sources, 4 (nd + 1) blocks; the four of kx = 0 also look at the
+//               range and the spread of the sources (see below).
 //   k_fft_sum   one block per offset and component of E or B: product of spectra, then the
 //               inverse transforms along z, y and x in registers, passed on through
 //               shared memory.
@@ -29,6 +29,7 @@
 // sign, or whose largest value lies outside [1e-28, 1e25], where sums could over- or underflow (a
 // NaN charge leaves NaN in every cell either way).
 #include <algorithm>
+#include <cmath>
 
 #include "field_fft.h"
 #include "fft_regs.cuh"
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(256) k_fft_plan(const DevLbm L, const FftField
 // long as wide lie lower, eight times as long below the line.  F.spread holds the square of the
 // line times kappa.  (All of it in fixed order: a batch decides as its domains do alone.)
 template <int ND>
-__device__ __forceinline__ bool concentrated(const DevLbm& L, const FftField& F, const float* s, const float scale) {
+__device__ __forceinline__ bool concentrated(const DevLbm& L, const FftField& F, const float* s, const float scale, float& norm) {
     constexpr uint32_t G = ND / 4;  // bins a group and axis
     __shared__ float s_sum[64], s_sq[64], s_inv[64];
     __shared__ uint32_t s_min;
@@ -181,6 +182,7 @@ __device__ __forceinline__ bool concentrated(const DevLbm& L, const FftField& F,
     if (sub == 0u) atomicMin(&s_min, __float_as_uint(a));  // (in any order; a >= 0)
     __syncthreads();
     const float least = __uint_as_float(s_min);
+    norm = sqrtf(q);
     return least * least < F.spread * q;
 }
 
@@ -214,11 +216,18 @@ __device__ __forceinline__ void fft_src(const DevLbm& L, const FftField& F, cons
     __syncthreads();
     if (kx == 0u) {  // the component's block decides for it
         const uint32_t v = s_max[1];
-        bool bad = false;
-        if (s_max[0] <= 0x7F800000u && v != 0u)  // a NaN charge makes every cell's E and B NaN either way
-            bad = !(v >= __float_as_uint(1e-28f) && v <= __float_as_uint(1e25f)) ||
-                  concentrated<ND>(L, F, s, __uint_as_float(0x7E800000u - (v & 0x7F800000u)));
-        if (threadIdx.x == 0u) F.direct[c] = bad;
+        const float scale = __uint_as_float(0x7E800000u - (v & 0x7F800000u));
+        bool bad = false, few = false;
+        float norm = 0.0f;
+        if (s_max[0] <= 0x7F800000u && v != 0u) {  // a NaN charge makes every cell's E and B NaN either way
+            bad = !(v >= __float_as_uint(1e-28f) && v <= __float_as_uint(1e25f));
+            if (!bad) few = concentrated<ND>(L, F, s, scale, norm);
+        }
+        if (threadIdx.x == 0u) {
+            F.direct[c] = bad || (few && c == 0u);
+            if (c == 0u) F.direct[FFT_LATE] = 0u;
+            else F.noise[c] = few ? F.kappa * (norm / scale) : 0.0f;
+        }
     }
     // along x at this kx
     for (uint32_t t = threadIdx.x; t < ND * ND; t += SRC_THREADS) {
@@ -434,6 +443,9 @@ __device__ __forceinline__ void fft_put(const DevLbm& L, const FftField& F, uint
     const float* const stat = B ? L.b_stat : L.e_stat;
     float* const dyn = B ? L.b_dyn : L.e_dyn;
     const float scale = B ? L.kmu : L.ke;
+    const float noise = B ? F.noise[1] + F.noise[2] + F.noise[3] : 0.0f;
+    const float least = 256.0f * fabsf(L.kmu) * noise;
+    uint32_t small = noise > 0.0f ? (1u << PUT) - 1u : 0u;  // bit k: cell k's B is not above that so far
     bool on[PUT];
 #pragma unroll
     for (uint32_t k = 0; k < PUT; k++) on[k] = e < plane_xy && (L.flags[n0 + k * row] & F_BO) != F_S;
@@ -449,8 +461,15 @@ __device__ __forceinline__ void fft_put(const DevLbm& L, const FftField& F, uint
         for (uint32_t k = 0; k < PUT; k++) st[k] = on[k] ? stat[c * N + n0 + k * row] : 0.0f;
 #pragma unroll
         for (uint32_t k = 0; k < PUT; k++)
-            if (on[k]) dyn[c * N + n0 + k * row] = st[k] + scale * s[c][y0 + k * YS][xl];
+            if (on[k]) {
+                const float r = st[k] + scale * s[c][y0 + k * YS][xl];
+                dyn[c * N + n0 + k * row] = r;
+                if (fabsf(r) > least) small &= ~(1u << k);
+            } else {
+                small &= ~(1u << k);
+            }
     }
+    if (small) atomicOr(F.direct + FFT_LATE, 1u);
 }
 
 // gate: null, or the kernels run only when *gate != 0.  Then resident blocks walk the work, so
@@ -599,7 +618,7 @@ void fft_field_sizes(const DevLbm& L, FftField& F, size_t* g_bytes, size_t* s_by
 
 // The line of `concentrated`: (4 kappa)^2 or (2.75 kappa)^2.  kappa^2 is taken over the bins up to
 // four apart (1/|R|^4 falls fast) and up to four offsets an axis.
-float fft_field_spread(const DevLbm& L) {
+void fft_field_spread(const DevLbm& L, FftField& F) {
     const uint32_t bs[3] = {L.bsx, L.bsy, L.bsz};
     double r2[3][4][9], sum = 0.0;  // squares along an axis, [offset][difference of the bins]
     for (int a = 0; a < 3; a++)
@@ -614,8 +633,9 @@ float fft_field_spread(const DevLbm& L) {
             const double r = r2[0][o % 4][d % 9] + r2[1][o / 4 % 4][d / 9 % 9] + r2[2][o / 16][d / 81];
             sum += 1.0 / (r * r);
         }
-    const double M = 2.0 * L.nd, line = L.nd == 16u ? 4.0 : 2.75;
-    return (float)(line * line * sum / (64.0 * M * M * M));
+    const double M = 2.0 * L.nd, line = L.nd == 16u ? 4.0 : 2.75, k2 = sum / (64.0 * M * M * M);
+    F.kappa = (float)std::sqrt(k2);
+    F.spread = (float)(line * line * k2);
 }
 
 cudaError_t launch_fft_plan(const DevLbm& L, const FftField& F, cudaStream_t s) {

@@ -8,16 +8,20 @@ namespace ion {
 
 struct DevLbm;
 
+// FftField::direct: a word per component, known before the sums, and the word that the last kernel sets
+constexpr uint32_t FFT_LATE = 4;
+
 // What one domain keeps for the convolution (device memory, laid out once per grid shape):
 // the spectra of R/|R|^3 for every distinct offset of a cell inside its bin.
 struct FftField {
     float2* G = nullptr;       // [uz][uy][ux][kx = 0..nd][component][kz][ky]
     float2* S = nullptr;       // [kx = 0..nd][q, q vx, q vy, q vz][kz][ky], of the present step
     float* out = nullptr;      // [6][oz of a chunk][oy][ox][Ix][Iz][Iy]: the sums, before they go to the cells
-    uint32_t* direct = nullptr;  // [4], one non-zero: the sources' range or spread asks for the direct sum
+    uint32_t* direct = nullptr;  // [FFT_LATE + 1], one non-zero: the sources' range or spread asks for the direct sum
+    float* noise = nullptr;    // [4], from [1]: rounding of a concentrated current (0: it is spread out)
     uint32_t ux = 0, uy = 0, uz = 0;  // distinct offsets per axis: bin edge / 2 + 1
     uint32_t chunk = 0;        // in-bin z offsets whose sums fit in `out`
-    float spread = 0.0f;       // how spread out the sources have to be (field_fft.cu, concentrated)
+    float spread = 0.0f, kappa = 0.0f;  // how spread out the sources have to be (field_fft.cu, concentrated)
 };
 
 // bytes of the sums that are held at once (a few in-bin z offsets of a large grid)
@@ -26,10 +30,10 @@ constexpr size_t FFT_OUT_BYTES = 48ull << 20;
 // whether a domain's FAST field runs as the convolution, and its sizes in bytes
 bool fft_field_fits(const DevLbm& L);
 void fft_field_sizes(const DevLbm& L, FftField& F, size_t* g_bytes, size_t* s_bytes, size_t* out_bytes);
-float fft_field_spread(const DevLbm& L);
+void fft_field_spread(const DevLbm& L, FftField& F);
 cudaError_t launch_fft_plan(const DevLbm& L, const FftField& F, cudaStream_t s);
 // sources -> spectra, sums of every cell, E/B; returns the number of launches.  F.direct is
-// left with a non-zero word (and E/B untouched) when the direct sum has to run instead.  gate: null, or
+// left with a non-zero word when the direct sum has to run instead, over all of E and B.  gate: null, or
 // nothing runs while *gate is 0.
 uint32_t launch_fft_field(const DevLbm& L, const FftField& F, const uint32_t* gate, cudaStream_t s);
 

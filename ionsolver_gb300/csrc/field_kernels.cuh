@@ -599,7 +599,7 @@ __device__ __forceinline__ bool eb_tile(const DevLbm& L, const uint32_t brick, c
 // 7.3 us at 192^3)
 static __global__ void __launch_bounds__(256, 2) k_update_e_b_gated(const DevLbm L, uint32_t* err, const uint32_t* gate,
                                                                     const uint32_t* direct, const uint32_t bricks) {
-    if ((gate && *gate == 0u) || (direct && !any_of(direct))) return;
+    if ((gate && *gate == 0u) || (direct && !field_direct(direct))) return;
     __shared__ __align__(16) EbSmem<true> sm;
     eb_init(sm);
     uint32_t uses[2] = {0u, 0u};

@@ -321,7 +321,7 @@ int setup_field(ion_lbm* h, int mode) {
     // (SURROGATE handles fall back to the FAST field)
     if (h->fft.G || !fft_field_fits(h->L)) return ION_OK;
     FftField F;
-    size_t bytes[4] = {0, 0, 0, 16}, at[5] = {0, 0, 0, 0, 0};
+    size_t bytes[4] = {0, 0, 0, 64}, at[5] = {0, 0, 0, 0, 0};
     fft_field_sizes(h->L, F, &bytes[0], &bytes[1], &bytes[2]);
     for (int i = 0; i < 4; i++) at[i + 1] = at[i] + (bytes[i] + 255) / 256 * 256;
     char* base;
@@ -330,11 +330,12 @@ int setup_field(ion_lbm* h, int mode) {
     F.S = (float2*)(base + at[1]);
     F.out = (float*)(base + at[2]);
     F.direct = (uint32_t*)(base + at[3]);
-    F.spread = fft_field_spread(h->L);
+    F.noise = (float*)(F.direct + 8);
+    fft_field_spread(h->L, F);
     h->fft = F;
     h->fft_bytes = at[4];
     g_launches++;
-    cudaError_t e = cudaMemsetAsync(F.direct, 0, 16, h->stream);
+    cudaError_t e = cudaMemsetAsync(F.direct, 0, bytes[3], h->stream);
     if (e == cudaSuccess) e = launch_fft_plan(h->L, F, h->stream);
     if (e != cudaSuccess) {
         drop_plan(h);

@@ -149,6 +149,8 @@ __device__ __forceinline__ bool any_of(const uint32_t* w) {
     const uint4 v = *reinterpret_cast<const uint4*>(w);
     return (v.x | v.y | v.z | v.w) != 0u;
 }
+// whether the convolution left a field to the direct sum (FftField::direct)
+__device__ __forceinline__ bool field_direct(const uint32_t* w) { return any_of(w) || w[4] != 0u; }
 
 // Packed FP32 pairs (PTX add/sub/mul/fma .f32x2, sm_100 and later): one
 // instruction does the same IEEE round-to-nearest operation on the two halves
