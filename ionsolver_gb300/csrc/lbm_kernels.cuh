@@ -799,7 +799,8 @@ __host__ __device__ constexpr int ws_min_ctas() {
 template <int FT, bool MHD, bool TRT, uint32_t RS>
 __global__ void __launch_bounds__(ws_bound<FT, RS, MHD, TRT>(), ws_min_ctas<FT, RS, MHD, TRT>()) k_sc_rows_ws(const DevLbm L, const uint32_t odd_k, uint32_t* err) {
     using T = typename Ddf<FT>::T;
-    const uint32_t odd_t = odd_k & 1u, K = odd_k >> 1;  // parity of the step, rows a group (an argument of its own: FP16C with TRT 2.4% slower)
+    // parity of the step, rows a group (as an argument of its own FP16C with TRT was 2.4% slower)
+    const uint32_t odd_t = odd_k & 1u, K = odd_k >> 1;
     constexpr uint32_t RB = ws_row_bytes<FT, MHD, RS>();
     constexpr uint32_t SB = RS * (uint32_t)sizeof(T);  // bytes per stream row
     constexpr uint32_t eb_off = row_streams<FT, MHD>() * SB, fl_off = eb_off + (MHD ? 6u * RS * 4u : 0u);
@@ -908,10 +909,11 @@ struct RowPlan {
     int per_sm;           // 0: the rows do not fit
 };
 
-// The smallest stride that holds a row, with as many rows a group as the resident blocks leave it (a
-// group's copies are issued by one thread, row by row where a neighbour row wraps around: with six
-// rows a group 16^3 took 8.3 us plain and 16.5 us with MHD, with one 5.2 and 10.4; 16x96x96 with
-// one 15.4 and 39.0 us, with four or six 9.4 to 12.3 and 24.8 to 28.8).  Or, but for FP32 with
+// The smallest stride that holds a row, with as many rows a group as leave half the resident blocks
+// one (a group's copies are issued by one thread, row by row where a neighbour row wraps around:
+// with six rows a group 16^3 took 8.3 us plain and 16.5 us with MHD, with one 5.2 and 10.4;
+// 16x96x96 with one 15.4 and 39.0 us, with four or six 9.4 to 12.3 and 24.8 to 28.8.  With all resident
+// blocks instead of half, 16x44x44 and 32x44x44 took 7.2 us instead of 6.2).  Or, but for FP32 with
 // MHD, a wider stride that stages several short rows at a time: the one thread that issues the
 // copies then has fewer, longer ones.  It is taken where it keeps at least 5% more cells on an SM and the
 // groups still feed every resident block at least twice.  The smallest stride against the
@@ -936,7 +938,8 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
     RowPlan best{device, L.nx, L.ny, L.nz, 0, 0u, 0u, 0u, 0};
     failed = false;
     const bool ws = L.nx <= WS_ROW;  // producer warp + one cell per thread and row
-    const bool bounded = FT == ION_FP32 && (MHD || !TRT) && L.nx >= 96u && (uint64_t)L.n * ((MHD ? 45u : 19u) * 4u) > 96ull << 20;  // (L2: 129 MB)
+    const bool bounded = FT == ION_FP32 && (MHD || !TRT) && L.nx >= 96u &&
+                         (uint64_t)L.n * ((MHD ? 45u : 19u) * 4u) > 96ull << 20;  // (L2: 129 MB)
     for (int v = ws ? 0 : 5; v < 6; v++) {
         RowPlan p = best;
         p.v = v;
@@ -966,9 +969,9 @@ RowPlan make_row_plan(const DevLbm& L, int device, int sms, bool& failed) {
         };
         occupancy();
         if (v < 5 && best.per_sm == 0 && p.per_sm > 0 && ws_rows(v) / L.nx > 1u) {
-            // more rows a group only where a row each would give the resident blocks more than one
-            const uint32_t resident = (uint32_t)(p.per_sm * sms);
-            set_rows(std::min(ws_rows(v) / L.nx, (L.ny * L.nz + resident - 1u) / resident));
+            // more rows a group only where a row each would fill more than half the resident blocks
+            const uint32_t half = std::max(1u, (uint32_t)(p.per_sm * sms) / 2u);
+            set_rows(std::min(ws_rows(v) / L.nx, (L.ny * L.nz + half - 1u) / half));
             occupancy();
         }
         if (p.per_sm < 1) continue;

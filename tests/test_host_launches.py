@@ -105,6 +105,16 @@ def test_many_short_rows_are_staged_in_groups(fake):  # noqa: F811
     lbm.close()
 
 
+@pytest.mark.parametrize("shape", [(16, 44, 44), (32, 44, 44), (32, 52, 33)])
+def test_rows_that_would_fill_the_resident_blocks_are_staged_in_pairs(fake, shape):  # noqa: F811
+    """A row each would take more than half the resident blocks (32x44x44: 7.2 us instead of 6.2)."""
+    lbm = _plain(shape)
+    lbm.do_time_step()
+    k = fake.kernel("k_sc_rows_ws")
+    assert k["block"] == 2 * shape[0] + 32 and k["grid"] == (shape[1] + 1) // 2 * shape[2]
+    lbm.close()
+
+
 @pytest.mark.parametrize("shape,mhd,blocks", [((160, 128, 128), False, 4), ((224, 128, 128), False, 3), ((128, 128, 128), False, 5),
                                               ((160, 64, 64), False, 5), ((96, 96, 96), True, 4)])
 def test_fp32_rows_beyond_l2_are_staged_on_fewer_blocks(fake, shape, mhd, blocks):  # noqa: F811
