@@ -343,7 +343,8 @@ typedef struct ion_batch ion_batch;
 int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out);
 int ion_batch_destroy(ion_batch* b);
 /* Advances every domain by `steps`.  The first call autotunes the launch
- * shape on its first steps (each candidate shape runs two real steps) and
+ * shape on its first steps (each candidate shape runs two real steps; not
+ * where every domain's FAST field is a convolution) and
  * then replays a CUDA graph of two steps. Asynchronous. */
 int ion_batch_run(ion_batch* b, uint64_t steps);
 /* bounded wait for the batch's stream; reports device-side timeouts */

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(BATCH_SC_THREADS, MHD ? 3 : 4) k_batch_stream(
 // Phase A over x-rows, when every domain's rows are whole 16-byte streams of
 // at most BATCH_ROW_MAX cells: the producer-warp form of k_sc_rows_ws (lbm_kernels.cuh)
 // walking the rows of all domains (global row g = blockIdx.x + k gridDim.x, its domain by
-// binary search over the prefix sums of ny nz).  The last warp stages each row and writes
+// binary search over the prefix sums of the domains' groups of rows).  The last warp stages each row and writes
 // the new DDFs back from the staged rows; the others run sc_cell on the row's cells (one
 // per thread).  A row's domain view is copied into the buffer's shared-memory slot when it
 // changes.  Per cell it runs sc_cell exactly as the single-domain row kernel does, so the

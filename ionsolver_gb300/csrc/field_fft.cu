@@ -49,7 +49,7 @@ __host__ __device__ constexpr uint32_t sum_smem(uint32_t nd) { return ((nd - pla
 static_assert(planes(16) * slot_elems(16) <= stage_elems(16) && planes(8) * slot_elems(8) <= stage_elems(8),
               "the last planes' slots lie inside the staging area");
 constexpr uint32_t SUM_THREADS = 128, SRC_THREADS = 512, PUT_THREADS = 256, PUT_X = 128;
-// k_fft_sum's blocks per SM: 96 registers at nd = 16 (with six it spills, 122 -> 155 us at 128^3),
+// k_fft_sum's blocks per SM: 96 registers at nd = 16 (with six it spills, 111 -> 148 us at 128^3),
 // half the line at nd = 8
 __host__ __device__ constexpr int sum_blocks(int nd) { return nd == 16 ? 5 : 8; }
 

@@ -17,11 +17,12 @@ struct FftField {
     float2* G = nullptr;       // [uz][uy][ux][kx = 0..nd][component][kz][ky]
     float2* S = nullptr;       // [kx = 0..nd][q, q vx, q vy, q vz][kz][ky], of the present step
     float* out = nullptr;      // [6][oz of a chunk][oy][ox][Ix][Iz][Iy]: the sums, before they go to the cells
-    uint32_t* direct = nullptr;  // [FFT_LATE + 1], one non-zero: the sources' range or spread asks for the direct sum
+    uint32_t* direct = nullptr;  // [FFT_LATE + 1], one non-zero: the sources ask for the direct sum
     float* noise = nullptr;    // [4], from [1]: rounding of a concentrated current (0: it is spread out)
     uint32_t ux = 0, uy = 0, uz = 0;  // distinct offsets per axis: bin edge / 2 + 1
     uint32_t chunk = 0;        // in-bin z offsets whose sums fit in `out`
-    float spread = 0.0f, kappa = 0.0f;  // how spread out the sources have to be (field_fft.cu, concentrated)
+    float spread = 0.0f;       // how spread out the sources have to be (field_fft.cu, concentrated)
+    float kappa = 0.0f;        // root of the mean of 1/|R|^4 on the padded lattice
 };
 
 // bytes of the sums that are held at once (a few in-bin z offsets of a large grid)

@@ -17,7 +17,7 @@
 // of source bins every step needs one new table entry, the others move on by a cell: R + nd - 1
 // entries per row of nd sources and R cells.  Lanes are neighbouring offsets (coalesced table
 // rows, one broadcast source), the warps of a block the R-groups of the same offsets, whose
-// entries overlap in L1.  Bound by FP32 issue: 21 of 22 instructions per term (R = 4).
+// entries overlap in L1.  Bound by FP32 issue: 22.6 instructions per term, of which 21 are its operations (R = 4).
 #include "field_table.h"
 #include "ion_device.cuh"
 #include "ion_launch.h"

@@ -1596,7 +1596,7 @@ int ion_batch_create(ion_lbm* const* domains, uint32_t count, ion_batch** out) {
         b->allocs.push_back(*p);
         return ION_OK;
     };
-    // a domain takes the path of its own steps
+    // FAST: a domain takes the path of its own steps (BITWISE domains take the direct sum)
     auto convolved = [&](uint32_t i) { return b->fast && domains[i]->fft.G != nullptr; };
     std::vector<DevLbm> views(count);
     std::vector<uint32_t> bins(count + 1, 0);

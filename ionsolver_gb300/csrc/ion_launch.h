@@ -104,7 +104,8 @@ ION_DECLARE_LBM_DISPATCH(q9)
 void launch_lod_bins(const DevLbm& L, cudaStream_t s);
 void launch_update_e_b(const DevLbm& L, bool fast, uint32_t* err, cudaStream_t s);
 void launch_div_check(uint64_t samples, uint64_t seed, unsigned long long* bad, float* first_bad, cudaStream_t s);
-// gate: null, or nothing runs while *gate is 0; direct: null, or FftField::direct, nothing runs while all its words are 0
+// gate: null, or nothing runs while *gate is 0; direct: null, or FftField::direct, nothing runs while
+// all its words are 0
 void launch_update_e_b_gated(const DevLbm& L, uint32_t* err, const uint32_t* gate, const uint32_t* direct, cudaStream_t s);
 void launch_voxelize(const DevLbm& L, const VoxArgs& A, cudaStream_t s);
 void launch_compact(const DevLbm& L, uint8_t mask, uint32_t* tiles, uint32_t* list, uint32_t* total, cudaStream_t s);
