@@ -12,6 +12,7 @@ import pytest
 
 import ionsolver_gb300 as I
 from ionsolver_gb300 import workloads as W
+from tests import _util as U
 
 pytestmark = pytest.mark.gpu
 SCALE = np.float32(2.0 ** 90)
@@ -81,3 +82,37 @@ def test_a_current_below_the_rounding_of_b_keeps_the_convolution(shape, depth):
         b_stat[:, 0] = 0.0
         e, b, direct = _fields(lbm, q, v, b_stat)
         assert np.array_equal(e, direct)
+
+
+def _moving_cluster(shape, depth):
+    """Charge everywhere, a few cells that move, no static field."""
+    case = W.mhd_plasma(shape=shape, depth=depth, field_mode=1)
+    case["meshes"], case["precompute_b"] = [], False
+    nx, ny, nz = shape
+    u = np.zeros((3, nz, ny, nx), np.float32)
+    u[0, nz // 2:nz // 2 + 2, ny // 2:ny // 2 + 2, nx - 6:nx - 4] = 1e-3
+    case["fields"]["u"] = u.reshape(-1)
+    return case
+
+
+@pytest.mark.parametrize("shapes", [[((48, 32, 48), 4), ((40, 24, 32), 3)], [((32, 32, 32), 4)]])
+def test_batch_takes_the_direct_sum_as_its_domains_do(shapes):
+    cases = [_moving_cluster(*s) for s in shapes] + [W.mhd_plasma(shape=(32, 32, 32), depth=3, field_mode=1)]
+    steps = 2
+    solo = [U.run_gpu(c, steps) for c in cases]
+    for (shape, depth), s in zip(shapes, solo):
+        first = sum(8 ** k for k in range(depth))
+        lod = s.read("qu_lod").reshape(-1, 4)[first:8 ** depth].astype(np.float64)
+        for w, few in ((lod[:, 0], False), (lod[:, 0] * lod[:, 1], True)):  # as many evenly filled bins; the line: 300 and 70
+            bins = np.abs(w).sum() ** 2 / (w ** 2).sum()
+            assert bins < (150, 40)[depth == 3] if few else bins > (1000, 120)[depth == 3], bins
+    doms = [U.setup_gpu(c) for c in cases]
+    for d in doms:
+        d.initialize()
+    b = I.Batch(doms)
+    b.run(steps)
+    b.finish(120000)
+    for c, d, s in zip(cases, doms, solo):
+        for name in U.field_names(c):
+            assert U.bit_diff_nan(d.read(name), s.read(name)) == 0, name
+    b.close()
